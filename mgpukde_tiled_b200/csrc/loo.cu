@@ -11,25 +11,28 @@
 //   loo_j(h) = sum_{i != j, d^2 < 9h^2} exp(-d^2 / 2h^2) / (h^2 TWO_PI) w_i e_i(h)
 //   logL(h)  = sum_j log(max(loo_j(h), EPSILONDENSITY))
 // for every h of a list, as one persistent launch over work items
-// (h, group of 128 queries), heaviest h first, fed from a global item
-// counter.  The points are indexed once per bandwidth octave (row-major bins
-// of side in (0.375 h, 0.75 h] for the h that use the level), so the
-// candidates of a group are one contiguous range per bin row; they arrive in
-// batches of up to 128 (one bin row's range at a time) through a
-// double-buffered TMA bulk copy into shared memory, and every thread (one
-// query) scans them.  The cutoff is decided in FP32
-// with a band around 9h^2 re-decided by the oracle's exact FP64 test, so the
-// summed pair set is exactly the oracle's; terms are FP32 (an exp2 by range
-// reduction and a polynomial, free of the systematic bias an approximate
-// special-function exp2 would add to every one of the sum's terms), summed
-// per batch and added into a Kahan-compensated FP32 accumulator; the per-query log is FP64, and the per-group and per-h sums
-// are fixed-order FP64 trees (bitwise reproducible).  The argmax is taken on
-// the device.  The whole sequence (edge weights for every h, the gather, the
+// (h, group of 128 queries, quarter of the group[, part of its candidates]),
+// one warp each, heaviest h first, fed from a global item counter.  The points
+// are indexed once per bandwidth octave (row-major bins of side in (0.375 h,
+// 0.75 h] for the h that use the level), so the candidates of a group are one
+// contiguous range per bin row.  A group is 128 consecutive records of the
+// Z-order of the bins.  Candidates come in batches of 64, two per lane, into
+// the warp's shared memory; every lane (one query) scans them, two candidates
+// at a time in packed FP32.  The cutoff is decided in FP32 with a band around
+// 9h^2 re-decided by the oracle's exact FP64 test, so the summed pair set is
+// exactly the oracle's; terms are FP32 (an exp2 by range reduction and a
+// polynomial, free of the systematic bias an approximate special-function
+// exp2 would add to every one of the sum's terms), summed over at most 128
+// candidates of one bin row and added into a Kahan-compensated FP32
+// accumulator; the per-query log is FP64, and the per-group and per-h sums are
+// fixed-order FP64 trees (bitwise reproducible).  The argmax is taken on the
+// device.  The whole sequence (edge weights for every h, the gather, the
 // sums, the argmax) is captured once into a CUDA graph and replayed, with the
 // bandwidths read from device memory, so a golden-section step is one graph
 // launch.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -37,14 +40,23 @@
 
 namespace {
 
-constexpr int kLooQ = 128;    // queries (threads) per work item
-// candidates per staged batch (at most one per thread, which reads its
-// candidate's weight): with the scan unrolled by 8, 32, 64 and 128 gave
-// 271, 257 and 251 ms for the 64-bandwidth selection (C2)
-constexpr int kLooB = 128;
-static_assert(kLooB <= kLooQ, "one thread per staged candidate");
+constexpr int kLooQ = 128;    // queries of a group; a work item is a quarter of one, a query per lane
+constexpr int kLooSub = kLooQ / 32;
+constexpr int kLooB = 64;     // candidates per staged batch, two per lane
+constexpr int kLooSum = 128;  // candidates of a bin row summed in plain FP32 before each Kahan step
+constexpr int kLooWarps = 4;  // warps per CTA, each with work items of its own
 constexpr int kMaxLev = 16;   // bandwidth octaves
-constexpr long long kLooSpin = 1ll << 24;
+constexpr int kMaxSplit = 16;
+// The cutoff in the scan's exponents, 9 h^2 log2(e) / (2 h^2), and the band
+// around it in which FP32 does not decide.
+constexpr float kLooCut = (float)(0.5 * MGK_CUT * MGK_LOG2E);
+constexpr float kLooBand = 4e-6f * kLooCut;
+// candidates of a batch scanned at a time (one test for the rare cases)
+#ifndef MGK_LOO_TRIP
+#define MGK_LOO_TRIP 8
+#endif
+constexpr int kLooTrip = MGK_LOO_TRIP;
+static_assert(kLooB % kLooTrip == 0 && kLooTrip % 2 == 0 && kLooSum % kLooTrip == 0, "whole trips");
 
 struct LevelDesc {
     const MgkPt* pts;
@@ -53,26 +65,13 @@ struct LevelDesc {
     const int32_t* qord;  // query order: record positions in Z-order of the bins
     double ox, oy, side, inv_side;
     int64_t nbx, nby;
-    double quantum;       // coordinate quantum of the records' hi/lo split
 };
-
-// Rejects most out-of-cutoff candidates on their hi parts (4 instructions)
-// before the exact pair arithmetic.
-#ifndef MGK_LOO_PREFILTER
-#define MGK_LOO_PREFILTER 1
-#endif
-// candidates per trip of the scan loop: 8 measured fastest on the
-// 64-bandwidth selection (C2: 317, 290, 282, 271, 274 and 290 ms at 1, 2, 4,
-// 8, 16 and 32; the compiler's own choice gave 290)
-#ifndef MGK_LOO_UNROLL
-#define MGK_LOO_UNROLL 8
-#endif
-constexpr int kLooUnroll = MGK_LOO_UNROLL;
 
 struct LooParams {
     const LevelDesc* lev;  // [nlev], device
     double side[kMaxLev];  // bin side of each level
     int nlev;
+    int nsplit;  // parts of a group's candidates, each a work item of its own
     int64_t n;
     int ngroups;
     int g0, gcount;       // this share's query groups [g0, g0 + gcount) (all groups: 0, ngroups)
@@ -86,51 +85,90 @@ struct LooParams {
     // chunk of n points, [nh][n], in a single-process batch)
     const float* ew;
     int64_t ew_chunk, ew_cstride;
-    double* part;         // [nh][gcount]
+    // w e of every record of the level that h_k uses, in record order ([nh][n]), or null
+    float* wl;
+    double* psum;         // [nsplit][nh][gcount * kLooSub][32] unnormalised sums (nsplit > 1), else null
+    double* part;         // [nh][gcount * kLooSub]
     unsigned* counter;    // work-item queue head
     unsigned long long* evals;
-    unsigned long long* err;
 };
 
-// ---- TMA bulk copy + mbarrier (sm_90+ PTX) ---------------------------------
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+// ---- two FP32 values in a 64-bit register (sm_100 f32x2; each half is
+// rounded as the scalar operation is)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_dup(float a) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
 }
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t* b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* b) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(b))
-                 : "memory");
+__device__ __forceinline__ void f2_get(f2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
-    for (long long i = 0; i < kLooSpin; i++)
-        if (mbar_try_wait(b, parity)) return true;
-    return false;
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-__device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
+__device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double t = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += sh[i];
-    return t;
+    return v;
+}
+
+// The log of a query's leave-one-out density from its unnormalised sum.
+__device__ __forceinline__ double loo_log(double sum, double h2) {
+    const double loo = sum / (h2 * (double)MGK_TWO_PI_F);
+    const double fl = (double)MGK_EPS_DENSITY_F;
+    return log(loo > fl ? loo : fl);
+}
+
+// 2^-g for g in [-1/2, 1/2]: a degree-6 polynomial, fitted to 2^-g by least
+// squares on Chebyshev nodes with the mean error held where the rounding of
+// the scan's terms leaves none, each coefficient rounded to float before the
+// next ones are fitted (truncation 3.3e-9 relative; the weighted mean error of
+// the terms over the cutoff's disc is 1e-12, that of a degree-8 Taylor form on
+// an unscaled distance -6e-11).  Scalar with immediate coefficients: a packed
+// FMA with three register pairs runs at 3.3 cycles instead of 2.
+__device__ __forceinline__ float exp2_neg_frac(float g) {
+    float p = __fmaf_rn(0.00015285507834050804f, g, -0.001339130220003426f);
+    p = __fmaf_rn(p, g, 0.009618666023015976f);
+    p = __fmaf_rn(p, g, -0.055503588169813156f);
+    p = __fmaf_rn(p, g, 0.24022646248340607f);
+    p = __fmaf_rn(p, g, -0.6931471824645996f);
+    return __fmaf_rn(p, g, 1.0f);
+}
+
+// v on a grid of step q = m / (1.5 2^52) (hi) and the remainder (lo)
+__device__ __forceinline__ void split_at(double v, double m, float& hi, float& lo) {
+    const double t = __dsub_rn(__dadd_rn(v, m), m);
+    hi = (float)t;
+    lo = (float)__dsub_rn(v, t);
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
 // Level and processing order of every h (one CTA; nh is small).
@@ -150,184 +188,340 @@ __global__ void k_loo_prep(LooParams P) {
     }
 }
 
-__global__ void __launch_bounds__(kLooQ) k_loo_multi(LooParams P) {
-    __shared__ __align__(128) MgkPt stage[2][kLooB];
-    __shared__ float sw[2][kLooB];
-    __shared__ __align__(8) uint64_t mbar[2];
-    __shared__ double red[kLooQ / 32];
-    __shared__ float bb[4][kLooQ / 32];
-    __shared__ int s_item;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
-        fence_mbar_init();
+// wl[k][i] = w e(h_k) of record i of the level of h_k: the scan then reads its
+// candidates' weights in order instead of through the permutation.
+__global__ void k_loo_weights(LooParams P) {
+    const int k = blockIdx.y;
+    const LevelDesc L = P.lev[P.klevel[k]];
+    const float* ewk = P.ew + (int64_t)k * P.ew_chunk;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t pi = L.perm[i], ch = pi / P.ew_chunk;
+        P.wl[(int64_t)k * P.n + i] = L.pts[i].wk * ewk[ch * P.ew_cstride + (pi - ch * P.ew_chunk)];
     }
-    __syncthreads();
-    unsigned ph0 = 0u, ph1 = 0u;  // mbarrier phase parities of the two buffers
-    const unsigned total = (unsigned)P.nh * (unsigned)P.gcount;
+}
+
+// What bounds it: the issue slots and the FMA pipe together (about 23
+// instructions and 21 FMA-pipe cycles per candidate and warp; ncu: 73 % of the
+// issue slots, 68 % of the FMA cycles).  200,000 points, 64 bandwidths in
+// [5, 500]: 225 ms before (scalar FP32, 128 queries a CTA between two
+// barriers per batch, 1.72 tests per pair), 125 ms now.  What gave it:
+//  - distances, exponents and range reduction two candidates at a time
+//    (f32x2), with the coordinates scaled so that the squared distance is the
+//    exponent (two packed operations fewer per pair of candidates);
+//  - the polynomial scalar, its coefficients immediates (see exp2_neg_frac);
+//  - pair counts from sign bits: a predicated increment costs two instructions;
+//  - a warp its own work item: no CTA barriers, and rows cut to the disc
+//    around 32 queries instead of the square around 128 (1.38 tests a pair).
+// Finer bins or a Hilbert order would cut the tests to 1.2 a pair, but then
+// the pieces summed in plain FP32 hold other candidates, and with edge weights
+// of points outside the study area (10^6 and more) logL moves by 3e-9.
+// More resident warps (80 or 64 registers) spill and are slower: 134 ms.
+// Resident CTAs per SM that bound the registers.
+#ifndef MGK_LOO_MIN_CTAS
+#define MGK_LOO_MIN_CTAS 4
+#endif
+
+__global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(LooParams P) {
+    // per warp: candidates by component (xh, yh, xl, yl, weight), two batches
+    __shared__ __align__(16) float s_cand[kLooWarps][2][5][kLooB];
+    // of the window's rows: their slots end, what takes a slot to its place in
+    // the group's range of the row, that range's first record, the place where
+    // this item's part of it ends
+    __shared__ int4 s_row[kLooWarps][32];
+    const int warp = threadIdx.x >> 5;
+    int lane;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));  // kept in a register
+    float(*cand)[5][kLooB] = s_cand[warp];
+    int4* row = s_row[warp];
+    const unsigned ngs = (unsigned)P.gcount * kLooSub;  // quarters of groups
+    const unsigned per_h = ngs * (unsigned)P.nsplit;
+    const unsigned total = (unsigned)P.nh * per_h;
+    const f2 magic = f2_dup(12582912.0f);  // 1.5 2^23: adding it rounds to the nearest integer
     unsigned long long cnt_all = 0;
     for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(P.counter, 1u);
-        __syncthreads();
-        const unsigned item = (unsigned)s_item;
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(P.counter, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= total) break;
-        const int k = P.korder[item / (unsigned)P.gcount];
-        const int grp = P.g0 + (int)(item % (unsigned)P.gcount);
-        const LevelDesc L = P.lev[P.klevel[k]];
+        const int k = P.korder[item / per_h];
+        const int split = (int)((item % per_h) / ngs);
+        const int gi = (int)((item % per_h) % ngs);  // quarter gi % kLooSub of group gi / kLooSub
+        const LevelDesc& L = P.lev[P.klevel[k]];
         const float h = P.hgrid[k];
         const double h2 = mgk_h2(h);
         const double cut = MGK_CUT * h2;
-        const float cutf = (float)cut;
-        const float epsd2 = cutf * 4e-6f;
-        // log2(e) / (2 h^2) as a float pair: a one-float scale would bias every
-        // exponent of the batch the same way
-        const double k2 = MGK_LOG2E / (2.0 * h2);
-        const float k2h = (float)k2, k2l = (float)(k2 - (double)k2h);
         const double reach = sqrt(cut) * (1.0 + 1e-9);
-        // squared hi-part distance beyond which a candidate is surely outside
-        // the cutoff (|lo parts| <= q / 2 each; 1e-5 covers the float rounding)
-        const float far2 = (float)((reach + 2.0 * L.quantum) * (reach + 2.0 * L.quantum) * (1.0 + 1e-5));
-        const float* ewk = P.ew ? P.ew + (int64_t)k * P.ew_chunk : nullptr;
+        const MgkPt* __restrict__ pts = L.pts;
+        const float* __restrict__ wl = P.wl ? P.wl + (int64_t)k * P.n : nullptr;
 
-        // this item's query
-        // the group's queries: 128 consecutive records of the Z-order, a
-        // compact patch of bins (row-major runs would be long thin strips)
-        const int64_t qk = (int64_t)grp * kLooQ + tid;
-        const bool qv = qk < P.n;
-        const int64_t qpos = qv ? (int64_t)L.qord[qk] : -1;
-        MgkPt q{};
-        if (qv) q = L.pts[qpos];
-        const float qx = q.xh + q.xl, qy = q.yh + q.yl;
-        // bounding box of the group's queries
-        float mnx = qv ? qx : FLT_MAX, mxx = qv ? qx : -FLT_MAX, mny = qv ? qy : FLT_MAX, mxy = qv ? qy : -FLT_MAX;
+        // this lane's query, and the bounding boxes of the item's queries and of the group's
+        const int64_t q0 = (int64_t)(P.g0 + gi / kLooSub) * kLooQ;
+        int qpos = -1;
+        float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float mnx = FLT_MAX, mxx = -FLT_MAX, mny = FLT_MAX, mxy = -FLT_MAX;
+        float gmnx = FLT_MAX, gmxx = -FLT_MAX;
+#pragma unroll
+        for (int i = 0; i < kLooSub; i++) {
+            const int64_t qk = q0 + 32 * i + lane;
+            if (qk >= P.n) continue;
+            const int qp = L.qord[qk];
+            const float4 v = *reinterpret_cast<const float4*>(pts + qp);
+            const float vx = v.x + v.z, vy = v.y + v.w;
+            gmnx = fminf(gmnx, vx);
+            gmxx = fmaxf(gmxx, vx);
+            if (i == gi % kLooSub) {
+                q = v;
+                qpos = qp;
+                mnx = mxx = vx;
+                mny = mxy = vy;
+            }
+        }
+        const bool qv = qpos >= 0;
+        const float qx = q.x + q.z, qy = q.y + q.w;
         for (int o = 16; o; o >>= 1) {
             mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
             mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
             mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
             mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+            gmnx = fminf(gmnx, __shfl_xor_sync(0xffffffffu, gmnx, o));
+            gmxx = fmaxf(gmxx, __shfl_xor_sync(0xffffffffu, gmxx, o));
         }
-        if (lane == 0) {
-            bb[0][warp] = mnx;
-            bb[1][warp] = mxx;
-            bb[2][warp] = mny;
-            bb[3][warp] = mxy;
+        if (mnx > mxx) {  // no query in this quarter
+            if (P.psum) P.psum[(((int64_t)split * P.nh + k) * ngs + gi) * 32 + lane] = 0.0;
+            else if (lane == 0) P.part[(int64_t)k * ngs + gi] = 0.0;
+            continue;
         }
-        __syncthreads();
-        for (int i = 0; i < kLooQ / 32; i++) {
-            mnx = fminf(mnx, bb[0][i]);
-            mxx = fmaxf(mxx, bb[1][i]);
-            mny = fminf(mny, bb[2][i]);
-            mxy = fmaxf(mxy, bb[3][i]);
-        }
-        const int64_t bx0 = mgk_max64(0, (int64_t)floor(((double)mnx - reach - L.ox) * L.inv_side));
-        const int64_t bx1 = mgk_min64(L.nbx - 1, (int64_t)floor(((double)mxx + reach - L.ox) * L.inv_side));
-        const int64_t by0 = mgk_max64(0, (int64_t)floor(((double)mny - reach - L.oy) * L.inv_side));
-        const int64_t by1 = mgk_min64(L.nby - 1, (int64_t)floor(((double)mxy + reach - L.oy) * L.inv_side));
+        const int by0 = (int)fmax(0.0, floor(((double)mny - reach - L.oy) * L.inv_side));
+        const int by1 = (int)fmin((double)(L.nby - 1), floor(((double)mxy + reach - L.oy) * L.inv_side));
+        // the group's bin columns
+        const double g0 = fmax(0.0, floor(((double)gmnx - reach - L.ox) * L.inv_side));
+        const double g1 = fmin((double)(L.nbx - 1), floor(((double)gmxx + reach - L.ox) * L.inv_side));
+        // the query's bin row, as the index assigns it
+        const int qby = (int)fmin(fmax(floor(((double)qy - L.oy) * L.inv_side), 0.0), (double)(L.nby - 1));
 
-        float s = 0.0f, c = 0.0f;
-        unsigned cnt = 0;
-        // candidate stream: batches of <= kLooB within one bin row
-        int64_t by = by0, pos = 0, end = 0;
-        auto next = [&](int64_t& src) -> int {
-            while (pos >= end) {
-                if (by > by1 || bx0 > bx1) return 0;
-                pos = L.bin_start[by * L.nbx + bx0];
-                end = L.bin_start[by * L.nbx + bx1 + 1];
-                by++;
-            }
-            const int m = (int)mgk_min64(kLooB, end - pos);
-            src = pos;
-            pos += m;
-            return m;
+        // Coordinates relative to the box's centre and scaled by sqrt(log2(e) / 2) / h,
+        // so that the exponent is the plain squared distance and the cutoff
+        // 4.5 log2(e) for every h; as float pairs on a grid on which the
+        // differences of the hi parts are exact.
+        const double scale = sqrt(0.5 * MGK_LOG2E / h2);
+        const double ccx = 0.5 * ((double)mnx + (double)mxx), ccy = 0.5 * ((double)mny + (double)mxy);
+        const double ext = (0.5 * fmax((double)mxx - (double)mnx, (double)mxy - (double)mny) + reach) * scale;
+        const double grid = 1.5 * 1073741824.0 * mgk_pow2(ilogb(ext) + 1);  // 1.5 2^52 q, q = 2^-22 2^(ilogb + 1)
+        float qsx, qsy, qlx, qly;
+        split_at(((double)qx - ccx) * scale, grid, qsx, qlx);
+        split_at(((double)qy - ccy) * scale, grid, qsy, qly);
+        const f2 qxh = f2_dup(qsx), qyh = f2_dup(qsy), qxl = f2_dup(qlx), qyl = f2_dup(qly);
+        const f2 cut2 = f2_dup(kLooCut);
+        // part: the candidates of a bin row since the last multiple of kLooSum
+        // of the group's range in it (a group's queries are all summed in the
+        // same pieces), then into the compensated sum
+        float s = 0.0f, c = 0.0f, part = 0.0f;
+        auto flush = [&] {
+            const float y = part - c;
+            const float tt = s + y;
+            c = (tt - s) - y;
+            s = tt;
+            part = 0.0f;
         };
-        int64_t src = 0, nsrc = 0;
-        int m = next(src);
-        int buf = 0;
-        if (m > 0 && tid == 0) {
-            mbar_arrive_tx(&mbar[0], (unsigned)(m * sizeof(MgkPt)));
-            bulk_g2s(&stage[0][0], L.pts + src, (unsigned)(m * sizeof(MgkPt)), &mbar[0]);
-        }
-        while (m > 0) {
-            const int nm = next(nsrc);
-            if (nm > 0 && tid == 0) {
-                mbar_arrive_tx(&mbar[buf ^ 1], (unsigned)(nm * sizeof(MgkPt)));
-                bulk_g2s(&stage[buf ^ 1][0], L.pts + nsrc, (unsigned)(nm * sizeof(MgkPt)), &mbar[buf ^ 1]);
-            }
-            if (tid < m) {
-                const int64_t i = src + tid;
-                float e = 1.0f;
-                if (ewk) {
-                    const int64_t pi = L.perm[i], ch = pi / P.ew_chunk;
-                    e = ewk[ch * P.ew_cstride + (pi - ch * P.ew_chunk)];
-                }
-                sw[buf][tid] = L.pts[i].wk * e;
-            }
-            const unsigned par = buf ? ph1 : ph0;
-            const bool ok = mbar_wait(&mbar[buf], par);
-            if (__syncthreads_or(!ok)) {
-                // a staging wait ran out: flag it and give the copies in
-                // flight a second bounded wait before the CTA goes away
-                if (tid == 0) {
-                    atomicExch(P.err, 1ull);
-                    mbar_wait(&mbar[buf], par);
-                    if (nm > 0) mbar_wait(&mbar[buf ^ 1], buf ? ph0 : ph1);
-                }
-                __syncthreads();
-                return;
-            }
-            if (buf) ph1 ^= 1u;
-            else ph0 ^= 1u;
-            if (qv) {
-                float part = 0.0f;
-                const MgkPt* st = stage[buf];
-#pragma unroll kLooUnroll
-                for (int t = 0; t < m; t++) {
-                    const float4 cp = *reinterpret_cast<const float4*>(&st[t]);
-#if MGK_LOO_PREFILTER
-                    // the hi parts alone first: their difference is exact and
-                    // the lo parts move d by at most 2 quanta, so a candidate
-                    // beyond far2 is outside the cutoff (2 of 3 tested are)
-                    const float dxh = __fsub_rn(cp.x, q.xh), dyh = __fsub_rn(cp.y, q.yh);
-                    if (__fmaf_rn(dxh, dxh, __fmul_rn(dyh, dyh)) > far2) continue;
-#endif
-                    const float dx = __fadd_rn(__fsub_rn(cp.x, q.xh), __fsub_rn(cp.z, q.xl));
-                    const float dy = __fadd_rn(__fsub_rn(cp.y, q.yh), __fsub_rn(cp.w, q.yl));
-                    const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                    bool in = d2 < cutf;
-                    if (fabsf(d2 - cutf) <= epsd2)  // near the cutoff: the oracle's FP64 decision
-                        in = mgk_d2_exact(qx, qy, cp.x + cp.z, cp.y + cp.w) < cut;
-                    if (in && src + t != qpos) {
-                        const float a = __fmaf_rn(d2, k2h, __fmul_rn(d2, k2l));
-                        part = __fmaf_rn(mgk_exp2_neg_poly(a), sw[buf][t], part);
-                        cnt++;
+        unsigned cnt = 0;
+        // The item's bin rows, 32 at a time.  The candidates of a stretch of
+        // rows are numbered through in slots, each row's from a multiple of
+        // kLooTrip of the group's range and to a whole number of trips.
+        for (int rb = by0; rb <= by1; rb += 32) {
+            __syncwarp();  // the previous stretch's tables have been read
+            {
+                // a point of the row can be in reach of the box only within
+                // sqrt(reach^2 - dy^2) of it, dy the rows' distance (a lower
+                // bound): the window is the box grown by a disc
+                int4 rw = make_int4(0, 0, 0, 0);
+                const int by = rb + lane;
+                if (by <= by1) {
+                    const double rlo = L.oy + (double)by * L.side, rhi = rlo + L.side;
+                    const double dy = fmax(0.0, fmax(rlo - (double)mxy, (double)mny - rhi)) * (1.0 - 1e-9);
+                    const double rr = reach * reach - dy * dy;
+                    if (rr >= 0.0) {
+                        const double hw = sqrt(rr) * (1.0 + 1e-9) + 1e-9 * reach;
+                        const double f0 = fmax(g0, floor(((double)mnx - hw - L.ox) * L.inv_side));
+                        const double f1 = fmin(g1, floor(((double)mxx + hw - L.ox) * L.inv_side));
+                        if (f0 <= f1) {
+                            const int32_t* bs = L.bin_start + (int64_t)by * L.nbx;
+                            rw.z = bs[(int64_t)g0];
+                            rw.y = (bs[(int64_t)f0] - rw.z) / kLooTrip * kLooTrip;
+                            rw.w = bs[(int64_t)f1 + 1] - rw.z;
+                        }
                     }
                 }
-                const float y = part - c;
-                const float tt = s + y;
-                c = (tt - s) - y;
-                s = tt;
+                const int len = rw.w > rw.y ? (rw.w - rw.y + kLooTrip - 1) / kLooTrip * kLooTrip : 0;
+                int end = len;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, end, o);
+                    if (lane >= o) end += v;
+                }
+                rw.x = end;
+                rw.y -= end - len;
+                row[lane] = rw;
             }
-            __syncthreads();  // stage[buf] and sw[buf] are reused two batches on
-            m = nm;
-            src = nsrc;
-            buf ^= 1;
+            __syncwarp();
+            // this part's slots, between multiples of kLooSum of the rows' ranges
+            const int64_t T = row[31].x;
+            auto part_at = [&](int sp) {
+                int j = (int)(T * sp / P.nsplit), i = 0, pre = 0;
+                if (sp == 0 || sp == P.nsplit || T == 0) return j;  // (no row ends beyond slot 0 if T is 0)
+                while (j >= row[i].x) pre = row[i++].x;
+                j = (j + row[i].y) / kLooSum * kLooSum - row[i].y;
+                return max(j, pre);
+            };
+            const int j0 = part_at(split), j1 = part_at(split + 1);
+            // the query's own slot
+            const int jself =
+                qv && qby >= rb && qby < rb + 32 ? qpos - row[qby - rb].z - row[qby - rb].y : -1;
+            // the row of this lane's next candidate
+            int r = 0, pre = 0;
+            int4 rw = row[0];
+            // this lane's two candidates of the coming batch
+            float4 cp[2];
+            float cw[2];
+            unsigned new_sum[2];  // bit b: the trip that starts at the b-th slot begins a piece of its row
+            auto fetch = [&](int jb) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int j = jb + 32 * i;
+                    cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end
+                    cw[i] = 0.0f;
+                    bool first = false;
+                    int o = INT_MAX;
+                    if (j < j1) {
+                        while (j >= rw.x) {
+                            pre = rw.x;
+                            rw = row[++r];
+                        }
+                        o = j + rw.y;
+                        first = j == pre || o % kLooSum == 0;
+                    }
+                    new_sum[i] = __ballot_sync(0xffffffffu, first);
+                    if (o >= rw.w) continue;
+                    const int cpos = rw.z + o;
+                    cp[i] = *reinterpret_cast<const float4*>(pts + cpos);
+                    if (wl) {
+                        cw[i] = wl[cpos];
+                    } else {
+                        cw[i] = pts[cpos].wk;
+                        if (P.ew) {
+                            const int64_t pi = L.perm[cpos], ch = pi / P.ew_chunk;
+                            cw[i] *= P.ew[(int64_t)k * P.ew_chunk + ch * P.ew_cstride + (pi - ch * P.ew_chunk)];
+                        }
+                    }
+                }
+            };
+            auto put = [&](int buf) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    float xh, xl, yh, yl;
+                    split_at(((double)(cp[i].x + cp[i].z) - ccx) * scale, grid, xh, xl);
+                    split_at(((double)(cp[i].y + cp[i].w) - ccy) * scale, grid, yh, yl);
+                    cand[buf][0][lane + 32 * i] = cp[i].x < 1e18f ? xh : 1e18f;  // past the end: far outside the cutoff
+                    cand[buf][1][lane + 32 * i] = yh;
+                    cand[buf][2][lane + 32 * i] = xl;
+                    cand[buf][3][lane + 32 * i] = yl;
+                    cand[buf][4][lane + 32 * i] = cw[i];
+                }
+            };
+            int buf = 0;
+            fetch(j0 + lane);
+            put(0);
+            __syncwarp();
+            flush();
+            for (int j = j0; j < j1; j += kLooB) {
+                const int m = min(kLooB, j1 - j);
+                const bool more = j + kLooB < j1;
+                const unsigned long long pieces = ((unsigned long long)new_sum[1] << 32) | new_sum[0];
+                if (more) fetch(j + kLooB + lane);
+#pragma unroll 1
+                for (int t = 0; t < m; t += kLooTrip) {
+                    if ((pieces >> t) & 1u) flush();
+                    // x < 0: inside the cutoff; the term is p times the weight ws
+                    float p[kLooTrip], x[kLooTrip], ws[kLooTrip];
+#pragma unroll
+                    for (int u = 0; u < kLooTrip; u += 2) {
+                        const f2 xh = *reinterpret_cast<const f2*>(&cand[buf][0][t + u]);
+                        const f2 yh = *reinterpret_cast<const f2*>(&cand[buf][1][t + u]);
+                        const f2 xl = *reinterpret_cast<const f2*>(&cand[buf][2][t + u]);
+                        const f2 yl = *reinterpret_cast<const f2*>(&cand[buf][3][t + u]);
+                        const f2 w = *reinterpret_cast<const f2*>(&cand[buf][4][t + u]);
+                        const f2 dx = f2_add(f2_sub(xh, qxh), f2_sub(xl, qxl));
+                        const f2 dy = f2_add(f2_sub(yh, qyh), f2_sub(yl, qyl));
+                        const f2 a = f2_fma(dx, dx, f2_mul(dy, dy));
+                        f2_get(f2_sub(a, cut2), x[u], x[u + 1]);
+                        // 2^-a = 2^-n 2^-g with a = n + g, |g| <= 1/2.  2^-n comes from the
+                        // special-function unit, which is exact for integers and idle
+                        // otherwise, not from a shift into the exponent bits
+                        const f2 n = f2_sub(f2_sub(magic, a), magic);  // -n
+                        float g0, g1, n0, n1;
+                        f2_get(f2_add(a, n), g0, g1);
+                        f2_get(n, n0, n1);
+                        p[u] = exp2_neg_frac(g0);
+                        p[u + 1] = exp2_neg_frac(g1);
+                        f2_get(f2_mul(w, f2_make(mgk_ex2(n0), mgk_ex2(n1))), ws[u], ws[u + 1]);
+                    }
+                    const int ts = jself - (j + t);  // the query's own place in the trip, if in it
+                    float near = fabsf(x[0]);
+#pragma unroll
+                    for (int u = 1; u + 1 < kLooTrip; u += 2) near = min3(near, fabsf(x[u]), fabsf(x[u + 1]));
+                    near = fminf(near, fabsf(x[kLooTrip - 1]));
+                    if (near <= kLooBand || (unsigned)ts < (unsigned)kLooTrip) {
+#pragma unroll
+                        for (int u = 0; u < kLooTrip; u++) {
+                            if (fabsf(x[u]) <= kLooBand) {  // near the cutoff: the oracle's FP64 decision
+                                int rr = 0;
+                                while (j + t + u >= row[rr].x) rr++;
+                                const float4 cc =
+                                    *reinterpret_cast<const float4*>(pts + (j + t + u + row[rr].y + row[rr].z));
+                                x[u] = mgk_d2_exact(qx, qy, cc.x + cc.z, cc.y + cc.w) < cut ? -1.0f : 1.0f;
+                            }
+                            if (u == ts) x[u] = 1.0f;  // the query itself
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kLooTrip; u++) {
+                        if (x[u] < 0.0f) part = __fmaf_rn(p[u], ws[u], part);
+                        cnt += __float_as_uint(x[u]) >> 31;
+                    }
+                }
+                if (more) put(buf ^ 1);
+                __syncwarp();  // this batch has been scanned, the next one is in place
+                buf ^= 1;
+            }
         }
-        double lg = 0.0;
-        if (qv) {
-            const double loo = ((double)s - (double)c) / (h2 * (double)MGK_TWO_PI_F);
-            const double fl = (double)MGK_EPS_DENSITY_F;
-            lg = log(loo > fl ? loo : fl);
+        flush();
+        if (qv) cnt_all += cnt;
+        const double sum_q = (double)s - (double)c;
+        if (P.psum) {
+            P.psum[(((int64_t)split * P.nh + k) * ngs + gi) * 32 + lane] = sum_q;
+        } else {
+            const double sum = warp_sum(qv ? loo_log(sum_q, h2) : 0.0);
+            if (lane == 0) P.part[(int64_t)k * ngs + gi] = sum;
         }
-        const double sum = block_sum_fixed(lg, red);
-        if (tid == 0) P.part[(int64_t)k * P.gcount + (grp - P.g0)] = sum;
-        cnt_all += cnt;
-        __syncthreads();  // s_item is rewritten next
     }
     if (P.evals) {
         for (int o = 16; o; o >>= 1) cnt_all += __shfl_xor_sync(0xffffffffu, cnt_all, o);
         if (lane == 0 && cnt_all) atomicAdd(P.evals, cnt_all);
     }
+}
+
+// The log sums of the groups' quarters from the parts' sums of each query,
+// added in order (one warp per quarter).
+__global__ void __launch_bounds__(kLooWarps * 32) k_loo_combine(LooParams P) {
+    const int lane = threadIdx.x & 31, gi = blockIdx.x * kLooWarps + (threadIdx.x >> 5), k = blockIdx.y;
+    const int64_t ngs = (int64_t)P.gcount * kLooSub;
+    if (gi >= ngs) return;
+    double lg = 0.0;
+    if ((int64_t)P.g0 * kLooQ + (int64_t)gi * 32 + lane < P.n) {
+        double v = 0.0;
+        for (int sp = 0; sp < P.nsplit; sp++) v += P.psum[(((int64_t)sp * P.nh + k) * ngs + gi) * 32 + lane];
+        lg = loo_log(v, mgk_h2(P.hgrid[k]));
+    }
+    const double sum = warp_sum(lg);
+    if (lane == 0) P.part[k * ngs + gi] = sum;
 }
 
 // logL[k] = fixed-order sum of the group partials of h_k (one CTA per h).
@@ -374,40 +568,52 @@ struct mgk_loo_batch {
     cudaStream_t cap = nullptr;  // capture stream
     int* d_korder = nullptr;
     int* d_klevel = nullptr;
+    float* d_wl = nullptr;
+    double* d_psum = nullptr;
     double* d_part = nullptr;
     double* d_logl = nullptr;
     int* d_best = nullptr;
     unsigned* d_counter = nullptr;
     unsigned long long* d_evals = nullptr;  // [0] edge, [1] loo
-    unsigned long long* d_err = nullptr;
     float* h_h = nullptr;       // pinned
     double* h_logl = nullptr;   // pinned: nh logL, then the argmax and the eval counts
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     LooParams P{};
-    size_t bytes_ew = 0, bytes_part = 0;
+    size_t bytes_ew = 0, bytes_wl = 0, bytes_psum = 0, bytes_part = 0;
+    int grid = 1;
 };
+
+// Kernels of a batch, the edge weights' aside.
+static int loo_launches(const mgk_loo_batch* B) {
+    return 3 + (B->P.wl ? 1 : 0) + (B->P.gcount > 0 ? 1 : 0) + (B->P.gcount > 0 && B->P.psum ? 1 : 0);
+}
 
 static int loo_enqueue(mgk_loo_batch* B) {
     mgk_ctx* ctx = B->ctx;
     cudaStream_t s = ctx->stream;
     MGK_CHECK_CUDA(ctx, cudaMemsetAsync(B->d_counter, 0, sizeof(unsigned), s));
     MGK_CHECK_CUDA(ctx, cudaMemsetAsync(B->d_evals, 0, 2 * sizeof(unsigned long long), s));
-    MGK_CHECK_CUDA(ctx, cudaMemsetAsync(B->d_err, 0, sizeof(unsigned long long), s));
     if (B->mask) {
         int st = mgk_launch_edge_weights_multi(ctx, B->n, B->pts->x, B->pts->y, nullptr, 0.0f, B->d_h, B->nh,
                                                B->pts->dist2, B->mask, B->d_ew, B->n, B->d_evals);
         if (st) return st;
     }
     k_loo_prep<<<1, 256, 0, s>>>(B->P);
-    const int occ = 8;  // resident CTAs of 128 threads per SM targeted by the persistent grid
-    const unsigned items = (unsigned)B->nh * (unsigned)std::max(B->P.gcount, 1);
-    const unsigned grid = std::max(1u, std::min(items, (unsigned)(ctx->sm_count * occ)));
-    k_loo_multi<<<grid, kLooQ, 0, s>>>(B->P);
-    k_loo_finish<<<B->nh, 256, 0, s>>>(B->d_part, B->P.gcount, B->d_logl);
+    if (B->P.wl) {
+        const unsigned gx = (unsigned)std::min<int64_t>((B->n + 255) / 256, 4 * (int64_t)ctx->sm_count);
+        k_loo_weights<<<dim3(gx, (unsigned)B->nh), 256, 0, s>>>(B->P);
+    }
+    if (B->P.gcount > 0) {
+        k_loo_multi<<<(unsigned)B->grid, kLooWarps * 32, 0, s>>>(B->P);
+        if (B->P.psum)
+            k_loo_combine<<<dim3((unsigned)((B->P.gcount * kLooSub + kLooWarps - 1) / kLooWarps), (unsigned)B->nh),
+                            kLooWarps * 32, 0, s>>>(B->P);
+    }
+    k_loo_finish<<<B->nh, 256, 0, s>>>(B->d_part, B->P.gcount * kLooSub, B->d_logl);
     k_argmax<<<1, 32, 0, s>>>(B->d_logl, B->nh, B->d_best);
     MGK_CHECK_LAUNCH(ctx, "loo batch");
-    MGK_COUNT_LAUNCH(ctx, 4);
+    MGK_COUNT_LAUNCH(ctx, loo_launches(B));
     return MGK_OK;
 }
 
@@ -425,12 +631,13 @@ void mgk_loo_batch_destroy(mgk_loo_batch* B) {
     mgk_free(c, B->d_ew, B->bytes_ew);
     mgk_free(c, B->d_korder, sizeof(int) * nh);
     mgk_free(c, B->d_klevel, sizeof(int) * nh);
+    mgk_free(c, B->d_wl, B->bytes_wl);
+    mgk_free(c, B->d_psum, B->bytes_psum);
     mgk_free(c, B->d_part, B->bytes_part);
     mgk_free(c, B->d_logl, sizeof(double) * nh);
     mgk_free(c, B->d_best, sizeof(int));
     mgk_free(c, B->d_counter, sizeof(unsigned));
     mgk_free(c, B->d_evals, 2 * sizeof(unsigned long long));
-    mgk_free(c, B->d_err, sizeof(unsigned long long));
     if (B->h_h) cudaFreeHost(B->h_h);
     if (B->h_logl) cudaFreeHost(B->h_logl);
     delete B;
@@ -485,7 +692,7 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     }
     const size_t n1 = (size_t)std::max<int64_t>(p->n, 1);
     B->bytes_ew = r ? sizeof(float) * n1 * (size_t)nh : 16;
-    B->bytes_part = sizeof(double) * (size_t)nh * (size_t)std::max(B->gcount, 1);
+    B->bytes_part = sizeof(double) * (size_t)nh * (size_t)std::max(B->gcount, 1) * kLooSub;
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_h, sizeof(float) * nh);
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_ew, B->bytes_ew);
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_korder, sizeof(int) * nh);
@@ -495,12 +702,33 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_best, sizeof(int));
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_counter, sizeof(unsigned));
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_evals, 2 * sizeof(unsigned long long));
-    if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_err, sizeof(unsigned long long));
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_lev, sizeof(LevelDesc) * kMaxLev);
+    // Parts of a group's candidates: enough work items for about two rounds of
+    // the resident CTAs (a golden-section step on 20,000 points has 314
+    // groups, 2 a CTA slot's quarter).  From the whole problem's groups, so a
+    // share of it sums each query as the whole does.
+    int nsplit = 1;
+    int occ = 1;
+    if (st == MGK_OK && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_loo_multi, kLooWarps * 32, 0) != cudaSuccess)
+        st = mgk_fail(c, MGK_ERR_CUDA, "loo batch: occupancy");
+    const int64_t resident = (int64_t)c->sm_count * std::max(occ, 1) * kLooWarps;  // warps
+    const int64_t items = (int64_t)nh * std::max(B->ngroups, 1) * kLooSub;
+    if (items < 2 * resident) nsplit = (int)std::min<int64_t>(kMaxSplit, (2 * resident + items - 1) / items);
+    if (st == MGK_OK && nsplit > 1) {
+        B->bytes_psum = sizeof(double) * (size_t)nsplit * (size_t)nh * (size_t)std::max(B->gcount, 1) * kLooQ;
+        if (mgk_alloc(c, (void**)&B->d_psum, B->bytes_psum)) nsplit = 1;  // no memory: whole groups
+    }
+    // The weights in record order are a shortcut: without the memory for them
+    // the scan gathers each weight through the permutation.
+    const bool has_ew = r || ew_ext;
+    if (st == MGK_OK && has_ew) {
+        B->bytes_wl = sizeof(float) * n1 * (size_t)nh;
+        if (mgk_alloc(c, (void**)&B->d_wl, B->bytes_wl)) B->d_wl = nullptr;
+    }
     if (st == MGK_OK && r) st = mgk_raster_runs(c, const_cast<mgk_raster*>(r));
     if (st == MGK_OK && cudaMallocHost((void**)&B->h_h, sizeof(float) * nh) != cudaSuccess)
         st = mgk_fail(c, MGK_ERR_CUDA, "loo batch: pinned allocation");
-    if (st == MGK_OK && cudaMallocHost((void**)&B->h_logl, sizeof(double) * (nh + 3)) != cudaSuccess)
+    if (st == MGK_OK && cudaMallocHost((void**)&B->h_logl, sizeof(double) * (nh + 2)) != cudaSuccess)
         st = mgk_fail(c, MGK_ERR_CUDA, "loo batch: pinned allocation");
     if (st) {
         mgk_loo_batch_destroy(B);
@@ -512,7 +740,7 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     for (int l = 0; l < P.nlev; l++) {
         const mgk_index* I = B->lev[l];
         hl[l] = LevelDesc{I->pts, I->bin_start, I->perm, B->qord[l], I->ox, I->oy, I->side, 1.0 / I->side, I->nbx,
-                          I->nby, std::ldexp(1.0, -I->qexp)};
+                          I->nby};
         P.side[l] = I->side;
     }
     if (cudaMemcpy(B->d_lev, hl, sizeof(LevelDesc) * P.nlev, cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -539,10 +767,14 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
         P.ew_chunk = 1;
     }
     P.ew_cstride = P.ew_chunk * (int64_t)nh;
+    P.nsplit = nsplit;
+    P.wl = B->d_wl;
+    P.psum = nsplit > 1 ? B->d_psum : nullptr;
     P.part = B->d_part;
+    B->grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)nh * B->gcount * kLooSub * nsplit + kLooWarps - 1) / kLooWarps,
+                                                     resident / kLooWarps));
     P.counter = B->d_counter;
     P.evals = B->d_evals + 1;
-    P.err = B->d_err;
     // capture the sequence into a graph on a private stream (the graph is
     // then launched into the context's stream); if capture fails, or the
     // batch runs once (replay false: capture and instantiation would cost
@@ -581,7 +813,7 @@ int mgk_loo_batch_run(mgk_loo_batch* B, const float* hs, double* logl, int* best
     MGK_CHECK_CUDA(c, cudaEventRecord(c->ev_a, s));
     if (B->exec) {
         MGK_CHECK_CUDA(c, cudaGraphLaunch(B->exec, s));
-        MGK_COUNT_LAUNCH(c, 4 + (B->mask ? 1 : 0));
+        MGK_COUNT_LAUNCH(c, loo_launches(B) + (B->mask ? 1 : 0));
     } else {
         int st = loo_enqueue(B);
         if (st) return st;
@@ -590,11 +822,9 @@ int mgk_loo_batch_run(mgk_loo_batch* B, const float* hs, double* logl, int* best
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(B->h_logl, B->d_logl, sizeof(double) * B->nh, cudaMemcpyDeviceToHost, s));
     unsigned long long* tail = reinterpret_cast<unsigned long long*>(B->h_logl + B->nh);
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(tail, B->d_evals, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    MGK_CHECK_CUDA(c, cudaMemcpyAsync(tail + 2, B->d_err, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     int* hb = reinterpret_cast<int*>(c->h_counter);
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(hb, B->d_best, sizeof(int), cudaMemcpyDeviceToHost, s));
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(s));
-    if (tail[2]) return mgk_fail(c, MGK_ERR_TIMEOUT, "loo batch: a staging wait timed out");
     for (int k = 0; k < B->nh; k++) logl[k] = B->h_logl[k];
     if (best) *best = *hb;
     if (edge_evals) *edge_evals = (int64_t)tail[0];
