@@ -17,9 +17,9 @@
 //
 // On the device: steps 1 and 4 are k_edge_rows; steps 2 and 5 are
 // k_point_density over a cell-binned index of the points (fixed-h index for
-// the pilot, per-point-h index for the LOO sum), one thread per query, the
+// the pilot, per-point-h index for the LOO sum), one lane per query, the
 // candidates staged through shared memory, the cutoff decided in FP32 with a
-// band re-decided by the oracle's FP64 test, terms from the unbiased
+// band re-decided by the oracle's FP64 test, terms from an unbiased
 // polynomial exp2, Kahan-compensated FP32 partials and an FP64 result per
 // point; the geometric mean, the bandwidths and the log sum are FP64 on the
 // device (fixed-order reductions).  The search itself runs on the host with
@@ -35,46 +35,58 @@
 
 namespace {
 
-constexpr int kPdQ = 128;  // queries (threads) per CTA
-constexpr int kPdB = 32;   // candidates per staged batch
+constexpr int kPdQ = 32;    // queries of a CTA, one per lane of its one warp
+constexpr int kPdB = 64;    // candidates per staged batch, two per lane
+constexpr int kPdTrip = 8;  // candidates scanned at a time
+constexpr int kPdSeg = 64;  // runs of bins scanned together
+// Warps per SM to split a launch into: nine rounds of the 16 that are
+// resident (three rounds leave a quarter of the slots idle in the tail, groups
+// in clusters take longest: 32.4 ms per search against 31.3)
+constexpr int kPdWarps = 144;
+// The cutoff in exponents, 9 h^2 log2(e) / (2 h^2) for every h, and the band
+// around it in which FP32 does not decide.
+constexpr float kPdCut = (float)(0.5 * MGK_CUT * MGK_LOG2E);
+constexpr float kPdBand = 4e-6f * kPdCut;
 
 // psum[y][q] = sum over candidates i (the points of the index within reach
-// of the CTA's 128 consecutive queries, in the bin rows y, y + nsplit, ... of
+// of the CTA's 32 consecutive queries, in the bin rows y, y + nsplit, ... of
 // the window, y = blockIdx.y) of [in cutoff] K w_i e_i, unnormalised; the
 // query itself is included when SELF.  Fixed h: terms exp2(-d^2 k2) w e;
 // per-point h (VARH): the candidate's own k2 and cutoff, weights already
 // carry 1/(h_i^2 TWO_PI).  Splitting the rows over nsplit CTAs gives a
 // launch enough CTAs for the whole GPU when there are few queries.
 //
-// Per-point h: the window is the group's bounding box grown by the largest
-// reach of all points, but in each bin row only the span from the first to
-// the last bin whose own largest reach (bin_r2: 9 h^2 of its widest point)
-// can touch the box is read, so points with small h far from the group are
-// never tested.
-// candidates per trip of the scan loop (8: 49.5 ms per adaptive search
-// against 50.6 ms at the compiler's own choice, 49.7 at 4 and 16)
-#ifndef MGK_PD_UNROLL
-#define MGK_PD_UNROLL 8
-#endif
-constexpr int kPdUnroll = MGK_PD_UNROLL;
-
+// The candidates are runs of bins: with fixed h one run per bin row (the box
+// around the queries grown by a disc), with per-point h the bins of the row
+// whose own largest reach (bin_r2: 9 h^2 of its widest point) can touch the
+// box, so points with small h far from the group are not tested even where a
+// wide point lies beyond them.  Up to 64 runs are numbered through and scanned
+// as one list, two candidates at a time in packed FP32 (f32x2).
+//
+// Bound by the issue slots and the FMA pipe, as the leave-one-out scan is
+// (about 25 instructions per candidate and warp).  50,000 points, one
+// likelihood's sum with per-point h: 1.06 ms with 128 queries a CTA, scalar
+// FP32 and one span of bins per row, 0.41 ms now.
 template <bool VARH, bool SELF>
-__global__ void __launch_bounds__(kPdQ) k_point_density(int64_t n, const MgkPt* __restrict__ pts,
-                                                        const int32_t* __restrict__ bin_start, double ox,
-                                                        double oy, double side, int64_t nbx, int64_t nby,
-                                                        double reach, double h2, const float* __restrict__ bin_r2,
-                                                        double quantum, double* __restrict__ psum,
-                                                        unsigned long long* __restrict__ evals) {
-    __shared__ __align__(16) MgkPt st[kPdB];
-    __shared__ float bb[4][kPdQ / 32];
-    __shared__ int s_span[2];
+__global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const MgkPt* __restrict__ pts,
+                                                            const int32_t* __restrict__ bin_start, double ox,
+                                                            double oy, double side, int64_t nbx, int64_t nby,
+                                                            double reach, double h2, const float* __restrict__ bin_r2,
+                                                            double* __restrict__ psum,
+                                                            unsigned long long* __restrict__ evals) {
+    // candidates by component: xh, yh, xl, yl, weight, k2h, k2l; two batches
+    constexpr int kComp = VARH ? 7 : 5;
+    __shared__ __align__(16) float cand[2][kComp][kPdB];
+    __shared__ int2 seg[kPdSeg];  // slots before its end, what takes a slot to its record
     const double inv_side = 1.0 / side;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t qpos = (int64_t)blockIdx.x * kPdQ + tid;
+    int lane;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));  // kept in a register
+    const unsigned lt = (1u << lane) - 1u;
+    const int64_t qpos = (int64_t)blockIdx.x * kPdQ + lane;
     const bool qv = qpos < n;
-    MgkPt q{};
-    if (qv) q = pts[qpos];
-    const float qx = q.xh + q.xl, qy = q.yh + q.yl;
+    float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (qv) q = *reinterpret_cast<const float4*>(pts + qpos);
+    const float qx = q.x + q.z, qy = q.y + q.w;
     float mnx = qv ? qx : FLT_MAX, mxx = qv ? qx : -FLT_MAX, mny = qv ? qy : FLT_MAX, mxy = qv ? qy : -FLT_MAX;
     for (int o = 16; o; o >>= 1) {
         mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
@@ -82,115 +94,206 @@ __global__ void __launch_bounds__(kPdQ) k_point_density(int64_t n, const MgkPt* 
         mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
         mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
     }
-    if (lane == 0) {
-        bb[0][warp] = mnx;
-        bb[1][warp] = mxx;
-        bb[2][warp] = mny;
-        bb[3][warp] = mxy;
-    }
-    __syncthreads();
-    for (int i = 0; i < kPdQ / 32; i++) {
-        mnx = fminf(mnx, bb[0][i]);
-        mxx = fmaxf(mxx, bb[1][i]);
-        mny = fminf(mny, bb[2][i]);
-        mxy = fmaxf(mxy, bb[3][i]);
-    }
-    const int64_t bx0 = mgk_max64(0, (int64_t)floor(((double)mnx - reach - ox) * inv_side));
-    const int64_t bx1 = mgk_min64(nbx - 1, (int64_t)floor(((double)mxx + reach - ox) * inv_side));
-    const int64_t by0 = mgk_max64(0, (int64_t)floor(((double)mny - reach - oy) * inv_side));
-    const int64_t by1 = mgk_min64(nby - 1, (int64_t)floor(((double)mxy + reach - oy) * inv_side));
+    const int by0 = (int)fmax(0.0, floor(((double)mny - reach - oy) * inv_side));
+    const int by1 = (int)fmin((double)(nby - 1), floor(((double)mxy + reach - oy) * inv_side));
     // fixed-h constants
-    const double cut = MGK_CUT * h2;
-    const float cutf = (float)cut;
     const double k2 = MGK_LOG2E / (2.0 * h2);
-    const float k2h = (float)k2, k2l = (float)(k2 - (double)k2h);
-    // squared hi-part distance beyond which a candidate is outside its cutoff:
-    // the hi parts' difference is exact and the lo parts move d by at most
-    // two quanta, so (3h + 2q)^2 = 9h^2 + 12 h q + 4 q^2 bounds it (h <= the
-    // widest reach / 3; 1e-5 covers the float rounding).  Fixed h: one bound.
-    const float far2 = (float)((reach + 2.0 * quantum) * (reach + 2.0 * quantum) * (1.0 + 1e-5));
-    const float far_add = (float)((4.0 * reach * quantum + 4.0 * quantum * quantum) * (1.0 + 1e-5));
+    const f2 k2hc = f2_dup((float)k2), k2lc = f2_dup((float)(k2 - (double)(float)k2));
+    const f2 qxh = f2_dup(q.x), qyh = f2_dup(q.y), qxl = f2_dup(q.z), qyl = f2_dup(q.w);
+    const f2 cut2 = f2_dup(kPdCut), magic = f2_dup(12582912.0f);
     float s = 0.0f, c = 0.0f;
     unsigned cnt = 0;
-    for (int64_t by = by0 + blockIdx.y; by <= by1 && bx0 <= bx1; by += gridDim.y) {
-        int64_t lo = bx0, hi = bx1;
-        if (VARH) {
-            __syncthreads();  // s_span of the previous row has been read
-            if (tid == 0) {
-                s_span[0] = INT_MAX;
-                s_span[1] = -1;
+    int nseg = 0;
+    // Scans the nseg runs in seg, there as (candidates, first record).
+    auto scan = [&] {
+        __syncwarp();
+        const int2 e0 = lane < nseg ? seg[lane] : make_int2(0, 0);
+        const int2 e1 = lane + 32 < nseg ? seg[lane + 32] : make_int2(0, 0);
+        int p0 = e0.x, p1 = e1.x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v0 = __shfl_up_sync(0xffffffffu, p0, o), v1 = __shfl_up_sync(0xffffffffu, p1, o);
+            if (lane >= o) {
+                p0 += v0;
+                p1 += v1;
             }
-            __syncthreads();
-            const double ry0 = oy + (double)by * side, ry1 = ry0 + side;
-            const double ddy = fmax(0.0, fmax(ry0 - (double)mxy, (double)mny - ry1));
-            for (int64_t bx = bx0 + tid; bx <= bx1; bx += kPdQ) {
-                const float r2 = bin_r2[by * nbx + bx];
-                if (r2 < 0.0f) continue;  // empty bin
-                const double rx0 = ox + (double)bx * side, rx1 = rx0 + side;
-                const double ddx = fmax(0.0, fmax(rx0 - (double)mxx, (double)mnx - rx1));
-                // a margin over the bin edges' rounding and the float h^2
-                if (ddx * ddx + ddy * ddy <= (double)r2 * (1.0 + 1e-5) + 1e-6 * side * side) {
-                    atomicMin(&s_span[0], (int)(bx - bx0));
-                    atomicMax(&s_span[1], (int)(bx - bx0));
+        }
+        p1 += __shfl_sync(0xffffffffu, p0, 31);
+        const int T = __shfl_sync(0xffffffffu, p1, 31);
+        seg[lane] = make_int2(p0, e0.y - (p0 - e0.x));
+        seg[lane + 32] = make_int2(p1, e1.y - (p1 - e1.x));
+        __syncwarp();
+        // the query's own slot
+        int jself = -1;
+        if (!SELF) {
+            int pre = 0;
+            for (int i = 0; i < nseg; i++) {
+                const int2 g = seg[i];
+                const int64_t j = qpos - g.y;
+                if (j >= pre && j < g.x) jself = (int)j;
+                pre = g.x;
+            }
+        }
+        int r = 0;
+        int2 sg = seg[0];
+        float4 cp[2], cq[2];
+        auto fetch = [&](int jb) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int j = jb + 32 * i;
+                cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end: far outside the cutoff
+                cq[i] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+                if (j >= T) continue;
+                while (j >= sg.x) sg = seg[++r];
+                const float4* rec = reinterpret_cast<const float4*>(pts + (j + sg.y));
+                cp[i] = rec[0];
+                cq[i] = rec[1];  // wk, k2h, k2l, hh
+            }
+        };
+        auto put = [&](int buf) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                cand[buf][0][lane + 32 * i] = cp[i].x;
+                cand[buf][1][lane + 32 * i] = cp[i].y;
+                cand[buf][2][lane + 32 * i] = cp[i].z;
+                cand[buf][3][lane + 32 * i] = cp[i].w;
+                cand[buf][4][lane + 32 * i] = cq[i].x;
+                if (VARH) {
+                    cand[buf][kComp - 2][lane + 32 * i] = cq[i].y;
+                    cand[buf][kComp - 1][lane + 32 * i] = cq[i].z;
                 }
             }
-            __syncthreads();
-            if (s_span[1] < 0) continue;  // no bin of the row reaches the group (uniform)
-            lo = bx0 + s_span[0];
-            hi = bx0 + s_span[1];
-        }
-        const int64_t sb = bin_start[by * nbx + lo], se = bin_start[by * nbx + hi + 1];
-        for (int64_t base = sb; base < se; base += kPdB) {
-            const int m = (int)mgk_min64(kPdB, se - base);
-            __syncthreads();
-            if (tid < m) st[tid] = pts[base + tid];
-            __syncthreads();
-            if (!qv) continue;
+        };
+        int buf = 0;
+        fetch(lane);
+        put(0);
+        __syncwarp();
+        for (int j = 0; j < T; j += kPdB) {
+            const int m = min(kPdB, T - j);
+            const bool more = j + kPdB < T;
+            if (more) fetch(j + kPdB + lane);
             float part = 0.0f;
-#pragma unroll kPdUnroll
-            for (int t = 0; t < m; t++) {
-                const MgkPt p = st[t];
-                const float dxh = __fsub_rn(p.xh, q.xh), dyh = __fsub_rn(p.yh, q.yh);
-                const float lim = VARH ? __fmaf_rn(9.0f * p.hh, 1.00001f, far_add) : far2;
-                if (__fmaf_rn(dxh, dxh, __fmul_rn(dyh, dyh)) > lim) continue;
-                const float dx = __fadd_rn(__fsub_rn(p.xh, q.xh), __fsub_rn(p.xl, q.xl));
-                const float dy = __fadd_rn(__fsub_rn(p.yh, q.yh), __fsub_rn(p.yl, q.yl));
-                const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                const float cf = VARH ? 9.0f * p.hh : cutf;
-                bool in = d2 < cf;
-                if (fabsf(d2 - cf) <= cf * 4e-6f)  // near the cutoff: the oracle's FP64 decision
-                    in = mgk_d2_exact(qx, qy, p.xh + p.xl, p.yh + p.yl) < (VARH ? MGK_CUT * (double)p.hh : cut);
-                if (!SELF && base + t == qpos) in = false;
-                if (in) {
-                    const float a = VARH ? __fmaf_rn(d2, p.k2h, __fmul_rn(d2, p.k2l))
-                                         : __fmaf_rn(d2, k2h, __fmul_rn(d2, k2l));
-                    part = __fmaf_rn(mgk_exp2_neg_poly(a), p.wk, part);
-                    cnt++;
+#pragma unroll 1
+            for (int t = 0; t < m; t += kPdTrip) {
+                // x < 0: inside the cutoff; the term is p times the weight ws
+                float p[kPdTrip], x[kPdTrip], ws[kPdTrip];
+#pragma unroll
+                for (int u = 0; u < kPdTrip; u += 2) {
+                    auto at = [&](int k) { return *reinterpret_cast<const f2*>(&cand[buf][k][t + u]); };
+                    const f2 dx = f2_add(f2_sub(at(0), qxh), f2_sub(at(2), qxl));
+                    const f2 dy = f2_add(f2_sub(at(1), qyh), f2_sub(at(3), qyl));
+                    const f2 d2 = f2_fma(dx, dx, f2_mul(dy, dy));
+                    const f2 a = f2_fma(d2, VARH ? at(kComp - 2) : k2hc, f2_mul(d2, VARH ? at(kComp - 1) : k2lc));
+                    f2_get(f2_sub(a, cut2), x[u], x[u + 1]);
+                    const f2 m1 = f2_sub(f2_sub(magic, a), magic);  // -n, a = n + g
+                    float g0, g1, n0, n1;
+                    f2_get(f2_add(a, m1), g0, g1);
+                    f2_get(m1, n0, n1);
+                    p[u] = mgk_exp2_neg_frac(g0);
+                    p[u + 1] = mgk_exp2_neg_frac(g1);
+                    f2_get(f2_mul(at(4), f2_make(mgk_ex2(n0), mgk_ex2(n1))), ws[u], ws[u + 1]);
+                }
+                const int ts = jself - (j + t);  // the query's own place in the trip, if in it
+                float near = fabsf(x[0]);
+#pragma unroll
+                for (int u = 1; u + 1 < kPdTrip; u += 2) near = mgk_min3(near, fabsf(x[u]), fabsf(x[u + 1]));
+                near = fminf(near, fabsf(x[kPdTrip - 1]));
+                if (near <= kPdBand || (unsigned)ts < (unsigned)kPdTrip) {
+#pragma unroll
+                    for (int u = 0; u < kPdTrip; u++) {
+                        if (fabsf(x[u]) <= kPdBand) {  // near the cutoff: the oracle's FP64 decision
+                            int i = 0;
+                            while (j + t + u >= seg[i].x) i++;
+                            const MgkPt cc = pts[j + t + u + seg[i].y];
+                            const double cut = MGK_CUT * (VARH ? (double)cc.hh : h2);
+                            x[u] = mgk_d2_exact(qx, qy, cc.xh + cc.xl, cc.yh + cc.yl) < cut ? -1.0f : 1.0f;
+                        }
+                        if (u == ts) x[u] = 1.0f;  // the query itself
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kPdTrip; u++) {
+                    if (x[u] < 0.0f) part = __fmaf_rn(p[u], ws[u], part);
+                    cnt += __float_as_uint(x[u]) >> 31;
                 }
             }
             const float y = part - c;
             const float tt = s + y;
             c = (tt - s) - y;
             s = tt;
+            if (more) put(buf ^ 1);
+            __syncwarp();  // this batch has been scanned, the next one is in place
+            buf ^= 1;
+        }
+        nseg = 0;
+    };
+    for (int by = by0 + (int)blockIdx.y; by <= by1; by += (int)gridDim.y) {
+        // a point of the row can be in reach of the box only within
+        // sqrt(reach^2 - dy^2) of it, dy the rows' distance (a lower bound)
+        const double rlo = oy + (double)by * side, rhi = rlo + side;
+        const double ddy = fmax(0.0, fmax(rlo - (double)mxy, (double)mny - rhi)) * (1.0 - 1e-9);
+        const double rr = reach * reach - ddy * ddy;
+        if (!(rr >= 0.0)) continue;
+        const double hw = sqrt(rr) * (1.0 + 1e-9) + 1e-9 * reach;
+        const double f0 = fmax(0.0, floor(((double)mnx - hw - ox) * inv_side));
+        const double f1 = fmin((double)(nbx - 1), floor(((double)mxx + hw - ox) * inv_side));
+        if (!(f0 <= f1)) continue;
+        const int b0 = (int)f0, b1 = (int)f1;
+        const int32_t* bs = bin_start + (int64_t)by * nbx;
+        if constexpr (!VARH) {
+            const int pos = bs[b0], len = bs[b1 + 1] - pos;
+            if (len == 0) continue;
+            if (nseg == kPdSeg) scan();
+            if (lane == 0) seg[nseg] = make_int2(len, pos);
+            nseg++;
+        } else {
+            for (int bx = b0; bx <= b1; bx += 32) {
+                bool ok = false;
+                int pos = 0, end = 0;
+                if (bx + lane <= b1) {
+                    const float r2 = bin_r2[(int64_t)by * nbx + bx + lane];
+                    const double rx0 = ox + (double)(bx + lane) * side, rx1 = rx0 + side;
+                    const double ddx = fmax(0.0, fmax(rx0 - (double)mxx, (double)mnx - rx1));
+                    // a margin over the bin edges' rounding and the float h^2; r2 < 0: an empty bin
+                    ok = r2 >= 0.0f && ddx * ddx + ddy * ddy <= (double)r2 * (1.0 + 1e-5) + 1e-6 * side * side;
+                    if (ok) {
+                        pos = bs[bx + lane];
+                        end = bs[bx + lane + 1];
+                    }
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, ok);
+                const unsigned first = m & ~(m << 1);  // the lanes whose bin begins a run
+                const int nrun = __popc(first);
+                if (nseg + nrun > kPdSeg) scan();
+                // the run's last bin: before the first clear bit above the lane's
+                const unsigned gap = ~(m >> lane);
+                const int last = gap ? lane + __ffs(gap) - 2 : 31;
+                end = __shfl_sync(0xffffffffu, end, last & 31);
+                if ((first >> lane) & 1u) seg[nseg + __popc(first & lt)] = make_int2(end - pos, pos);
+                nseg += nrun;
+            }
         }
     }
+    if (nseg) scan();
     if (qv) psum[(int64_t)blockIdx.y * n + qpos] = (double)s - (double)c;
     if (evals) {
+        if (!qv) cnt = 0;
         for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
         if (lane == 0 && cnt) atomicAdd(evals, (unsigned long long)cnt);
     }
 }
 
+constexpr int kPdC = 128;  // threads of the combining kernel
+
 // den[perm[q]] = the nsplit partials of query q summed in order (times
 // 1/(h^2 TWO_PI) for a fixed h), and part[CTA] = the CTA's fixed-order sum of
 // log(max(den, floor_v)).
-__global__ void __launch_bounds__(kPdQ) k_pd_combine(int64_t n, int nsplit, const double* __restrict__ psum,
+__global__ void __launch_bounds__(kPdC) k_pd_combine(int64_t n, int nsplit, const double* __restrict__ psum,
                                                      const int32_t* __restrict__ perm, bool varh, double h2,
                                                      double floor_v, double* __restrict__ den,
                                                      double* __restrict__ part) {
-    __shared__ double s_lg[kPdQ / 32];
+    __shared__ double s_lg[kPdC / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t q = (int64_t)blockIdx.x * kPdQ + tid;
+    const int64_t q = (int64_t)blockIdx.x * kPdC + tid;
     double lg = 0.0;
     if (q < n) {
         double v = 0.0;
@@ -204,7 +307,7 @@ __global__ void __launch_bounds__(kPdQ) k_pd_combine(int64_t n, int nsplit, cons
     __syncthreads();
     if (tid == 0) {
         double t = 0.0;
-        for (int i = 0; i < kPdQ / 32; i++) t += s_lg[i];
+        for (int i = 0; i < kPdC / 32; i++) t += s_lg[i];
         part[blockIdx.x] = t;
     }
 }
@@ -274,10 +377,11 @@ int point_density(mgk_ctx* c, const mgk_index* idx, bool self, double* d_den, do
         MGK_CHECK_CUDA(c, cudaMemsetAsync(d_logsum, 0, sizeof(double), s));
         return MGK_OK;
     }
-    // bin rows split over enough CTAs to give every SM about 8 of them
-    const int nsplit = (int)std::min<int64_t>(8, std::max<int64_t>(1, (8 * (int64_t)c->sm_count + g - 1) / g));
+    // bin rows split over enough warps to keep every SM busy to the end
+    const int nsplit = (int)std::min<int64_t>(24, std::max<int64_t>(1, (kPdWarps * (int64_t)c->sm_count + g - 1) / g));
+    const int64_t gc = (idx->n + kPdC - 1) / kPdC;
     const int64_t nbins = idx->varh ? idx->nbx * idx->nby : 0;
-    const size_t b_part = sizeof(double) * (size_t)g, b_r2 = sizeof(float) * (size_t)std::max<int64_t>(nbins, 1);
+    const size_t b_part = sizeof(double) * (size_t)gc, b_r2 = sizeof(float) * (size_t)std::max<int64_t>(nbins, 1);
     const size_t b_psum = sizeof(double) * (size_t)idx->n * (size_t)nsplit;
     double *part = nullptr, *psum = nullptr;
     float* r2 = nullptr;
@@ -297,22 +401,22 @@ int point_density(mgk_ctx* c, const mgk_index* idx, bool self, double* d_den, do
         k_bin_reach2<<<(unsigned)((nbins + 255) / 256), 256, 0, s>>>(nbins, idx->bin_start, idx->pts, r2);
         k_point_density<true, false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
                                                            idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                           idx->h2, r2, std::ldexp(1.0, -idx->qexp), psum,
+                                                           idx->h2, r2, psum,
                                                            pair_count(c));
     } else if (self) {
         k_point_density<false, true><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
                                                            idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                           idx->h2, nullptr, std::ldexp(1.0, -idx->qexp), psum,
+                                                           idx->h2, nullptr, psum,
                                                            pair_count(c));
     } else {
         k_point_density<false, false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
                                                             idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                            idx->h2, nullptr, std::ldexp(1.0, -idx->qexp), psum,
+                                                            idx->h2, nullptr, psum,
                                                             pair_count(c));
     }
-    k_pd_combine<<<(unsigned)g, kPdQ, 0, s>>>(idx->n, nsplit, psum, idx->perm, idx->varh, idx->h2, floor_v, d_den,
+    k_pd_combine<<<(unsigned)gc, kPdC, 0, s>>>(idx->n, nsplit, psum, idx->perm, idx->varh, idx->h2, floor_v, d_den,
                                               part);
-    k_sum_parts<<<1, 256, 0, s>>>(g, part, d_logsum);
+    k_sum_parts<<<1, 256, 0, s>>>(gc, part, d_logsum);
     const cudaError_t e = cudaGetLastError();
     // pooled blocks: a later allocation of them is ordered on the same stream
     mgk_free(c, part, b_part);

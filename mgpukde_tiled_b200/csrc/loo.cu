@@ -93,43 +93,6 @@ struct LooParams {
     unsigned long long* evals;
 };
 
-// ---- two FP32 values in a 64-bit register (sm_100 f32x2; each half is
-// rounded as the scalar operation is)
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2_dup(float a) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
-    return r;
-}
-__device__ __forceinline__ f2 f2_make(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_get(f2 v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -142,33 +105,11 @@ __device__ __forceinline__ double loo_log(double sum, double h2) {
     return log(loo > fl ? loo : fl);
 }
 
-// 2^-g for g in [-1/2, 1/2]: a degree-6 polynomial, fitted to 2^-g by least
-// squares on Chebyshev nodes with the mean error held where the rounding of
-// the scan's terms leaves none, each coefficient rounded to float before the
-// next ones are fitted (truncation 3.3e-9 relative; the weighted mean error of
-// the terms over the cutoff's disc is 1e-12, that of a degree-8 Taylor form on
-// an unscaled distance -6e-11).  Scalar with immediate coefficients: a packed
-// FMA with three register pairs runs at 3.3 cycles instead of 2.
-__device__ __forceinline__ float exp2_neg_frac(float g) {
-    float p = __fmaf_rn(0.00015285507834050804f, g, -0.001339130220003426f);
-    p = __fmaf_rn(p, g, 0.009618666023015976f);
-    p = __fmaf_rn(p, g, -0.055503588169813156f);
-    p = __fmaf_rn(p, g, 0.24022646248340607f);
-    p = __fmaf_rn(p, g, -0.6931471824645996f);
-    return __fmaf_rn(p, g, 1.0f);
-}
-
 // v on a grid of step q = m / (1.5 2^52) (hi) and the remainder (lo)
 __device__ __forceinline__ void split_at(double v, double m, float& hi, float& lo) {
     const double t = __dsub_rn(__dadd_rn(v, m), m);
     hi = (float)t;
     lo = (float)__dsub_rn(v, t);
-}
-
-__device__ __forceinline__ float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
 }
 
 // Level and processing order of every h (one CTA; nh is small).
@@ -208,7 +149,7 @@ __global__ void k_loo_weights(LooParams P) {
 //  - distances, exponents and range reduction two candidates at a time
 //    (f32x2), with the coordinates scaled so that the squared distance is the
 //    exponent (two packed operations fewer per pair of candidates);
-//  - the polynomial scalar, its coefficients immediates (see exp2_neg_frac);
+//  - the polynomial scalar, its coefficients immediates (see mgk_exp2_neg_frac);
 //  - pair counts from sign bits: a predicated increment costs two instructions;
 //  - a warp its own work item: no CTA barriers, and rows cut to the disc
 //    around 32 queries instead of the square around 128 (1.38 tests a pair).
@@ -459,14 +400,14 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
                         float g0, g1, n0, n1;
                         f2_get(f2_add(a, n), g0, g1);
                         f2_get(n, n0, n1);
-                        p[u] = exp2_neg_frac(g0);
-                        p[u + 1] = exp2_neg_frac(g1);
+                        p[u] = mgk_exp2_neg_frac(g0);
+                        p[u + 1] = mgk_exp2_neg_frac(g1);
                         f2_get(f2_mul(w, f2_make(mgk_ex2(n0), mgk_ex2(n1))), ws[u], ws[u + 1]);
                     }
                     const int ts = jself - (j + t);  // the query's own place in the trip, if in it
                     float near = fabsf(x[0]);
 #pragma unroll
-                    for (int u = 1; u + 1 < kLooTrip; u += 2) near = min3(near, fabsf(x[u]), fabsf(x[u + 1]));
+                    for (int u = 1; u + 1 < kLooTrip; u += 2) near = mgk_min3(near, fabsf(x[u]), fabsf(x[u + 1]));
                     near = fminf(near, fabsf(x[kLooTrip - 1]));
                     if (near <= kLooBand || (unsigned)ts < (unsigned)kLooTrip) {
 #pragma unroll

@@ -198,6 +198,65 @@ __device__ __forceinline__ float mgk_exp2_neg_poly(float a) {
     return __fmul_rn(p, __int_as_float((127 - (int)n) << 23));
 }
 
+// Two FP32 values in a 64-bit register (sm_100 f32x2; each half is
+// rounded as the scalar operation is)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_dup(float a) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_get(f2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// 2^-g for g in [-1/2, 1/2]: a degree-6 polynomial, fitted to 2^-g by least
+// squares on Chebyshev nodes with the mean error held where the rounding of
+// the scan's terms leaves none, each coefficient rounded to float before the
+// next ones are fitted (truncation 3.3e-9 relative; the weighted mean error of
+// the terms over the cutoff's disc is 1e-12, that of a degree-8 Taylor form on
+// an unscaled distance -6e-11).  Scalar with immediate coefficients: a packed
+// FMA with three register pairs runs at 3.3 cycles instead of 2.
+__device__ __forceinline__ float mgk_exp2_neg_frac(float g) {
+    float p = __fmaf_rn(0.00015285507834050804f, g, -0.001339130220003426f);
+    p = __fmaf_rn(p, g, 0.009618666023015976f);
+    p = __fmaf_rn(p, g, -0.055503588169813156f);
+    p = __fmaf_rn(p, g, 0.24022646248340607f);
+    p = __fmaf_rn(p, g, -0.6931471824645996f);
+    return __fmaf_rn(p, g, 1.0f);
+}
+
+__device__ __forceinline__ float mgk_min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // Cell centres as the reference computes them (Utilities.h:13-14): double
 // arithmetic, stored to float.
 __device__ __host__ __forceinline__ float mgk_cell_x(double xll, double cs, int64_t col) {
