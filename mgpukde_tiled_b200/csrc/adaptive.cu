@@ -363,6 +363,7 @@ int count_end(mgk_ctx* c) {
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(c->h_counter + 5, c->d_counter + 5, 2 * sizeof(unsigned long long),
                                       cudaMemcpyDeviceToHost, c->stream));
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (const int st = mgk_sort_check(c)) return st;
     c->last_loo_evals[0] = (int64_t)c->h_counter[5];
     c->last_loo_evals[1] = (int64_t)c->h_counter[6];
     MGK_CHECK_CUDA(c, cudaEventElapsedTime(&c->last_loo_ms, c->ev_a, c->ev_b));
@@ -439,6 +440,7 @@ struct PilotCache {
     double* buf[kEntries] = {};  // den0[max(n, 1)], then the log sum
     uint64_t last[kEntries] = {};
     uint64_t tick = 0;
+    mgk_extent extent;  // of the points (any h)
     size_t bytes() const { return sizeof(double) * (size_t)(std::max<int64_t>(n, 1) + 1); }
     ~PilotCache() {
         for (int i = 0; i < kEntries; i++)
@@ -471,7 +473,7 @@ int pilot_density(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, Pilot
     if (st == MGK_OK) {
         p->has_ew = true;
         mgk_index* idx = nullptr;
-        if ((st = mgk_index_build(c, p, h, 0.0f, &idx)) == MGK_OK) {  // h > 0: fixed-h index
+        if ((st = mgk_index_build_async(c, p, h, 0.0f, &pc.extent, &idx)) == MGK_OK) {  // h > 0: fixed-h index
             st = point_density(c, idx, true, den, 0.0, den + std::max<int64_t>(p->n, 1));
             mgk_index_destroy(idx);
         }
@@ -509,7 +511,7 @@ int loglik_adaptive(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, flo
     // per-point h; bins of 0.75 h (the geometric mean of hs is h), not of the
     // widest h, so that the per-bin reach can cut the window down
     mgk_index* idx = nullptr;
-    if ((st = mgk_index_build(c, p, 0.0f, 0.75f * h, &idx))) return st;
+    if ((st = mgk_index_build_async(c, p, 0.0f, 0.75f * h, nullptr, &idx))) return st;
     st = point_density(c, idx, false, d_den, (double)MGK_EPS_DENSITY_F, d_scal + 1);
     mgk_index_destroy(idx);
     if (st) return st;
@@ -553,7 +555,8 @@ int mgk_loglik_adaptive(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h,
         PilotCache pc;
         pc.c = c;
         pc.n = p->n;
-        st = count_begin(c);
+        st = mgk_points_extent(c, p, false, &pc.extent);
+        if (st == MGK_OK) st = count_begin(c);
         if (st == MGK_OK) st = loglik_adaptive(c, p, r, h, alpha, d_den, d_scal, logl, pc);
         if (st == MGK_OK) st = count_end(c);
     }
@@ -603,7 +606,8 @@ int mgk_adaptive_bandwidths(mgk_ctx* c, mgk_points* p, const mgk_raster* r, floa
         if (s2 == MGK_OK && last != 3) s2 = ll(h0, alpha0 - stepA, &L[4]);
         return s2;
     };
-    st = count_begin(c);
+    st = mgk_points_extent(c, p, false, &pc.extent);
+    if (st == MGK_OK) st = count_begin(c);
     if (st == MGK_OK) st = around(-1);
     float Lm = L[0];
     const float sH = stepH / 10, sA = stepA / 10;

@@ -122,6 +122,20 @@ void mgk_free(mgk_ctx* ctx, void* p, size_t bytes) {
     ctx->pool.emplace(size_class(bytes ? bytes : 16), p);
 }
 
+int mgk_index_build_async(mgk_ctx* c, const mgk_points* p, float h, float bin_size, const mgk_extent* extent,
+                          mgk_index** out) {
+    if (!c || !p || !out) return mgk_fail(c, MGK_ERR_INVALID, "index_build: bad arguments");
+    mgk_index* idx = new (std::nothrow) mgk_index();
+    if (!idx) return MGK_ERR_INVALID;
+    const int st = mgk_launch_index_build(c, p, h, bin_size, extent, idx);
+    if (st) {
+        mgk_index_destroy(idx);
+        return st;
+    }
+    *out = idx;
+    return MGK_OK;
+}
+
 extern "C" {
 
 const char* mgk_status_string(int status) {
@@ -167,10 +181,13 @@ int mgk_ctx_create(int device, uint64_t hbm_budget_bytes, mgk_ctx** out) {
         cudaMalloc(&c->d_sum, 256 * sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&c->h_counter, 8 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMallocHost(&c->h_sum, 256 * sizeof(double)) != cudaSuccess ||
+        cudaHostAlloc((void**)&c->h_map, 16384, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&c->d_map, c->h_map, 0) != cudaSuccess ||
         cudaEventCreate(&c->ev_a) != cudaSuccess || cudaEventCreate(&c->ev_b) != cudaSuccess) {
         mgk_ctx_destroy(c);
         return MGK_ERR_CUDA;
     }
+    memset(c->h_map, 0, 16384);
     *out = c;
     return MGK_OK;
 }
@@ -184,6 +201,7 @@ int mgk_ctx_destroy(mgk_ctx* c) {
     if (c->d_sum) cudaFree(c->d_sum);
     if (c->h_counter) cudaFreeHost(c->h_counter);
     if (c->h_sum) cudaFreeHost(c->h_sum);
+    if (c->h_map) cudaFreeHost(c->h_map);
     for (int i = 0; i < mgk_ctx::kStageSlots; i++)
         if (c->h_stage[i]) cudaFreeHost(c->h_stage[i]);
     if (c->ev_a) cudaEventDestroy(c->ev_a);
@@ -541,10 +559,12 @@ int mgk_edge_weights_unit(mgk_ctx* c, mgk_points* p) {
 
 // ------------------------------------------------------------------ index --
 int mgk_index_build(mgk_ctx* c, const mgk_points* p, float h, float bin_size, mgk_index** out) {
-    if (!c || !p || !out) return mgk_fail(c, MGK_ERR_INVALID, "index_build: bad arguments");
-    mgk_index* idx = new (std::nothrow) mgk_index();
-    if (!idx) return MGK_ERR_INVALID;
-    int st = mgk_launch_index_build(c, p, h, bin_size, idx);
+    mgk_index* idx = nullptr;
+    int st = mgk_index_build_async(c, p, h, bin_size, nullptr, &idx);
+    if (st) return st;
+    // the index is complete on return: the points may go, and other streams may read it
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    st = e != cudaSuccess ? mgk_cuda_fail(c, e, "index build") : mgk_sort_check(c);
     if (st) {
         mgk_index_destroy(idx);
         return st;
@@ -1095,7 +1115,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     // the first tile's float mask travels while the points are prepared (a
     // packed band's bits follow the counts: the packer may still be at work)
     if (st == MGK_OK && !packed && (ce = mask_in(0)) != cudaSuccess) st = mgk_cuda_fail(c, ce, "kde_raster mask");
-    if (st == MGK_OK) st = mgk_index_build(c, p, hfix, 0.0f, &idx);
+    if (st == MGK_OK) st = mgk_index_build_async(c, p, hfix, 0.0f, nullptr, &idx);
     if (st == MGK_OK) {
         if (edge_correction) {
             // distances exact up to 3 h_max: all the edge-weight short-circuit reads
@@ -1299,7 +1319,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         ce = cudaMemcpy(c->h_counter + 4, c->d_counter + 4, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
         if (ce != cudaSuccess) st = mgk_cuda_fail(c, ce, "kde_raster counters");
         else if (c->h_counter[7]) st = mgk_fail(c, MGK_ERR_TIMEOUT, "density: a shared-memory staging wait timed out");
-        else ev_den = (int64_t)c->h_counter[4];
+        else if ((st = mgk_sort_check(c)) == MGK_OK) ev_den = (int64_t)c->h_counter[4];
     }
     for (int i = 0; i < kDepth; i++) {
         if (d_out[i]) mgk_free(c, d_out[i], tb);

@@ -8,9 +8,10 @@
 // contiguous range: a raster tile's candidates within 3h are a handful of
 // ranges, one per bin row.
 //
-// The sort is a stable LSD radix sort (8-bit digits) of the bin id, so the
-// order inside a bin is the input order and every build is bitwise
-// reproducible (the density sums are order-dependent in FP32).
+// The sort is a stable LSD radix sort of the bin id (digits of up to 9 bits,
+// one kernel per digit), so the order inside a bin is the input order and
+// every build is bitwise reproducible (the density sums are order-dependent
+// in FP32).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -22,69 +23,78 @@
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 32;  // per thread per tile
-constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kMaxDigits = 512;   // digits of up to 9 bits: 18-bit bin ids sort in two passes
+constexpr int kMaxPasses = 4;     // 32-bit keys
+constexpr long long kSortSpin = 1ll << 24;
+constexpr int kExtentCtas = 512;  // their words fit the context's mapped page
 
 __device__ __forceinline__ unsigned f2ord(float f) {
     unsigned u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__device__ __forceinline__ float ord2f(unsigned u) {
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-
-// bbox[0..3] = ordered-int min x, min y, max x, max y
-__global__ void k_bbox(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
-                       unsigned* bbox) {
-    unsigned mnx = 0xffffffffu, mny = 0xffffffffu, mxx = 0, mxy = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        unsigned ox = f2ord(x[i]), oy = f2ord(y[i]);
-        mnx = min(mnx, ox);
-        mny = min(mny, oy);
-        mxx = max(mxx, ox);
-        mxy = max(mxy, oy);
+// The points' extent (and largest h): each CTA's ordered-integer minima and
+// maxima (min x, min y, max x, max y, max h) into its words of mapped host
+// memory, so that no copy goes through a copy engine.
+__global__ void __launch_bounds__(256) k_extent(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
+                                                const float* __restrict__ h, unsigned* out) {
+    __shared__ unsigned sh[8][5];
+    unsigned v[5] = {0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned ox = f2ord(x[i]), oy = f2ord(y[i]);
+        v[0] = min(v[0], ox);
+        v[1] = min(v[1], oy);
+        v[2] = max(v[2], ox);
+        v[3] = max(v[3], oy);
+        if (h) v[4] = max(v[4], f2ord(h[i]));
     }
-    for (int o = 16; o; o >>= 1) {
-        mnx = min(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-        mny = min(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-        mxx = max(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-        mxy = max(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&bbox[0], mnx);
-        atomicMin(&bbox[1], mny);
-        atomicMax(&bbox[2], mxx);
-        atomicMax(&bbox[3], mxy);
-    }
-}
-
-__global__ void k_bin_keys(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
-                           double ox, double oy, double inv_side, int64_t nbx, int64_t nby,
-                           unsigned* __restrict__ keys, int32_t* __restrict__ vals) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int64_t bx = (int64_t)floor(((double)x[i] - ox) * inv_side);
-    int64_t by = (int64_t)floor(((double)y[i] - oy) * inv_side);
-    bx = bx < 0 ? 0 : (bx >= nbx ? nbx - 1 : bx);
-    by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
-    keys[i] = (unsigned)(by * nbx + bx);
-    vals[i] = (int32_t)i;
-}
-
-// Per-tile histogram of one 8-bit digit: counts[d * ntiles + tile].
-__global__ void __launch_bounds__(kSortThreads) k_radix_hist(int64_t n, const unsigned* __restrict__ keys,
-                                                             int shift, int ntiles, unsigned* __restrict__ counts) {
-    __shared__ unsigned hist[256];
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int k = 0; k < kSortItems; k++) {
-        int64_t i = base + (int64_t)k * kSortThreads + threadIdx.x;
-        if (i < n) atomicAdd(&hist[(keys[i] >> shift) & 0xff], 1u);
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        v[k] = k < 2 ? __reduce_min_sync(0xffffffffu, v[k]) : __reduce_max_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][k] = v[k];
     }
     __syncthreads();
-    counts[(size_t)threadIdx.x * ntiles + blockIdx.x] = hist[threadIdx.x];
+    if (threadIdx.x < 5) {
+        const int k = threadIdx.x;
+        unsigned m = sh[0][k];
+        for (int w = 1; w < 8; w++) m = k < 2 ? min(m, sh[w][k]) : max(m, sh[w][k]);
+        out[blockIdx.x * 5 + k] = m;
+    }
+}
+
+// Keys of a sort and the histograms of all their digits (pass p: bits
+// [p db, (p + 1) db)) in one reading.
+template <typename KeyOf>
+__device__ __forceinline__ void keys_and_hist(int64_t n, const KeyOf& key_of, int db, int passes,
+                                              unsigned* __restrict__ keys, unsigned* __restrict__ hist) {
+    __shared__ unsigned sh[kMaxPasses * kMaxDigits];
+    const int nd = 1 << db;
+    for (int d = threadIdx.x; d < passes * nd; d += blockDim.x) sh[d] = 0;
+    __syncthreads();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned k = key_of(i);
+        keys[i] = k;
+        for (int p = 0; p < passes; p++) atomicAdd(&sh[p * nd + ((k >> (p * db)) & (nd - 1))], 1u);
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < passes * nd; d += blockDim.x)
+        if (sh[d]) atomicAdd(&hist[d], sh[d]);
+}
+
+__global__ void __launch_bounds__(256) k_bin_keys(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
+                                                  double ox, double oy, double inv_side, int64_t nbx, int64_t nby,
+                                                  int db, int passes, unsigned* __restrict__ keys,
+                                                  unsigned* __restrict__ hist) {
+    keys_and_hist(
+        n,
+        [&](int64_t i) {
+            int64_t bx = (int64_t)floor(((double)x[i] - ox) * inv_side);
+            int64_t by = (int64_t)floor(((double)y[i] - oy) * inv_side);
+            bx = bx < 0 ? 0 : (bx >= nbx ? nbx - 1 : bx);
+            by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
+            return (unsigned)(by * nbx + bx);
+        },
+        db, passes, keys, hist);
 }
 
 // Exclusive scan of `len` counts in one CTA of 1024 threads (chunked).
@@ -111,68 +121,190 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(unsigned* __restrict__ 
     }
 }
 
-// Stable scatter of one digit pass.  Items of a tile are taken in rounds of
-// 256 (round-major, thread-minor = input order); inside a round the rank of an
-// item among equal digits is its warp rank (match_any) plus the counts of the
-// same digit in lower warps and in earlier rounds.
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(
-    int64_t n, const unsigned* __restrict__ keys_in, const int32_t* __restrict__ vals_in,
-    unsigned* __restrict__ keys_out, int32_t* __restrict__ vals_out, int shift, int ntiles,
-    const unsigned* __restrict__ offsets) {
-    __shared__ unsigned warp_cnt[kSortThreads / 32][256];
-    __shared__ unsigned warp_pre[kSortThreads / 32][256];
-    __shared__ unsigned tile_base[256];
+// One digit of the stable sort in one kernel.  Tiles of 256 IPT items are
+// handed out in order by a counter; a tile ranks its items in registers (each
+// warp its own run of 32 IPT, match_any per round), publishes its digit
+// counts, and adds up those of the tiles before it, which are all running or
+// done, from their published counts or sums (state in the top two bits of a
+// word: 1 counts, 2 sums including all earlier tiles).  A pass reads and
+// writes each item once; the earlier form (a histogram kernel, a scan of all
+// tiles' counts in one CTA, a scatter in rounds of 256 items with five
+// barriers each, tiles of 8,192) took 85 us a pass on 10^6 points and 29 us on
+// 2,000, where one CTA did everything; this takes 36 and 6 us (an index build
+// 289 -> 144 and 99 -> 54 us).  vals_in null: the values are the items'
+// indexes.
+template <int IPT, typename W>
+__global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, const unsigned* __restrict__ keys_in,
+                                                             const int32_t* __restrict__ vals_in,
+                                                             unsigned* __restrict__ keys_out,
+                                                             int32_t* __restrict__ vals_out, int shift, int db,
+                                                             const unsigned* __restrict__ hist, W* look,
+                                                             unsigned* tick, unsigned* err) {
+    constexpr int kTop = sizeof(W) * 8 - 2;
+    constexpr W kVal = ((W)1 << kTop) - 1;
+    __shared__ unsigned cnt[kSortWarps][kMaxDigits];  // a warp's digit counts, then its offsets in the tile
+    __shared__ unsigned base[kMaxDigits];             // items of smaller digits, then the tile's first place
+    __shared__ unsigned wsum[kSortWarps];
+    __shared__ unsigned s_tile;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    tile_base[t] = offsets[(size_t)t * ntiles + blockIdx.x];
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int k = 0; k < kSortItems; k++) {
-        for (int w = 0; w < kSortThreads / 32; w++) warp_cnt[w][t] = 0;
-        __syncthreads();
-        const int64_t i = base + (int64_t)k * kSortThreads + t;
-        const bool valid = i < n;
-        unsigned key = 0, d = 0;
-        int32_t val = 0;
-        if (valid) {
-            key = keys_in[i];
-            val = vals_in[i];
-            d = (key >> shift) & 0xff;
+    const int nd = 1 << db;
+    if (t == 0) s_tile = atomicAdd(tick, 1u);
+    for (int d = t; d < nd; d += kSortThreads)
+        for (int w = 0; w < kSortWarps; w++) cnt[w][d] = 0;
+    // exclusive scan of the digits' counts (one or two digits per thread)
+    const int per = nd > kSortThreads ? 2 : 1;
+    unsigned h0 = t * per < nd ? hist[t * per] : 0u, h1 = per == 2 ? hist[2 * t + 1] : 0u;
+    unsigned sum = h0 + h1;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    if (lane == 31) wsum[wid] = sum;
+    __syncthreads();
+    for (int w = 0; w < wid; w++) sum += wsum[w];
+    if (t * per < nd) {
+        base[t * per] = sum - h0 - h1;
+        if (per == 2) base[2 * t + 1] = sum - h1;
+    }
+    const unsigned tile = s_tile;
+    const int64_t i0 = (int64_t)tile * (kSortThreads * IPT) + wid * (32 * IPT) + lane;
+    unsigned key[IPT], rank[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; k++) key[k] = i0 + 32 * k < n ? keys_in[i0 + 32 * k] : 0u;
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        const bool valid = i0 + 32 * k < n;
+        const unsigned d = valid ? (key[k] >> shift) & (nd - 1) : (unsigned)kMaxDigits;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned before = valid ? cnt[wid][d] : 0u;
+        rank[k] = before + __popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+        if (valid && (peers >> lane) == 1u) cnt[wid][d] = before + __popc(peers);  // the last of the peers
+        __syncwarp();
+    }
+    __syncthreads();
+    volatile W* lk = look;
+    for (int d = t; d < nd; d += kSortThreads) {
+        unsigned run = 0;
+        for (int w = 0; w < kSortWarps; w++) {
+            const unsigned c = cnt[w][d];
+            cnt[w][d] = run;
+            run += c;
         }
-        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-        unsigned rank = 0;
-        if (valid) {
-            const unsigned peers = __match_any_sync(vmask, d);
-            rank = __popc(peers & ((1u << lane) - 1u));
-            if (rank == 0) warp_cnt[wid][d] = __popc(peers);
-        }
-        __syncthreads();
-        {
-            unsigned run = 0;
-            for (int w = 0; w < kSortThreads / 32; w++) {
-                warp_pre[w][t] = run;
-                run += warp_cnt[w][t];
+        lk[(size_t)tile * nd + d] = ((W)(tile ? 1 : 2) << kTop) | run;
+        unsigned prev = 0;
+        for (unsigned p = tile; p > 0;) {
+            p--;
+            W v = 0;
+            long long spin = 0;
+            while ((v = lk[(size_t)p * nd + d]) >> kTop == 0 && ++spin < kSortSpin) {
             }
-            warp_cnt[0][t] = run;  // round total for digit t (warp_cnt[0] reused)
+            if (v >> kTop == 0) *err = 1u;  // ran out: reported by the host, the places stay in range
+            prev += (unsigned)(v & kVal);
+            if (v >> kTop != 1) break;
         }
-        __syncthreads();
-        if (valid) {
-            const unsigned pos = tile_base[d] + warp_pre[wid][d] + rank;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
-        tile_base[t] += warp_cnt[0][t];
-        __syncthreads();
+        if (tile) lk[(size_t)tile * nd + d] = ((W)2 << kTop) | (W)(prev + run);
+        base[d] += prev;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        const int64_t i = i0 + 32 * k;
+        if (i >= n) continue;
+        const unsigned d = (key[k] >> shift) & (nd - 1);
+        const unsigned pos = base[d] + cnt[wid][d] + rank[k];
+        keys_out[pos] = key[k];
+        vals_out[pos] = vals_in ? vals_in[i] : (int32_t)i;
     }
 }
 
-// bin_start[b] = first sorted position whose key >= b  (b in [0, nbins]).
-__global__ void k_bin_starts(int64_t n, const unsigned* __restrict__ keys, int64_t nbins,
-                             int32_t* __restrict__ start) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i > n) return;
-    const int64_t prev = i > 0 ? (int64_t)keys[i - 1] : -1;
-    const int64_t cur = i < n ? (int64_t)keys[i] : nbins;
-    for (int64_t b = prev + 1; b <= cur; b++) start[b] = (int32_t)i;
+// Passes and digit bits of a sort of `bits`-bit keys; its scratch words.
+struct SortPlan {
+    int passes, db, ipt;
+    int64_t ntiles;
+    bool wide;  // counts of 2^30 items and more: 64-bit state words
+    size_t look_bytes() const { return (size_t)ntiles * ((size_t)1 << db) * (wide ? 8 : 4); }
+    size_t bytes() const {  // [digit counts | tile counters | state words], zeroed before the keys
+        return sizeof(unsigned) * (kMaxPasses * kMaxDigits + 8) + (size_t)passes * look_bytes();
+    }
+};
+
+SortPlan sort_plan(int64_t n, int bits) {
+    SortPlan P;
+    bits = std::max(bits, 1);
+    P.passes = (bits + 8) / 9;
+    P.db = (bits + P.passes - 1) / P.passes;
+    // Large tiles shorten the look back, small ones keep the SMs busy: 16, 4, 4
+    // items a thread instead took 161 us for 10^6 points (144 with 16) and 4, 1
+    // for 200,000 125 us (109 with 4).
+    P.ipt = n >= (1 << 19) ? 16 : n >= (1 << 16) ? 4 : 1;
+    P.ntiles = (n + (int64_t)kSortThreads * P.ipt - 1) / ((int64_t)kSortThreads * P.ipt);
+    P.wide = n >= (1ll << 30);
+    return P;
+}
+
+unsigned* sort_hist(void* scratch) { return static_cast<unsigned*>(scratch); }
+
+// Sorts (keys in ka, values = indexes) with the histograms already in the
+// scratch, through kb, vb and back; the sorted keys and values end in kb, vb
+// after an odd number of passes, else in ka, va.
+void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, unsigned* ka, int32_t* va, unsigned* kb, int32_t* vb,
+                 void* scratch, unsigned* err) {
+    unsigned* hist = sort_hist(scratch);
+    unsigned* tick = hist + kMaxPasses * kMaxDigits;
+    char* look = reinterpret_cast<char*>(tick + 8);
+    for (int p = 0; p < P.passes; p++) {
+        const unsigned* ki = p & 1 ? kb : ka;
+        const int32_t* vi = p == 0 ? nullptr : p & 1 ? vb : va;
+        unsigned* ko = p & 1 ? ka : kb;
+        int32_t* vo = p & 1 ? va : vb;
+        const unsigned* h = hist + p * (1 << P.db);
+        char* lk = look + (size_t)p * P.look_bytes();
+        const unsigned g = (unsigned)P.ntiles;
+        if (P.wide)
+            k_radix_pass<16, unsigned long long><<<g, kSortThreads, 0, s>>>(
+                n, ki, vi, ko, vo, p * P.db, P.db, h, reinterpret_cast<unsigned long long*>(lk), tick + p, err);
+        else if (P.ipt == 16)
+            k_radix_pass<16, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
+                                                                  reinterpret_cast<unsigned*>(lk), tick + p, err);
+        else if (P.ipt == 4)
+            k_radix_pass<4, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
+                                                                 reinterpret_cast<unsigned*>(lk), tick + p, err);
+        else
+            k_radix_pass<1, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
+                                                                 reinterpret_cast<unsigned*>(lk), tick + p, err);
+    }
+}
+
+// start[b] = first sorted position whose key >= b  (b in [0, nbins]).  A warp
+// takes STRETCHES x 32 bins: searches bound each stretch's positions, and
+// where the bounds differ each bin is searched between them (empty stretches
+// are plain stores; one thread per point filling the gap before its key took
+// 58 us on 800,000 points in 7.5 million bins, where the gaps are long, this
+// 36 us).  One stretch per warp where that leaves warps enough for the GPU
+// (the searches are chains of loads), eight above 2^20 bins.
+template <int STRETCHES>
+__global__ void __launch_bounds__(256) k_bin_starts(int64_t n, const unsigned* __restrict__ keys, int64_t nbins,
+                                                    int32_t* __restrict__ start) {
+    const int lane = threadIdx.x & 31;
+    const int64_t b0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * (32 * STRETCHES);
+    if (b0 > nbins) return;
+    auto first_at = [&](int64_t b, int64_t lo, int64_t hi) {  // first position in [lo, hi] with key >= b
+        while (lo < hi) {
+            const int64_t m = lo + ((hi - lo) >> 1);
+            if ((int64_t)keys[m] >= b) hi = m;
+            else lo = m + 1;
+        }
+        return lo;
+    };
+    // lanes 0..STRETCHES bound the stretches
+    int64_t edge = 0;
+    if (lane <= STRETCHES) edge = first_at(b0 + 32 * lane, 0, n);
+    for (int k = 0; k < STRETCHES; k++) {
+        const int64_t lo = __shfl_sync(0xffffffffu, edge, k), hi = __shfl_sync(0xffffffffu, edge, k + 1);
+        const int64_t b = b0 + 32 * k + lane;
+        if (b <= nbins) start[b] = (int32_t)first_at(b, lo, hi);
+    }
 }
 
 // A record's weight: w * e, divided by h^2 TWO_PI for per-point bandwidths
@@ -217,15 +349,6 @@ __global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const floa
     out[i] = r;
 }
 
-__global__ void k_hmax(int64_t n, const float* __restrict__ h, unsigned* out) {
-    unsigned m = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        m = max(m, f2ord(h[i]));
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 // Z-order (Morton) key of the bin of each index record: bit-interleaved bin
 // column and row (16 bits each), value = the record's position.
 __device__ __forceinline__ unsigned spread16(unsigned v) {
@@ -237,17 +360,20 @@ __device__ __forceinline__ unsigned spread16(unsigned v) {
     return v;
 }
 
-__global__ void k_morton_keys(int64_t n, const MgkPt* __restrict__ pts, double ox, double oy, double inv_side,
-                              int64_t nbx, int64_t nby, unsigned* __restrict__ keys, int32_t* __restrict__ vals) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const MgkPt p = pts[i];
-    int64_t bx = (int64_t)floor(((double)(p.xh + p.xl) - ox) * inv_side);
-    int64_t by = (int64_t)floor(((double)(p.yh + p.yl) - oy) * inv_side);
-    bx = bx < 0 ? 0 : (bx >= nbx ? nbx - 1 : bx);
-    by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
-    keys[i] = spread16((unsigned)bx) | (spread16((unsigned)by) << 1);
-    vals[i] = (int32_t)i;
+__global__ void __launch_bounds__(256) k_morton_keys(int64_t n, const MgkPt* __restrict__ pts, double ox, double oy,
+                                                     double inv_side, int64_t nbx, int64_t nby, int db, int passes,
+                                                     unsigned* __restrict__ keys, unsigned* __restrict__ hist) {
+    keys_and_hist(
+        n,
+        [&](int64_t i) {
+            const float4 p = *reinterpret_cast<const float4*>(pts + i);
+            int64_t bx = (int64_t)floor(((double)(p.x + p.z) - ox) * inv_side);
+            int64_t by = (int64_t)floor(((double)(p.y + p.w) - oy) * inv_side);
+            bx = bx < 0 ? 0 : (bx >= nbx ? nbx - 1 : bx);
+            by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
+            return spread16((unsigned)bx) | (spread16((unsigned)by) << 1);
+        },
+        db, passes, keys, hist);
 }
 
 // ---- halo selection: the points inside a rectangle, in input order -------
@@ -354,6 +480,11 @@ int mgk_launch_points_select(mgk_ctx* ctx, const mgk_points* src, double xlo, do
     return MGK_OK;
 }
 
+// CTAs of a key kernel.
+static unsigned key_grid(const mgk_ctx* ctx, int64_t n) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 4 * (int64_t)ctx->sm_count));
+}
+
 int64_t mgk_points_select_scratch(int64_t n) { return (n + kSelTile - 1) / kSelTile + 1; }
 
 // Positions of the index records in Z-order of their bins (stable: records
@@ -364,42 +495,36 @@ int mgk_index_zorder(mgk_ctx* ctx, const mgk_index* idx, int32_t* d_order) {
     if (n == 0) return MGK_OK;
     if (idx->nbx > 65536 || idx->nby > 65536) return mgk_fail(ctx, MGK_ERR_INVALID, "index_zorder: bin grid too large");
     cudaStream_t s = ctx->stream;
-    const int ntiles = (int)((n + kSortTile - 1) / kSortTile);
-    const size_t b_keys = sizeof(unsigned) * (size_t)n, b_vals = sizeof(int32_t) * (size_t)n;
-    const size_t b_cnt = sizeof(unsigned) * 256 * (size_t)ntiles;
-    unsigned *k0 = nullptr, *k1 = nullptr, *cnt = nullptr;
-    int32_t* v0 = nullptr;
-    int st;
-    if ((st = mgk_alloc(ctx, (void**)&k0, b_keys))) return st;
-    if ((st = mgk_alloc(ctx, (void**)&k1, b_keys))) { mgk_free(ctx, k0, b_keys); return st; }
-    if ((st = mgk_alloc(ctx, (void**)&v0, b_vals))) { mgk_free(ctx, k0, b_keys); mgk_free(ctx, k1, b_keys); return st; }
-    if ((st = mgk_alloc(ctx, (void**)&cnt, b_cnt))) {
-        mgk_free(ctx, k0, b_keys); mgk_free(ctx, k1, b_keys); mgk_free(ctx, v0, b_vals);
-        return st;
-    }
-    k_morton_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, idx->pts, idx->ox, idx->oy, 1.0 / idx->side,
-                                                             idx->nbx, idx->nby, k0, v0);
     const uint64_t maxb = (uint64_t)std::max(idx->nbx, idx->nby) - 1;
     int bits = 0;
     while (bits < 16 && (maxb >> bits) != 0) bits++;
-    const int passes = std::max(1, (2 * bits + 7) / 8);
-    unsigned *kin = k0, *kout = k1;
-    int32_t *vin = v0, *vout = d_order;
-    for (int p = 0; p < passes; p++) {
-        k_radix_hist<<<ntiles, kSortThreads, 0, s>>>(n, kin, 8 * p, ntiles, cnt);
-        k_scan_exclusive<<<1, 1024, 0, s>>>(cnt, (int64_t)256 * ntiles);
-        k_radix_scatter<<<ntiles, kSortThreads, 0, s>>>(n, kin, vin, kout, vout, 8 * p, ntiles, cnt);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
+    const SortPlan P = sort_plan(n, 2 * bits);
+    const size_t b_keys = sizeof(unsigned) * (size_t)n, b_vals = sizeof(int32_t) * (size_t)n, b_scr = P.bytes();
+    unsigned *k0 = nullptr, *k1 = nullptr;
+    int32_t* v0 = nullptr;
+    void* scr = nullptr;
+    int st;
+    if ((st = mgk_alloc(ctx, (void**)&k0, b_keys)) || (st = mgk_alloc(ctx, (void**)&k1, b_keys)) ||
+        (st = mgk_alloc(ctx, (void**)&v0, b_vals)) || (st = mgk_alloc(ctx, &scr, b_scr))) {
+        mgk_free(ctx, k0, b_keys);
+        mgk_free(ctx, k1, b_keys);
+        mgk_free(ctx, v0, b_vals);
+        return st;
     }
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && vin != d_order) e = cudaMemcpyAsync(d_order, vin, b_vals, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the scratch is released below
-    MGK_COUNT_LAUNCH(ctx, 1 + 3 * passes);
+    cudaError_t e = cudaMemsetAsync(scr, 0, b_scr, s);
+    if (e == cudaSuccess) {
+        k_morton_keys<<<key_grid(ctx, n), 256, 0, s>>>(n, idx->pts, idx->ox, idx->oy, 1.0 / idx->side, idx->nbx,
+                                                       idx->nby, P.db, P.passes, k0, sort_hist(scr));
+        const bool odd = P.passes & 1;  // the values end in d_order
+        sort_passes(s, P, n, k0, odd ? v0 : d_order, k1, odd ? d_order : v0, scr, ctx->d_map);
+        e = cudaGetLastError();
+    }
+    MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
+    // back to the context's pool; later users are ordered after these kernels on the same stream
     mgk_free(ctx, k0, b_keys);
     mgk_free(ctx, k1, b_keys);
     mgk_free(ctx, v0, b_vals);
-    mgk_free(ctx, cnt, b_cnt);
+    mgk_free(ctx, scr, b_scr);
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index_zorder");
     return MGK_OK;
 }
@@ -414,7 +539,48 @@ int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pt
     return MGK_OK;
 }
 
-int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, mgk_index* idx) {
+// Extent of the points and, with want_h, their largest h (waits for the
+// stream).  No points: the unit square.
+int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_extent* out) {
+    *out = mgk_extent{};
+    if (pts->n <= 0) return MGK_OK;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(kExtentCtas, (pts->n + 1023) / 1024));
+    k_extent<<<blocks, 256, 0, ctx->stream>>>(pts->n, pts->x, pts->y, want_h ? pts->h : nullptr, ctx->d_map + 64);
+    MGK_CHECK_LAUNCH(ctx, "k_extent");
+    MGK_COUNT_LAUNCH(ctx, 1);
+    MGK_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const volatile unsigned* m = ctx->h_map + 64;
+    unsigned v[5] = {0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
+    for (int b = 0; b < blocks; b++)
+        for (int k = 0; k < 5; k++) {
+            const unsigned u = m[5 * b + k];
+            v[k] = k < 2 ? std::min(v[k], u) : std::max(v[k], u);
+        }
+    auto o2f = [](unsigned u) {
+        unsigned w = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
+        float f;
+        memcpy(&f, &w, 4);
+        return f;
+    };
+    out->xmin = o2f(v[0]);
+    out->ymin = o2f(v[1]);
+    out->xmax = o2f(v[2]);
+    out->ymax = o2f(v[3]);
+    if (want_h) out->hmax = o2f(v[4]);
+    return MGK_OK;
+}
+
+// Fails when a sort kernel's bounded wait ran out (after a wait for the stream).
+int mgk_sort_check(mgk_ctx* ctx) {
+    volatile unsigned* f = ctx->h_map;
+    if (!*f) return MGK_OK;
+    *f = 0;
+    return mgk_fail(ctx, MGK_ERR_TIMEOUT, "index sort: a wait for an earlier tile timed out");
+}
+
+// extent: the points' (with per-point h: their largest h too) if known, else null.
+int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
+                           mgk_index* idx) {
     const int64_t n = pts->n;
     cudaStream_t s = ctx->stream;
     idx->ctx = ctx;
@@ -422,37 +588,15 @@ int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float b
     idx->varh = (h <= 0.0f);
     if (idx->varh && !pts->h) return mgk_fail(ctx, MGK_ERR_INVALID, "index_build: h <= 0 but the points carry no per-point h");
     if (n >= (int64_t)INT32_MAX) return mgk_fail(ctx, MGK_ERR_INVALID, "index_build: too many points");
-    // bounding box (and max h for per-point bandwidths) -> host
-    unsigned* d_bb = reinterpret_cast<unsigned*>(ctx->d_counter);
-    const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0u};
-    MGK_CHECK_CUDA(ctx, cudaMemcpyAsync(d_bb, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    const int red_blocks = std::max(1, std::min<int>(ctx->sm_count * 4, (int)((n + 255) / 256)));
-    if (n > 0) {
-        k_bbox<<<red_blocks, 256, 0, s>>>(n, pts->x, pts->y, d_bb);
-        MGK_CHECK_LAUNCH(ctx, "k_bbox");
-        if (idx->varh) {
-            k_hmax<<<red_blocks, 256, 0, s>>>(n, pts->h, d_bb + 4);
-            MGK_CHECK_LAUNCH(ctx, "k_hmax");
-        }
+    int st;
+    mgk_extent ext_own;
+    if (!extent) {
+        if ((st = mgk_points_extent(ctx, pts, idx->varh, &ext_own))) return st;
+        extent = &ext_own;
     }
-    unsigned hb[6];
-    MGK_CHECK_CUDA(ctx, cudaMemcpyAsync(hb, d_bb, sizeof(hb), cudaMemcpyDeviceToHost, s));
-    MGK_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
-    auto o2f = [](unsigned u) {
-        unsigned v = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
-        float f;
-        memcpy(&f, &v, 4);
-        return f;
-    };
-    double xmin = 0, ymin = 0, xmax = 1, ymax = 1;
-    if (n > 0) {
-        xmin = o2f(hb[0]);
-        ymin = o2f(hb[1]);
-        xmax = o2f(hb[2]);
-        ymax = o2f(hb[3]);
-    }
+    const double xmin = extent->xmin, ymin = extent->ymin, xmax = extent->xmax, ymax = extent->ymax;
     float hmax = h;
-    if (idx->varh) hmax = n > 0 ? o2f(hb[4]) : 1.0f;
+    if (idx->varh) hmax = n > 0 ? extent->hmax : 1.0f;
     if (!(hmax > 0.0f) || !std::isfinite(hmax)) return mgk_fail(ctx, MGK_ERR_INVALID, "index_build: bandwidths must be positive and finite");
     idx->h = idx->varh ? 0.0f : h;
     idx->h2 = mgk_h2(hmax);
@@ -483,71 +627,48 @@ int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float b
     const size_t b_start = sizeof(int32_t) * (size_t)(nbins + 1);
     const size_t b_pts = sizeof(MgkPt) * (size_t)std::max<int64_t>(n, 1);
     const size_t b_perm = sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1);
-    int st;
     if ((st = mgk_alloc(ctx, (void**)&idx->bin_start, b_start))) return st;
     if ((st = mgk_alloc(ctx, (void**)&idx->pts, b_pts))) return st;
     if ((st = mgk_alloc(ctx, (void**)&idx->perm, b_perm))) return st;
     idx->bytes = b_start + b_pts + b_perm;
-
-    // scratch: keys x2, vals x1 (+ perm as second value buffer), counts
-    const int ntiles = (int)std::max<int64_t>(1, (n + kSortTile - 1) / kSortTile);
-    const size_t b_keys = sizeof(unsigned) * (size_t)std::max<int64_t>(n, 1);
-    const size_t b_vals = sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1);
-    const size_t b_cnt = sizeof(unsigned) * 256 * (size_t)ntiles;
-    unsigned *k0 = nullptr, *k1 = nullptr, *cnt = nullptr;
-    int32_t* v0 = nullptr;
-    if ((st = mgk_alloc(ctx, (void**)&k0, b_keys))) return st;
-    if ((st = mgk_alloc(ctx, (void**)&k1, b_keys))) { mgk_free(ctx, k0, b_keys); return st; }
-    if ((st = mgk_alloc(ctx, (void**)&v0, b_vals))) { mgk_free(ctx, k0, b_keys); mgk_free(ctx, k1, b_keys); return st; }
-    if ((st = mgk_alloc(ctx, (void**)&cnt, b_cnt))) {
-        mgk_free(ctx, k0, b_keys); mgk_free(ctx, k1, b_keys); mgk_free(ctx, v0, b_vals);
-        return st;
+    if (n == 0) {
+        MGK_CHECK_CUDA(ctx, cudaMemsetAsync(idx->bin_start, 0, b_start, s));
+        return MGK_OK;
     }
-    int rc = MGK_OK;
-    do {
-        if (n > 0) {
-            k_bin_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, pts->x, pts->y, idx->ox, idx->oy,
-                                                                   1.0 / side, idx->nbx, idx->nby, k0, v0);
-            if ((rc = cudaGetLastError()) != cudaSuccess) { rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "k_bin_keys"); break; }
-            int bits = 0;
-            while (bits < 32 && ((uint64_t)(nbins - 1) >> bits) != 0) bits++;
-            const int passes = std::max(1, (bits + 7) / 8);
-            unsigned *kin = k0, *kout = k1;
-            int32_t *vin = v0, *vout = idx->perm;
-            for (int p = 0; p < passes; p++) {
-                k_radix_hist<<<ntiles, kSortThreads, 0, s>>>(n, kin, 8 * p, ntiles, cnt);
-                k_scan_exclusive<<<1, 1024, 0, s>>>(cnt, (int64_t)256 * ntiles);
-                k_radix_scatter<<<ntiles, kSortThreads, 0, s>>>(n, kin, vin, kout, vout, 8 * p, ntiles, cnt);
-                std::swap(kin, kout);
-                std::swap(vin, vout);
-            }
-            if ((rc = cudaGetLastError()) != cudaSuccess) { rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "radix sort"); break; }
-            // sorted keys in kin, values in vin; make sure perm holds the values
-            if (vin != idx->perm) {
-                if ((rc = cudaMemcpyAsync(idx->perm, vin, b_vals, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) {
-                    rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "perm copy");
-                    break;
-                }
-            }
-            k_bin_starts<<<(unsigned)((n + 1 + 255) / 256), 256, 0, s>>>(n, kin, nbins, idx->bin_start);
-            k_gather<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, idx->perm, pts->x, pts->y, pts->w,
-                                                                 pts->has_ew ? pts->ew : nullptr,
-                                                                 idx->varh ? pts->h : nullptr, idx->qexp, idx->pts);
-            if ((rc = cudaGetLastError()) != cudaSuccess) { rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "index gather"); break; }
-            MGK_COUNT_LAUNCH(ctx, (idx->varh ? 2 : 1) + 1 + 3 * passes + 2);
-        } else {
-            if ((rc = cudaMemsetAsync(idx->bin_start, 0, b_start, s)) != cudaSuccess) {
-                rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "bin_start memset");
-                break;
-            }
-        }
-        // scratch must stay alive until the stream has used it
-        if ((rc = cudaStreamSynchronize(s)) != cudaSuccess) { rc = mgk_cuda_fail(ctx, (cudaError_t)rc, "index build"); break; }
-        rc = MGK_OK;
-    } while (0);
-    mgk_free(ctx, k0, b_keys);
-    mgk_free(ctx, k1, b_keys);
-    mgk_free(ctx, v0, b_vals);
-    mgk_free(ctx, cnt, b_cnt);
-    return rc;
+    // the sort's scratch (two key buffers, one value buffer, digit counts and
+    // state words) lies in the record buffer, which the gather fills last
+    int bits = 0;
+    while (bits < 32 && ((uint64_t)(nbins - 1) >> bits) != 0) bits++;
+    const SortPlan P = sort_plan(n, bits);
+    auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
+    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
+    char* base = reinterpret_cast<char*>(idx->pts);
+    void* own = nullptr;
+    if (need > b_pts) {  // few points: a buffer of its own
+        if ((st = mgk_alloc(ctx, &own, need))) return st;
+        base = static_cast<char*>(own);
+    }
+    unsigned *k0 = reinterpret_cast<unsigned*>(base), *k1 = reinterpret_cast<unsigned*>(base + b_buf);
+    int32_t* v0 = reinterpret_cast<int32_t*>(base + 2 * b_buf);
+    void* scr = base + 3 * b_buf;
+    const unsigned gn = (unsigned)((n + 255) / 256);
+    cudaError_t e = cudaMemsetAsync(scr, 0, P.bytes(), s);
+    if (e == cudaSuccess) {
+        k_bin_keys<<<key_grid(ctx, n), 256, 0, s>>>(n, pts->x, pts->y, idx->ox, idx->oy, 1.0 / side, idx->nbx, idx->nby,
+                                                    P.db, P.passes, k0, sort_hist(scr));
+        const bool odd = P.passes & 1;  // the values end in perm
+        sort_passes(s, P, n, k0, odd ? v0 : idx->perm, k1, odd ? idx->perm : v0, scr, ctx->d_map);
+        const unsigned* sorted = odd ? k1 : k0;
+        if (nbins < (1 << 20))
+            k_bin_starts<1><<<(unsigned)(nbins / 256 + 1), 256, 0, s>>>(n, sorted, nbins, idx->bin_start);
+        else
+            k_bin_starts<8><<<(unsigned)(nbins / 2048 + 1), 256, 0, s>>>(n, sorted, nbins, idx->bin_start);
+        k_gather<<<gn, 256, 0, s>>>(n, idx->perm, pts->x, pts->y, pts->w, pts->has_ew ? pts->ew : nullptr,
+                                    idx->varh ? pts->h : nullptr, idx->qexp, idx->pts);
+        e = cudaGetLastError();
+        MGK_COUNT_LAUNCH(ctx, 3 + P.passes);
+    }
+    if (own) mgk_free(ctx, own, need);  // later users are ordered after these kernels on the same stream
+    if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index build");
+    return MGK_OK;
 }

@@ -614,10 +614,12 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     view.has_ew = false;
     view.h = nullptr;
     const int nlev = std::min(kMaxLev, 1 + std::max(0, (int)std::ceil(std::log2((double)h_hi / (double)h_lo))));
+    mgk_extent ext;
+    st = mgk_points_extent(c, &view, false, &ext);
     for (int l = 0; l < nlev && st == MGK_OK; l++) {
         const float side = (float)(0.75 * (double)h_lo * std::ldexp(1.0, l));
         mgk_index* idx = nullptr;
-        st = mgk_index_build(c, &view, h_lo, side, &idx);
+        st = mgk_index_build_async(c, &view, h_lo, side, &ext, &idx);
         if (st == MGK_OK) {
             B->lev.push_back(idx);
             int32_t* q = nullptr;
@@ -766,6 +768,7 @@ int mgk_loo_batch_run(mgk_loo_batch* B, const float* hs, double* logl, int* best
     int* hb = reinterpret_cast<int*>(c->h_counter);
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(hb, B->d_best, sizeof(int), cudaMemcpyDeviceToHost, s));
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(s));
+    if (const int st = mgk_sort_check(c)) return st;
     for (int k = 0; k < B->nh; k++) logl[k] = B->h_logl[k];
     if (best) *best = *hb;
     if (edge_evals) *edge_evals = (int64_t)tail[0];

@@ -43,6 +43,9 @@ struct mgk_ctx {
     void* h_stage[kStageSlots] = {};
     void* d_stage[kStageSlots] = {};
     size_t h_stage_bytes[kStageSlots] = {};
+    // a small mapped page-locked page: word 0 the index sort's wait flag, words
+    // 64.. the extents of k_extent's CTAs
+    unsigned *h_map = nullptr, *d_map = nullptr;
     std::multimap<size_t, void*> pool;        // cached device blocks by size class
     uint64_t launches = 0;                    // kernels launched by this context
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
@@ -297,7 +300,19 @@ __device__ __host__ __forceinline__ double mgk_h2(float h) {
 }
 
 // ---- kernels launched across translation units ------------------------------
-int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, mgk_index* idx);
+struct mgk_extent {
+    double xmin = 0, ymin = 0, xmax = 1, ymax = 1;
+    float hmax = 0;
+};
+int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_extent* out);
+int mgk_sort_check(mgk_ctx* ctx);
+// Builds the index on ctx->stream without waiting for it (mgk_sort_check after
+// a wait); the points' arrays are read until then.
+int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
+                           mgk_index* idx);
+// The same into a new index, for callers that wait later on the same stream.
+int mgk_index_build_async(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
+                          mgk_index** out);
 // The index records' weights from the points' current edge weights (an index
 // built before the edge weights were known), stream-ordered on ctx->stream.
 int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pts);
