@@ -47,10 +47,6 @@ constexpr int kLooSum = 128;  // candidates of a bin row summed in plain FP32 be
 constexpr int kLooWarps = 4;  // warps per CTA, each with work items of its own
 constexpr int kMaxLev = 16;   // bandwidth octaves
 constexpr int kMaxSplit = 16;
-// The cutoff in the scan's exponents, 9 h^2 log2(e) / (2 h^2), and the band
-// around it in which FP32 does not decide.
-constexpr float kLooCut = (float)(0.5 * MGK_CUT * MGK_LOG2E);
-constexpr float kLooBand = 4e-6f * kLooCut;
 // candidates of a batch scanned at a time (one test for the rare cases)
 #ifndef MGK_LOO_TRIP
 #define MGK_LOO_TRIP 8
@@ -105,13 +101,6 @@ __device__ __forceinline__ double loo_log(double sum, double h2) {
     return log(loo > fl ? loo : fl);
 }
 
-// v on a grid of step q = m / (1.5 2^52) (hi) and the remainder (lo)
-__device__ __forceinline__ void split_at(double v, double m, float& hi, float& lo) {
-    const double t = __dsub_rn(__dadd_rn(v, m), m);
-    hi = (float)t;
-    lo = (float)__dsub_rn(v, t);
-}
-
 // Level and processing order of every h (one CTA; nh is small).
 __global__ void k_loo_prep(LooParams P) {
     for (int k = threadIdx.x; k < P.nh; k += blockDim.x) {
@@ -146,9 +135,7 @@ __global__ void k_loo_weights(LooParams P) {
 // issue slots, 68 % of the FMA cycles).  200,000 points, 64 bandwidths in
 // [5, 500]: 225 ms before (scalar FP32, 128 queries a CTA between two
 // barriers per batch, 1.72 tests per pair), 125 ms now.  What gave it:
-//  - distances, exponents and range reduction two candidates at a time
-//    (f32x2), with the coordinates scaled so that the squared distance is the
-//    exponent (two packed operations fewer per pair of candidates);
+//  - distances, exponents and range reduction two candidates at a time (f32x2);
 //  - the polynomial scalar, its coefficients immediates (see mgk_exp2_neg_frac);
 //  - pair counts from sign bits: a predicated increment costs two instructions;
 //  - a warp its own work item: no CTA barriers, and rows cut to the disc
@@ -191,6 +178,12 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
         const float h = P.hgrid[k];
         const double h2 = mgk_h2(h);
         const double cut = MGK_CUT * h2;
+        const float cutf = (float)cut;
+        const float epsd2 = cutf * 4e-6f;
+        // log2(e) / (2 h^2) as a float pair: a one-float scale would bias every
+        // exponent of the batch the same way
+        const double k2 = MGK_LOG2E / (2.0 * h2);
+        const float k2h = (float)k2, k2l = (float)(k2 - (double)k2h);
         const double reach = sqrt(cut) * (1.0 + 1e-9);
         const MgkPt* __restrict__ pts = L.pts;
         const float* __restrict__ wl = P.wl ? P.wl + (int64_t)k * P.n : nullptr;
@@ -240,19 +233,8 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
         // the query's bin row, as the index assigns it
         const int qby = (int)fmin(fmax(floor(((double)qy - L.oy) * L.inv_side), 0.0), (double)(L.nby - 1));
 
-        // Coordinates relative to the box's centre and scaled by sqrt(log2(e) / 2) / h,
-        // so that the exponent is the plain squared distance and the cutoff
-        // 4.5 log2(e) for every h; as float pairs on a grid on which the
-        // differences of the hi parts are exact.
-        const double scale = sqrt(0.5 * MGK_LOG2E / h2);
-        const double ccx = 0.5 * ((double)mnx + (double)mxx), ccy = 0.5 * ((double)mny + (double)mxy);
-        const double ext = (0.5 * fmax((double)mxx - (double)mnx, (double)mxy - (double)mny) + reach) * scale;
-        const double grid = 1.5 * 1073741824.0 * mgk_pow2(ilogb(ext) + 1);  // 1.5 2^52 q, q = 2^-22 2^(ilogb + 1)
-        float qsx, qsy, qlx, qly;
-        split_at(((double)qx - ccx) * scale, grid, qsx, qlx);
-        split_at(((double)qy - ccy) * scale, grid, qsy, qly);
-        const f2 qxh = f2_dup(qsx), qyh = f2_dup(qsy), qxl = f2_dup(qlx), qyl = f2_dup(qly);
-        const f2 cut2 = f2_dup(kLooCut);
+        const f2 qxh = f2_dup(q.x), qyh = f2_dup(q.y), qxl = f2_dup(q.z), qyl = f2_dup(q.w);
+        const f2 k2h2 = f2_dup(k2h), k2l2 = f2_dup(k2l), cut2 = f2_dup(cutf);
         // part: the candidates of a bin row since the last multiple of kLooSum
         // of the group's range in it (a group's queries are all summed in the
         // same pieces), then into the compensated sum
@@ -327,7 +309,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
                     const int j = jb + 32 * i;
-                    cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end
+                    cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end: far outside the cutoff
                     cw[i] = 0.0f;
                     bool first = false;
                     int o = INT_MAX;
@@ -357,13 +339,10 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
             auto put = [&](int buf) {
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    float xh, xl, yh, yl;
-                    split_at(((double)(cp[i].x + cp[i].z) - ccx) * scale, grid, xh, xl);
-                    split_at(((double)(cp[i].y + cp[i].w) - ccy) * scale, grid, yh, yl);
-                    cand[buf][0][lane + 32 * i] = cp[i].x < 1e18f ? xh : 1e18f;  // past the end: far outside the cutoff
-                    cand[buf][1][lane + 32 * i] = yh;
-                    cand[buf][2][lane + 32 * i] = xl;
-                    cand[buf][3][lane + 32 * i] = yl;
+                    cand[buf][0][lane + 32 * i] = cp[i].x;
+                    cand[buf][1][lane + 32 * i] = cp[i].y;
+                    cand[buf][2][lane + 32 * i] = cp[i].z;
+                    cand[buf][3][lane + 32 * i] = cp[i].w;
                     cand[buf][4][lane + 32 * i] = cw[i];
                 }
             };
@@ -391,11 +370,12 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
                         const f2 w = *reinterpret_cast<const f2*>(&cand[buf][4][t + u]);
                         const f2 dx = f2_add(f2_sub(xh, qxh), f2_sub(xl, qxl));
                         const f2 dy = f2_add(f2_sub(yh, qyh), f2_sub(yl, qyl));
-                        const f2 a = f2_fma(dx, dx, f2_mul(dy, dy));
-                        f2_get(f2_sub(a, cut2), x[u], x[u + 1]);
+                        const f2 d2 = f2_fma(dx, dx, f2_mul(dy, dy));
+                        f2_get(f2_sub(d2, cut2), x[u], x[u + 1]);
                         // 2^-a = 2^-n 2^-g with a = n + g, |g| <= 1/2.  2^-n comes from the
                         // special-function unit, which is exact for integers and idle
                         // otherwise, not from a shift into the exponent bits
+                        const f2 a = f2_fma(d2, k2h2, f2_mul(d2, k2l2));
                         const f2 n = f2_sub(f2_sub(magic, a), magic);  // -n
                         float g0, g1, n0, n1;
                         f2_get(f2_add(a, n), g0, g1);
@@ -409,10 +389,10 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
 #pragma unroll
                     for (int u = 1; u + 1 < kLooTrip; u += 2) near = mgk_min3(near, fabsf(x[u]), fabsf(x[u + 1]));
                     near = fminf(near, fabsf(x[kLooTrip - 1]));
-                    if (near <= kLooBand || (unsigned)ts < (unsigned)kLooTrip) {
+                    if (near <= epsd2 || (unsigned)ts < (unsigned)kLooTrip) {
 #pragma unroll
                         for (int u = 0; u < kLooTrip; u++) {
-                            if (fabsf(x[u]) <= kLooBand) {  // near the cutoff: the oracle's FP64 decision
+                            if (fabsf(x[u]) <= epsd2) {  // near the cutoff: the oracle's FP64 decision
                                 int rr = 0;
                                 while (j + t + u >= row[rr].x) rr++;
                                 const float4 cc =
