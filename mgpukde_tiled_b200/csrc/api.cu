@@ -442,6 +442,7 @@ int mgk_raster_destroy(mgk_raster* r) {
     mgk_free(c, r->cand, sizeof(float2) * (size_t)std::max<int64_t>(r->ncand, 1));
     mgk_free(c, r->run_start, sizeof(int64_t) * (size_t)(r->g.nrows + 1));
     mgk_free(c, r->runs, sizeof(int2) * (size_t)std::max<int64_t>(r->nruns, 1));
+    mgk_free(c, r->row_run, mgk_row_tables_bytes(r->g));
     delete r;
     return MGK_OK;
 }

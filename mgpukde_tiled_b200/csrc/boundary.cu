@@ -359,13 +359,14 @@ __global__ void k_dist2_cands(int64_t n, const int32_t* __restrict__ order, cons
 // MODE 1 writes them at the row's offset as half-open [a, b).
 template <int MODE>
 __global__ void k_row_runs(mgk_grid g, const float* __restrict__ mask, int64_t* __restrict__ start,
-                           int2* __restrict__ runs) {
+                           int2* __restrict__ runs, int4* __restrict__ first) {
     const int lane = threadIdx.x & 31;
     const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (r >= g.nrows) return;  // warp-uniform
     const float* row = mask + r * g.ncols;
     const float nd = g.nodata;
     int64_t ns = 0, ne = 0;
+    int a0 = 0, b0 = 0;  // the first run
     const int64_t base = MODE ? start[r] : 0;
     for (int64_t c0 = 0; c0 < g.ncols; c0 += 32) {
         const int64_t c = c0 + lane;
@@ -382,10 +383,22 @@ __global__ void k_row_runs(mgk_grid g, const float* __restrict__ mask, int64_t* 
             if (v && !vl) runs[base + ns + __popc(sm & lt)].x = (int)c;
             if (v && !vr) runs[base + ne + __popc(em & lt)].y = (int)(c + 1);
         }
+        if (!MODE && ns == 0 && sm) a0 = (int)c0 + __ffs(sm) - 1;
+        if (!MODE && ne == 0 && em) b0 = (int)c0 + __ffs(em);
         ns += __popc(sm);
         ne += __popc(em);
     }
-    if (!MODE && lane == 0) start[r] = ns;
+    if (!MODE && lane == 0) {
+        start[r] = ns;
+        first[r] = make_int4(a0, b0, (int)ns, 0);
+    }
+}
+
+// The cell centres, as doubles of their float values.
+__global__ void k_centres(mgk_grid g, double* __restrict__ cx, double* __restrict__ cy) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < g.ncols) cx[i] = (double)mgk_cell_x(g.xll, g.cs, i);
+    else if (i < g.ncols + g.nrows) cy[i - g.ncols] = (double)mgk_cell_y(g.yll, g.cs, g.nrows, i - g.ncols);
 }
 
 // Exclusive scan of n int64 values in one CTA; the total goes to a[n].
@@ -428,9 +441,18 @@ int mgk_raster_runs(mgk_ctx* ctx, mgk_raster* r) {
     const size_t sb = sizeof(int64_t) * (size_t)(g.nrows + 1);
     int st;
     if ((st = mgk_alloc(ctx, (void**)&r->run_start, sb))) return st;
+    if (!r->centre_x) {  // of the grid alone: once per raster
+        const size_t nc = (size_t)(g.ncols + g.nrows);
+        if ((st = mgk_alloc(ctx, (void**)&r->row_run, mgk_row_tables_bytes(g)))) return st;
+        r->centre_x = reinterpret_cast<double*>(r->row_run + g.nrows);
+        r->centre_y = r->centre_x + g.ncols;
+        k_centres<<<(unsigned)((nc + 255) / 256), 256, 0, s>>>(g, r->centre_x, r->centre_y);
+        MGK_CHECK_LAUNCH(ctx, "k_centres");
+        MGK_COUNT_LAUNCH(ctx, 1);
+    }
     MGK_CHECK_CUDA(ctx, cudaMemsetAsync(r->run_start, 0, sb, s));
     const unsigned grid = (unsigned)((g.nrows * 32 + 255) / 256);
-    k_row_runs<0><<<grid, 256, 0, s>>>(g, r->mask, r->run_start, nullptr);
+    k_row_runs<0><<<grid, 256, 0, s>>>(g, r->mask, r->run_start, nullptr, r->row_run);
     k_scan_i64<<<1, 1024, 0, s>>>(r->run_start, g.nrows);
     MGK_CHECK_LAUNCH(ctx, "k_row_runs count");
     MGK_COUNT_LAUNCH(ctx, 2);
@@ -439,7 +461,7 @@ int mgk_raster_runs(mgk_ctx* ctx, mgk_raster* r) {
     MGK_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
     if ((st = mgk_alloc(ctx, (void**)&r->runs, sizeof(int2) * (size_t)std::max<int64_t>(total, 1)))) return st;
     r->nruns = total;
-    k_row_runs<1><<<grid, 256, 0, s>>>(g, r->mask, r->run_start, r->runs);
+    k_row_runs<1><<<grid, 256, 0, s>>>(g, r->mask, r->run_start, r->runs, nullptr);
     MGK_CHECK_LAUNCH(ctx, "k_row_runs fill");
     MGK_COUNT_LAUNCH(ctx, 1);
     r->has_runs = true;

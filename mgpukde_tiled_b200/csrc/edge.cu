@@ -13,10 +13,10 @@
 // factors' prefix sums Q over the window,
 //   sum = sum_rows exp(-dy^2/2h^2) * sum_{valid runs of the row} (Q[b] - Q[a])
 // where [a, b) is a run of valid cells clipped to the row's in-cutoff
-// interval.  The interval ends are found with the oracle's exact FP64 test
-// (an estimate from sqrt(9h^2 - dy^2), verified, with a binary search when the
-// estimate misses), so the summed cell set and the eval count are exactly the
-// reference's.  Work per (point, h) is O(window width + window height) rather
+// interval.  The interval ends come from sqrt(9h^2 - dy^2) in FP32; where one
+// lies too near a cell centre for that to decide, the oracle's exact FP64 test
+// does (the estimate verified, with a binary search when it misses), so the
+// summed cell set and the eval count are exactly the reference's.  Work per (point, h) is O(window width + window height) rather
 // than O(width x height); the sums are FP64, the factors FP64 (per-point h)
 // or FP32 to about 1e-7 (fixed h, edge_factor).
 //
@@ -27,6 +27,7 @@
 // e_p(h) for every candidate h); the weights for h_k go to row k of the
 // output.
 #include <algorithm>
+#include <cmath>
 
 #include "mgk_internal.cuh"
 
@@ -45,8 +46,11 @@ struct EdgeParams {
     int nh;
     const double* dist2;  // may be null: no short-circuit
     mgk_grid g;
+    const double *cx, *cy;  // cell centres by column and row
+    float margin;           // cells by which a centre may lie off its regular place, and the estimates' rounding
     const int64_t* run_start;
     const int2* runs;
+    const int4* row_run;  // per row: its first run (x, y), the number of its runs (z)
     float* ew;  // [nh][ew_stride]
     int64_t ew_stride;
     unsigned long long* evals;
@@ -76,17 +80,16 @@ __global__ void k_edge_near(EdgeParams E, int* __restrict__ list, int* __restric
     if (near) list[base + __popc(b & ((1u << lane) - 1u))] = (int)p;
 }
 
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 __device__ __forceinline__ int64_t trunc_index(double v) {
     v = fmin(fmax(v, -1.0e15), 1.0e15);
     return (int64_t)trunc(v);
 }
-
-__device__ __forceinline__ int64_t clamp_index(double v, int64_t lo, int64_t hi) {
-    v = fmin(fmax(v, (double)lo), (double)hi);
-    return (int64_t)v;
-}
-
-__device__ __forceinline__ double cell_xd(const mgk_grid& g, int64_t c) { return (double)mgk_cell_x(g.xll, g.cs, c); }
 
 // exp(-d2 / 2h^2) for d2 within the cutoff (exponent <= 4.5).  Fixed h:
 // 2^-(d2 k2) with the exponent in FP64, split into a float pair, 2^-hi by
@@ -94,9 +97,10 @@ __device__ __forceinline__ double cell_xd(const mgk_grid& g, int64_t c) { return
 // (relative error about 1e-7; the weights then meet the 1e-6 density and
 // likelihood tolerances).  Per-point h (the adaptive search, whose
 // Hooke-Jeeves steps compare nearby likelihoods): the FP64 exp.
+// (m2: -1 / (2 h^2).)
 template <bool VARH>
-__device__ __forceinline__ double edge_factor(double d2, double h2, double k2) {
-    if (VARH) return exp(d2 / (-2.0 * h2));
+__device__ __forceinline__ double edge_factor(double d2, double m2, double k2) {
+    if (VARH) return exp(d2 * m2);
     const double a = d2 * k2;
     const float ah = (float)a;
     const float al = (float)(a - (double)ah);
@@ -105,84 +109,147 @@ __device__ __forceinline__ double edge_factor(double d2, double h2, double k2) {
 }
 
 // The oracle's FP64 cutoff decision for column c of a row at dy^2.
-__device__ __forceinline__ bool in_cut(const mgk_grid& g, int64_t c, double px, double dy2, double cut) {
-    const double dx = __dsub_rn(cell_xd(g, c), px);
+__device__ __forceinline__ bool in_cut(const double* cx, int c, double px, double dy2, double cut) {
+    const double dx = __dsub_rn(cx[c], px);
     return __dadd_rn(__dmul_rn(dx, dx), dy2) < cut;
 }
 
-// Smallest c in [a, b] with in_cut true; in_cut is false..true over [a, b]
-// and true at b.
-__device__ __forceinline__ int64_t first_in(const mgk_grid& g, int64_t a, int64_t b, double px, double dy2,
+// The columns [lo, hi] of [c0, c1] inside the cutoff by the exact test, from
+// estimates of the ends (out of line: few rows need it).  Empty: lo > hi.
+__device__ __noinline__ int2 exact_interval(const double* cx, int c0, int c1, int lo, int hi, double px, double dy2,
                                             double cut) {
+    // the column nearest the point: every non-empty interval holds it
+    int a = c0, b = c1 + 1;
     while (a < b) {
-        const int64_t m = a + ((b - a) >> 1);
-        if (in_cut(g, m, px, dy2, cut)) b = m;
+        const int m = a + ((b - a) >> 1);
+        if (cx[m] >= px) b = m;
         else a = m + 1;
     }
-    return a;
-}
-
-// Largest c in [a, b] with in_cut true; true..false over [a, b], true at a.
-__device__ __forceinline__ int64_t last_in(const mgk_grid& g, int64_t a, int64_t b, double px, double dy2,
-                                           double cut) {
+    int cm = a > c1 ? c1 : a;
+    if (a > c0 && a <= c1 && __dsub_rn(px, cx[a - 1]) < __dsub_rn(cx[a], px)) cm = a - 1;
+    if (!in_cut(cx, cm, px, dy2, cut)) return make_int2(1, 0);
+    // in_cut is false..true over [c0, cm] and true..false over [cm, c1]
+    a = c0;
+    b = cm;
+    lo = min(max(lo, c0), cm);
+    if (in_cut(cx, lo, px, dy2, cut)) {
+        b = lo;
+        if (lo == c0 || !in_cut(cx, lo - 1, px, dy2, cut)) a = lo;
+    } else {
+        a = lo + 1;
+    }
     while (a < b) {
-        const int64_t m = a + ((b - a + 1) >> 1);
-        if (in_cut(g, m, px, dy2, cut)) a = m;
+        const int m = a + ((b - a) >> 1);
+        if (in_cut(cx, m, px, dy2, cut)) b = m;
+        else a = m + 1;
+    }
+    lo = a;
+    a = cm;
+    b = c1;
+    hi = min(max(hi, cm), c1);
+    if (in_cut(cx, hi, px, dy2, cut)) {
+        a = hi;
+        if (hi == c1 || !in_cut(cx, hi + 1, px, dy2, cut)) b = hi;
+    } else {
+        b = hi - 1;
+    }
+    while (a < b) {
+        const int m = a + ((b - a + 1) >> 1);
+        if (in_cut(cx, m, px, dy2, cut)) a = m;
         else b = m - 1;
     }
-    return a;
+    return make_int2(lo, a);
 }
 
+// What bounds it: the latency of its chains (table loads, FP64 operations,
+// conversions at 16 lanes a clock) with 24 warps an SM to hide them.  64
+// bandwidths on 200,000 points: 23.6 ms with every interval end tested exactly
+// (five FP64 tests a row, each from a cell centre formed anew with three
+// conversions), 64-bit columns and one task's four divisions after the other;
+// 12.2 ms with the centres and each row's first run from tables, the exact
+// test only where FP32 cannot decide (a few rows in a hundred), and the tasks'
+// divisions side by side.  One bandwidth of 50 on the 10^6 points: 185 -> 121
+// us.
 template <bool VARH>
-__global__ void __launch_bounds__(kEdgeWarps * 32) k_edge_rows(EdgeParams E) {
+__global__ void __launch_bounds__(kEdgeWarps * 32, 6) k_edge_rows(EdgeParams E) {
     __shared__ double qsum[kEdgeWarps][kEdgeChunk + 1];
     const int lane = threadIdx.x & 31;
     double* Q = qsum[threadIdx.x >> 5];
     const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const mgk_grid g = E.g;
+    const mgk_grid& g = E.g;
     const double xll = g.xll, yll = g.yll, cs = g.cs;
-    const double inv_cs = 1.0 / cs;  // for the interval estimates, which the exact test then verifies
+    const float inv_cs = 1.0f / g.cs;
     const double cell_area = (double)(g.cs * g.cs);  // float product, kde_cuda_kdtr_tiled.cu:2698
-    const int nh = VARH ? 1 : E.nh;
+    const int64_t nlist = E.list ? (int64_t)*E.list_count : E.n;
+    const int64_t ntask = nlist * (VARH ? 1 : E.nh);
     unsigned long long cnt_total = 0;
-    const int64_t ntask = E.list ? (int64_t)*E.list_count : E.n;
-    for (int64_t t = warp0; t < ntask; t += nwarps) {
-        const int64_t p = E.list ? (int64_t)E.list[t] : t;
-        const double px = E.x[p], py = E.y[p];
-        const double d2b = E.dist2 ? E.dist2[p] : 0.0;
-        for (int k = 0; k < nh; k++) {
+    // Tasks (h by h, the points of one h in a row) in batches of up to 32, as
+    // large as leave every warp two or more: each lane prepares one, the divisions and square roots of a batch side by
+    // side, then the warp takes those that need the integral in turn.
+    int batch = 32;
+    while (batch > 1 && ntask < 2 * nwarps * batch) batch >>= 1;
+    for (int64_t t0 = warp0 * batch; t0 < ntask; t0 += nwarps * batch) {
+        bool need = false;
+        float* out = nullptr;
+        float fpx = 0.0f, fpy = 0.0f, fcol_l = 0.0f;
+        int icol_l = 0, cl_l = 0, cu_l = -1;
+        int64_t rl_l = 0, ru_l = -1;
+        double h2_l = 1.0, k2_l = 0.0, acc_l = 0.0;
+        if (lane < batch && t0 + lane < ntask) {
+            const int64_t k = (t0 + lane) / nlist, i = (t0 + lane) - k * nlist;
+            const int64_t p = E.list ? (int64_t)E.list[i] : i;
             const float hp = VARH ? E.hpp[p] : (E.hgrid ? E.hgrid[k] : E.hfix);
-            const double h2 = mgk_h2(hp);
-            const double cut = MGK_CUT * h2;
-            float* out = E.ew + (int64_t)k * E.ew_stride + p;
-            if (E.dist2 && d2b >= cut) {
-                if (lane == 0) *out = 1.0f;
-                continue;
+            h2_l = mgk_h2(hp);
+            out = E.ew + k * E.ew_stride + p;
+            need = !E.dist2 || E.dist2[p] < MGK_CUT * h2_l;
+            if (!need) *out = 1.0f;
+            if (need) {
+                fpx = E.x[p];
+                fpy = E.y[p];
+                const double px = fpx, py = fpy;
+                // the point's place in columns: an integer and a fraction
+                const double pcol = fmin(fmax((px - xll) / cs - 0.5, -1.0e9), 1.0e9);
+                icol_l = (int)floor(pcol);
+                fcol_l = (float)(pcol - (double)icol_l);
+                k2_l = MGK_LOG2E / (2.0 * h2_l);
+                // NARROW window (kde_cuda_kdtr_tiled.cu_l:2719-2727), truncating casts as in Utilities.h:16-17
+                const double reach = 3.0 * (double)hp;
+                rl_l = g.nrows - 1 - trunc_index((py + reach - yll) / cs);
+                ru_l = g.nrows - 1 - trunc_index((py - reach - yll) / cs);
+                rl_l = rl_l < 0 ? 0 : rl_l;
+                ru_l = ru_l > g.nrows - 1 ? g.nrows - 1 : ru_l;
+                cl_l = (int)mgk_min64(mgk_max64(trunc_index((px - reach - xll) / cs), 0), g.ncols);
+                cu_l = (int)mgk_max64(mgk_min64(trunc_index((px + reach - xll) / cs), g.ncols - 1), -1);
             }
-            const double reach = 3.0 * (double)hp;
-            // NARROW window (kde_cuda_kdtr_tiled.cu:2719-2727), truncating casts as in Utilities.h:16-17
-            int64_t rl = g.nrows - 1 - trunc_index((py + reach - yll) / cs);
-            int64_t ru = g.nrows - 1 - trunc_index((py - reach - yll) / cs);
-            int64_t cl = trunc_index((px - reach - xll) / cs);
-            int64_t cu = trunc_index((px + reach - xll) / cs);
-            rl = rl < 0 ? 0 : rl;
-            ru = ru > g.nrows - 1 ? g.nrows - 1 : ru;
-            cl = cl < 0 ? 0 : cl;
-            cu = cu > g.ncols - 1 ? g.ncols - 1 : cu;
-            const double k2 = MGK_LOG2E / (2.0 * h2);
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, need); todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const double px = __shfl_sync(0xffffffffu, fpx, src), py = __shfl_sync(0xffffffffu, fpy, src);
+            const double h2 = __shfl_sync(0xffffffffu, h2_l, src), k2 = __shfl_sync(0xffffffffu, k2_l, src);
+            const double cut = MGK_CUT * h2;
+            const double m2 = VARH ? -1.0 / (2.0 * h2) : 0.0;
+            const int cl = __shfl_sync(0xffffffffu, cl_l, src), cu = __shfl_sync(0xffffffffu, cu_l, src);
+            const int icol = __shfl_sync(0xffffffffu, icol_l, src);
+            const float fcol = __shfl_sync(0xffffffffu, fcol_l, src);
+            const int64_t rl = __shfl_sync(0xffffffffu, rl_l, src), ru = __shfl_sync(0xffffffffu, ru_l, src);
             double acc = 0.0;
             unsigned long long cnt = 0;
-            for (int64_t c0 = cl; c0 <= cu && rl <= ru; c0 += kEdgeChunk) {
-                const int64_t c1 = mgk_min64(cu, c0 + kEdgeChunk - 1);
-                const int len = (int)(c1 - c0 + 1);
-                // prefix sums of the column factors: Q[j] = sum of the first j
+            for (int c0 = cl; c0 <= cu && rl <= ru; c0 += kEdgeChunk) {
+                const int c1 = min(cu, c0 + kEdgeChunk - 1);
+                const int len = c1 - c0 + 1;
+                // the column factors, then their prefix sums: Q[j] = sum of the first j
+#pragma unroll 2
+                for (int j = lane; j < len; j += 32) {
+                    const double dx = __dsub_rn(E.cx[c0 + j], px);
+                    Q[j + 1] = edge_factor<VARH>(__dmul_rn(dx, dx), m2, k2);
+                }
+                __syncwarp();
                 const int per = (len + 31) >> 5;
                 const int j0 = min(len, lane * per), j1 = min(len, j0 + per);
                 double run = 0.0;
                 for (int j = j0; j < j1; j++) {
-                    const double dx = __dsub_rn(cell_xd(g, c0 + j), px);
-                    run += edge_factor<VARH>(__dmul_rn(dx, dx), h2, k2);
+                    run += Q[j + 1];
                     Q[j + 1] = run;
                 }
                 double off = run;
@@ -194,69 +261,82 @@ __global__ void __launch_bounds__(kEdgeWarps * 32) k_edge_rows(EdgeParams E) {
                 for (int j = j0; j < j1; j++) Q[j + 1] += off;
                 if (lane == 0) Q[0] = 0.0;
                 __syncwarp();
-                // the chunk column nearest the point: every non-empty row interval holds it
-                int64_t a = c0, b = c1 + 1;
-                while (a < b) {
-                    const int64_t m = a + ((b - a) >> 1);
-                    if (cell_xd(g, m) >= px) b = m;
-                    else a = m + 1;
+                // (the next row's table entries are on their way during a row)
+                int4 row_n = make_int4(0, 0, 0, 0);
+                double cy_n = 0.0;
+                if (rl + lane <= ru) {
+                    row_n = E.row_run[rl + lane];
+                    cy_n = E.cy[rl + lane];
                 }
-                int64_t cm = a > c1 ? c1 : a;
-                if (a > c0 && a <= c1 && __dsub_rn(px, cell_xd(g, a - 1)) < __dsub_rn(cell_xd(g, a), px)) cm = a - 1;
                 for (int64_t r = rl + lane; r <= ru; r += 32) {
-                    const double dy = __dsub_rn((double)mgk_cell_y(yll, cs, g.nrows, r), py);
+                    const int4 row = row_n;  // its first run and their number
+                    const double dy = __dsub_rn(cy_n, py);
+                    if (r + 32 <= ru) {
+                        row_n = E.row_run[r + 32];
+                        cy_n = E.cy[r + 32];
+                    }
                     const double dy2 = __dmul_rn(dy, dy);
-                    if (dy2 >= cut || !in_cut(g, cm, px, dy2, cut)) continue;
-                    const double t = sqrt(cut - dy2);
-                    int64_t lo = clamp_index(ceil((px - t - xll) * inv_cs - 0.5), c0, cm);
-                    if (in_cut(g, lo, px, dy2, cut)) {
-                        if (lo > c0 && in_cut(g, lo - 1, px, dy2, cut)) lo = first_in(g, c0, lo - 1, px, dy2, cut);
+                    if (dy2 >= cut) continue;
+                    // the half-chord in columns; the ends' places relative to icol
+                    const float tc = sqrt_approx((float)(cut - dy2)) * inv_cs;
+                    const float fl = fcol - tc, fh = fcol + tc;
+                    const float il = ceilf(fl), ih = floorf(fh);
+                    const float m = __fmaf_rn(1e-6f, tc, E.margin);
+                    int lo = icol + (int)il, hi = icol + (int)ih;
+                    if (il - fl < m || il - fl > 1.0f - m || fh - ih < m || fh - ih > 1.0f - m || tc < 2.0f * m) {
+                        const int2 ex = exact_interval(E.cx, c0, c1, lo, hi, px, dy2, cut);
+                        lo = ex.x;
+                        hi = ex.y;
                     } else {
-                        lo = first_in(g, lo + 1, cm, px, dy2, cut);
+                        lo = max(lo, c0);
+                        hi = min(hi, c1);
                     }
-                    int64_t hi = clamp_index(floor((px + t - xll) * inv_cs - 0.5), cm, c1);
-                    if (in_cut(g, hi, px, dy2, cut)) {
-                        if (hi < c1 && in_cut(g, hi + 1, px, dy2, cut)) hi = last_in(g, hi + 1, c1, px, dy2, cut);
-                    } else {
-                        hi = last_in(g, cm, hi - 1, px, dy2, cut);
-                    }
+                    if (lo > hi) continue;
                     // valid runs of the row clipped to [lo, hi]
-                    int64_t q = E.run_start[r];
-                    const int64_t qe = E.run_start[r + 1];
-                    if (qe - q > 8) {  // first run ending after lo
-                        int64_t x0 = q, x1 = qe;
-                        while (x0 < x1) {
-                            const int64_t m = x0 + ((x1 - x0) >> 1);
-                            if (E.runs[m].y <= lo) x0 = m + 1;
-                            else x1 = m;
-                        }
-                        q = x0;
-                    }
                     double S = 0.0;
-                    for (; q < qe; q++) {
-                        const int2 rr = E.runs[q];
-                        if (rr.y <= lo) continue;
-                        if (rr.x > hi) break;
-                        const int64_t ra = mgk_max64(rr.x, lo), rb = mgk_min64((int64_t)rr.y - 1, hi);
+                    auto add = [&](int ra, int rb) {  // the run [ra, rb)
+                        ra = max(ra, lo);
+                        rb = min(rb - 1, hi);
+                        if (ra > rb) return;
                         S += Q[rb - c0 + 1] - Q[ra - c0];
-                        cnt += (unsigned long long)(rb - ra + 1);
+                        cnt += (unsigned)(rb - ra + 1);
+                    };
+                    if (row.z > 0) add(row.x, row.y);
+                    if (row.z > 1 && row.y <= hi) {
+                        int64_t q = E.run_start[r] + 1;
+                        const int64_t qe = E.run_start[r + 1];
+                        if (qe - q > 8) {  // first run ending after lo
+                            int64_t x0 = q, x1 = qe;
+                            while (x0 < x1) {
+                                const int64_t m = x0 + ((x1 - x0) >> 1);
+                                if (E.runs[m].y <= lo) x0 = m + 1;
+                                else x1 = m;
+                            }
+                            q = x0;
+                        }
+                        for (; q < qe; q++) {
+                            const int2 rr = E.runs[q];
+                            if (rr.x > hi) break;
+                            add(rr.x, rr.y);
+                        }
                     }
-                    if (S != 0.0) acc += edge_factor<VARH>(dy2, h2, k2) * S;
+                    if (S != 0.0) acc += edge_factor<VARH>(dy2, m2, k2) * S;
                 }
                 __syncwarp();
             }
-            for (int o = 16; o; o >>= 1) {
-                acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            }
-            if (lane == 0) {
-                const double k0 = 1.0 / (h2 * (double)MGK_TWO_PI_F);
-                *out = (float)(1.0 / (acc * k0 * cell_area));
-                cnt_total += cnt;
-            }
+            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            cnt_total += cnt;
+            if (lane == src) acc_l = acc;
+        }
+        if (need) {
+            const double k0 = 1.0 / (h2_l * (double)MGK_TWO_PI_F);
+            *out = (float)(1.0 / (acc_l * k0 * cell_area));
         }
     }
-    if (E.evals && lane == 0 && cnt_total) atomicAdd(E.evals, cnt_total);
+    if (E.evals) {
+        for (int o = 16; o; o >>= 1) cnt_total += __shfl_xor_sync(0xffffffffu, cnt_total, o);
+        if (lane == 0 && cnt_total) atomicAdd(E.evals, cnt_total);
+    }
 }
 
 }  // namespace
@@ -279,6 +359,16 @@ int mgk_launch_edge_weights_multi(mgk_ctx* ctx, int64_t n, const float* x, const
     E.nh = hpp ? 1 : nh;
     E.dist2 = dist2;
     E.g = r->g;
+    E.cx = r->centre_x;
+    E.cy = r->centre_y;
+    {
+        // float centres lie within half an ulp of their regular places, the
+        // estimates within a few more and 1e-4 cells (their own rounding)
+        const double ext = std::max(std::fabs((double)r->g.xll),
+                                    std::fabs((double)r->g.xll + (double)r->g.ncols * (double)r->g.cs));
+        E.margin = (float)std::min(1.0, 1e-4 + 4.0 * ext * 0x1p-24 / (double)r->g.cs);
+    }
+    E.row_run = r->row_run;
     E.run_start = r->run_start;
     E.runs = r->runs;
     E.ew = ew_out;
@@ -292,7 +382,7 @@ int mgk_launch_edge_weights_multi(mgk_ctx* ctx, int64_t n, const float* x, const
         &occ, hpp ? (const void*)k_edge_rows<true> : (const void*)k_edge_rows<false>, threads, 0);
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "edge weights occupancy");
     occ = std::max(occ, 1);
-    const int64_t blocks = std::min<int64_t>((int64_t)ctx->sm_count * occ, (n + kEdgeWarps - 1) / kEdgeWarps);
+    const int64_t blocks = std::min<int64_t>((int64_t)ctx->sm_count * occ, (n * (int64_t)E.nh + kEdgeWarps - 1) / kEdgeWarps);
     int *list = nullptr, *count = nullptr;
     const size_t b_list = sizeof(int) * (size_t)n;
     const bool listed = E.nh == 1 && dist2 && n < (int64_t)INT32_MAX;

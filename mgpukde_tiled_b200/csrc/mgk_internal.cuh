@@ -98,7 +98,14 @@ struct mgk_raster {
     int2* runs = nullptr;
     int64_t nruns = 0;
     bool has_runs = false;
+    // per row its first run (x, y) and the number of its runs (z); cell centres
+    // by column and row (one block, mgk_row_tables_bytes)
+    int4* row_run = nullptr;
+    double *centre_x = nullptr, *centre_y = nullptr;
 };
+inline size_t mgk_row_tables_bytes(const mgk_grid& g) {
+    return sizeof(int4) * (size_t)g.nrows + sizeof(double) * (size_t)(g.ncols + g.nrows);
+}
 
 // One point of the bin-major index (32 B, one bulk copy moves whole records).
 // Coordinates are split on a global quantum q = 2^-qexp: x = xh + xl exactly,
@@ -240,11 +247,12 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 
 // 2^-g for g in [-1/2, 1/2]: a degree-6 polynomial, fitted to 2^-g by least
 // squares on Chebyshev nodes with the mean error held where the rounding of
-// the scan's terms leaves none, each coefficient rounded to float before the
-// next ones are fitted (truncation 3.3e-9 relative; the weighted mean error of
-// the terms over the cutoff's disc is 1e-12, that of a degree-8 Taylor form on
-// an unscaled distance -6e-11).  Scalar with immediate coefficients: a packed
-// FMA with three register pairs runs at 3.3 cycles instead of 2.
+// the terms leaves none, each coefficient rounded to float before the next
+// ones are fitted (truncation 3.3e-9 relative).  Terms 2^-a formed with it over
+// the cutoff's disc: relative error 7.04e-8 rms, 2.3e-7 at most, at most 2e-11
+// in the weighted mean (with the degree-8 Taylor form of mgk_exp2_neg_poly
+// 7.05e-8, 2.3e-7, 7e-11).  Scalar with immediate coefficients: a packed FMA
+// with three register pairs runs at 3.3 cycles instead of 2.
 __device__ __forceinline__ float mgk_exp2_neg_frac(float g) {
     float p = __fmaf_rn(0.00015285507834050804f, g, -0.001339130220003426f);
     p = __fmaf_rn(p, g, 0.009618666023015976f);
