@@ -1186,9 +1186,9 @@ void fill_params(DParams& P, const mgk_index* idx, const mgk_grid* g, int64_t ro
 }
 
 // Work items of one tile from its per-block candidate counts: blocks above K
-// candidates are split into items of at most K (about 8 waves of the
-// resident CTAs), each split item writing an FP64 partial into its own
-// scratch slot.  K depends on this tile alone, so a tile gets the same items
+// candidates are split into items of at most K, each split item writing an
+// FP64 partial into its own scratch slot (fine: small tiles are split finer;
+// without the memory for that, coarsely).  K depends on this tile alone, so a tile gets the same items
 // (and bitwise the same result) alone or batched with others.
 struct TilePlan {
     int nbx_t = 0, nby_t = 0;
@@ -1197,14 +1197,23 @@ struct TilePlan {
     int32_t nslots = 0;
 };
 
-void plan_tile(const int64_t* counts, int nbx_t, int nby_t, int sm_count, int waves, int job, TilePlan& T) {
+void plan_tile(const int64_t* counts, int nbx_t, int nby_t, int sm_count, int waves, int job, bool fine, TilePlan& T) {
+    T = TilePlan();
     const int nblk = nbx_t * nby_t;
     T.nbx_t = nbx_t;
     T.nby_t = nby_t;
     int64_t total = 0;
     for (int b = 0; b < nblk; b++) total += counts[b];
     const int64_t slots_resident = (int64_t)sm_count * 2;
-    int64_t K = std::max<int64_t>(2048, total / std::max<int64_t>(1, slots_resident * waves));
+    // Below about 1,200 candidates a slot the waves do not matter and the
+    // longest item does: 2,048 candidates are 32 batches, 345 us on an SM of
+    // its own.  Two items a slot then, but not under 256 candidates (a split
+    // item also writes and merges 64 KB): a 2,311 x 1,873 raster of 60,000
+    // points 5.65 -> 3.73 ms against 2,048 at least, 1.40 -> 1.40 ms where
+    // 800,000 points keep every slot busy; four a slot 1.45 ms there.
+    const int64_t least =
+        !fine ? 2048 : std::min<int64_t>(2048, std::max<int64_t>(256, total / (2 * slots_resident)));
+    int64_t K = std::max<int64_t>(least, total / std::max<int64_t>(1, slots_resident * waves));
     K = (K + kMB - 1) / kMB * kMB;
     T.items.reserve(nblk + 16);
     for (int b = 0; b < nblk; b++) {
@@ -1359,14 +1368,18 @@ static int plan_from_counts(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* 
     const int nbx_t = (int)((nc + kBC - 1) / kBC), nby_t = (int)((nr + kBR - 1) / kBR);
     int st;
     TilePlan& T = D->T;
-    plan_tile(counts, nbx_t, nby_t, ctx->sm_count, ctx->split_waves, 0, T);
-    sort_items(T.items);
-    const int32_t nslots = T.nslots;
-    D->b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(nslots, 1);
-    if (nslots && (st = mgk_alloc(ctx, (void**)&P.scratch, D->b_scr))) {
+    for (const bool fine : {true, false}) {
+        plan_tile(counts, nbx_t, nby_t, ctx->sm_count, ctx->split_waves, 0, fine, T);
+        D->b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(T.nslots, 1);
+        st = T.nslots ? mgk_alloc(ctx, (void**)&P.scratch, D->b_scr) : MGK_OK;
+        if (st == MGK_OK) break;
+    }
+    if (st) {
         delete D;
         return st;
     }
+    sort_items(T.items);
+    const int32_t nslots = T.nslots;
     // the work list, the split tables and the error flag in the staging:
     // [items | split blocks | split begins | err]
     auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
@@ -1602,12 +1615,19 @@ int mgk_launch_density_jobs(mgk_ctx* ctx, int njobs, const mgk_tile_job* jobs, u
     std::vector<int4> merges;
     int32_t nslots = 0;
     std::vector<int32_t> slot0(njobs, 0);
-    {
-        const int64_t* counts = reinterpret_cast<const int64_t*>(h_st);
+    size_t b_scr = 0;
+    double* d_scr = nullptr;
+    const std::vector<int64_t> counts(reinterpret_cast<const int64_t*>(h_st),
+                                      reinterpret_cast<const int64_t*>(h_st) + nblk_all);
+    for (const bool fine : {true, false}) {
+        items_fix.clear();
+        items_var.clear();
+        merges.clear();
+        nslots = 0;
         for (int j = 0; j < njobs; j++) {
             if (!nbx[j]) continue;
             TilePlan T;
-            plan_tile(counts + off[j], nbx[j], nby[j], ctx->sm_count, ctx->split_waves, j, T);
+            plan_tile(counts.data() + off[j], nbx[j], nby[j], ctx->sm_count, ctx->split_waves, j, fine, T);
             slot0[j] = nslots;
             for (size_t b = 0; b < T.split_blocks.size(); b++)
                 merges.push_back(make_int4(j, T.split_blocks[b], T.split_begin[b], T.split_begin[b + 1]));
@@ -1615,12 +1635,13 @@ int mgk_launch_density_jobs(mgk_ctx* ctx, int njobs, const mgk_tile_job* jobs, u
             std::vector<Item>& dst = jobs[j].index->varh ? items_var : items_fix;
             dst.insert(dst.end(), T.items.begin(), T.items.end());
         }
+        b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(nslots, 1);
+        st = nslots ? mgk_alloc(ctx, (void**)&d_scr, b_scr) : MGK_OK;
+        if (st == MGK_OK) break;
     }
+    if (st) return st;
     sort_items(items_fix);
     sort_items(items_var);
-    const size_t b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(nslots, 1);
-    double* d_scr = nullptr;
-    if (nslots && (st = mgk_alloc(ctx, (void**)&d_scr, b_scr))) return st;
     for (int j = 0; j < njobs; j++)
         P[j].scratch = d_scr ? d_scr + (size_t)slot0[j] * kCells : nullptr;  // slots are job-local
     // staging: [job parameters | items (fixed h, then per-point h) | merges | err]
