@@ -81,7 +81,8 @@ struct mgk_raster {
     float* mask = nullptr;
     bool owns = false;
     uint8_t* boundary = nullptr;  // per cell
-    float2* bcells = nullptr;     // boundary-cell centres, binned
+    float2* bcells = nullptr;     // boundary-cell centres, binned once the lists are built
+    bool binned = false;
     int* bstart = nullptr;        // bin offsets into bcells (nbins + 1)
     int* bnear = nullptr;         // per bin: first ring index holding a non-empty bin
     double* bub = nullptr;        // per bin: upper bound of the nearest-cell d^2 of its points
