@@ -20,6 +20,55 @@
 
 #include "mgk_internal.cuh"
 
+// device buffers of each kind (mask in, density out) in flight
+#ifndef MGK_RASTER_DEPTH
+#define MGK_RASTER_DEPTH 3
+#endif
+
+constexpr int kDepth = MGK_RASTER_DEPTH;
+
+// Streams and events of the whole-raster path, made by a context's first call
+// and kept for the next (making and dropping the four streams and thirteen
+// events took about 0.2 ms of each call).  Every call waits for its streams
+// before it returns, on errors too, so nothing is in flight between calls;
+// a context serves one thread at a time.
+struct mgk_raster_pipe {
+    cudaStream_t h2d = nullptr, d2h = nullptr, alt = nullptr, mrg = nullptr;
+    cudaEvent_t mask_ready[kDepth] = {}, done[kDepth] = {}, out_free[kDepth] = {}, dens[kDepth] = {};
+    cudaEvent_t counted = nullptr, em_ready = nullptr;
+    ~mgk_raster_pipe() {
+        for (int i = 0; i < kDepth; i++) {
+            if (mask_ready[i]) cudaEventDestroy(mask_ready[i]);
+            if (done[i]) cudaEventDestroy(done[i]);
+            if (out_free[i]) cudaEventDestroy(out_free[i]);
+            if (dens[i]) cudaEventDestroy(dens[i]);
+        }
+                if (h2d) cudaStreamDestroy(h2d);
+        if (d2h) cudaStreamDestroy(d2h);
+        if (alt) cudaStreamDestroy(alt);
+        if (mrg) cudaStreamDestroy(mrg);
+    }
+    cudaError_t init() {
+        cudaError_t e = cudaStreamCreateWithFlags(&h2d, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d2h, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&alt, cudaStreamNonBlocking);
+        // the merges of split blocks at the highest priority: a band's merge
+        // is scheduled ahead of the next band's pending CTAs
+        int least = 0, greatest = 0;
+        if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&mrg, cudaStreamNonBlocking, greatest);
+        for (int i = 0; i < kDepth && e == cudaSuccess; i++) {
+            e = cudaEventCreateWithFlags(&mask_ready[i], cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&out_free[i], cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&dens[i], cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&counted, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&em_ready, cudaEventDisableTiming);
+        return e;
+    }
+};
+
 // ---------------------------------------------------------------- helpers --
 int mgk_fail(mgk_ctx* ctx, int status, const std::string& msg) {
     if (ctx) ctx->last_error = msg;
@@ -202,6 +251,7 @@ int mgk_ctx_destroy(mgk_ctx* c) {
     if (c->h_counter) cudaFreeHost(c->h_counter);
     if (c->h_sum) cudaFreeHost(c->h_sum);
     if (c->h_map) cudaFreeHost(c->h_map);
+    delete c->pipe;
     for (int i = 0; i < mgk_ctx::kStageSlots; i++)
         if (c->h_stage[i]) cudaFreeHost(c->h_stage[i]);
     if (c->ev_a) cudaEventDestroy(c->ev_a);
@@ -793,14 +843,8 @@ int mgk_mle_fixed_bandwidth(mgk_ctx* c, mgk_points* p, const mgk_raster* r, floa
 #ifndef MGK_RASTER_BANDS
 #define MGK_RASTER_BANDS 8
 #endif
-// device buffers of each kind (mask in, density out) in flight
-#ifndef MGK_RASTER_DEPTH
-#define MGK_RASTER_DEPTH 3
-#endif
-
 namespace {
 constexpr int64_t kRasterBands = MGK_RASTER_BANDS;  // full-width bands without an explicit tile side
-constexpr int kDepth = MGK_RASTER_DEPTH;
 
 // cuStreamWaitValue32 / cuStreamWriteValue32 through the runtime's driver
 // entry points (no link-time dependency on the driver library).
@@ -850,39 +894,6 @@ bool stream_memops_work(mgk_ctx* c) {
     ok_by_device[c->device] = ok;
     return ok;
 }
-struct RasterPipe {
-    cudaStream_t h2d = nullptr, d2h = nullptr, alt = nullptr, mrg = nullptr;
-    cudaEvent_t mask_ready[kDepth] = {}, done[kDepth] = {}, out_free[kDepth] = {}, dens[kDepth] = {};
-    ~RasterPipe() {
-        for (int i = 0; i < kDepth; i++) {
-            if (mask_ready[i]) cudaEventDestroy(mask_ready[i]);
-            if (done[i]) cudaEventDestroy(done[i]);
-            if (out_free[i]) cudaEventDestroy(out_free[i]);
-            if (dens[i]) cudaEventDestroy(dens[i]);
-        }
-        if (h2d) cudaStreamDestroy(h2d);
-        if (d2h) cudaStreamDestroy(d2h);
-        if (alt) cudaStreamDestroy(alt);
-        if (mrg) cudaStreamDestroy(mrg);
-    }
-    cudaError_t init() {
-        cudaError_t e = cudaStreamCreateWithFlags(&h2d, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d2h, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&alt, cudaStreamNonBlocking);
-        // the merges of split blocks at the highest priority: a band's merge
-        // is scheduled ahead of the next band's pending CTAs
-        int least = 0, greatest = 0;
-        if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&mrg, cudaStreamNonBlocking, greatest);
-        for (int i = 0; i < kDepth && e == cudaSuccess; i++) {
-            e = cudaEventCreateWithFlags(&mask_ready[i], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&out_free[i], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&dens[i], cudaEventDisableTiming);
-        }
-        return e;
-    }
-};
 }  // namespace
 
 // The whole path over rows [row_lo, row_hi) of dg (dmask and out_density
@@ -943,6 +954,9 @@ class MaskPacker {
             for (int64_t r = band_r0[k]; r < band_r0[k + 1]; r += kChunk)
                 chunks_.push_back({k, r - row_lo, std::min<int64_t>(band_r0[k + 1], r + kChunk) - r});
         }
+        // a small mask is packed band by band by the caller, while the GPU
+        // works on the points: starting the threads would take longer
+        if (nb == 0 || ncols * (band_r0[nb] - band_r0[0]) <= kInlineCells) return;
         const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
         const int nt = (int)std::min<unsigned>(MGK_MASK_PACK_THREADS, std::max(1u, hw / 2));
         for (int t = 0; t < nt; t++) threads_.emplace_back([this] { work(); });
@@ -953,6 +967,8 @@ class MaskPacker {
     }
     // returns once band k is packed
     void wait_band(int64_t k) {
+        if (threads_.empty())
+            while (next_.load() < (int64_t)chunks_.size() && done_[k].load() < band_rows_[k]) pack_next();
         while (done_[k].load(std::memory_order_acquire) < band_rows_[k]) std::this_thread::yield();
     }
 
@@ -961,16 +977,21 @@ class MaskPacker {
         int64_t band, row, rows;
     };
     static constexpr int64_t kChunk = 64;
+    static constexpr int64_t kInlineCells = 1 << 19;
+    // packs the next chunk; false when none is left
+    bool pack_next() {
+        const int64_t i = next_.fetch_add(1);
+        if (i >= (int64_t)chunks_.size() || stop_.load()) return false;
+        const Chunk& ch = chunks_[i];
+        for (int64_t r = ch.row; r < ch.row + ch.rows; r++) {
+            if (avx2_) pack_mask_row_avx2(src_ + r * ncols_, ncols_, nodata_, dst_ + r * stride_, stride_);
+            else pack_mask_row(src_ + r * ncols_, ncols_, nodata_, dst_ + r * stride_, stride_);
+        }
+        done_[ch.band].fetch_add(ch.rows, std::memory_order_release);
+        return true;
+    }
     void work() {
-        for (;;) {
-            const int64_t i = next_.fetch_add(1);
-            if (i >= (int64_t)chunks_.size() || stop_.load()) return;
-            const Chunk& ch = chunks_[i];
-            for (int64_t r = ch.row; r < ch.row + ch.rows; r++) {
-                if (avx2_) pack_mask_row_avx2(src_ + r * ncols_, ncols_, nodata_, dst_ + r * stride_, stride_);
-                else pack_mask_row(src_ + r * ncols_, ncols_, nodata_, dst_ + r * stride_, stride_);
-            }
-            done_[ch.band].fetch_add(ch.rows, std::memory_order_release);
+        while (pack_next()) {
         }
     }
     const float* src_;
@@ -1024,9 +1045,14 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     const bool packed = dmask && !band_r0.empty();
     const int64_t mstride = (dg->ncols + 127) / 128 * 16;
     const size_t tbm = packed ? (size_t)tr * (size_t)mstride : tb;
-    RasterPipe pipe;
-    cudaError_t ce = pipe.init();
-    if (ce != cudaSuccess) return mgk_cuda_fail(c, ce, "kde_raster streams");
+    cudaError_t ce = cudaSuccess;
+    if (!c->pipe) {
+        std::unique_ptr<mgk_raster_pipe> made(new (std::nothrow) mgk_raster_pipe());
+        if (!made) return mgk_fail(c, MGK_ERR_INVALID, "kde_raster: out of host memory");
+        if ((ce = made->init()) != cudaSuccess) return mgk_cuda_fail(c, ce, "kde_raster streams");
+        c->pipe = made.release();
+    }
+    mgk_raster_pipe& pipe = *c->pipe;
     mgk_points* p = nullptr;
     mgk_raster* em = nullptr;
     mgk_index* idx = nullptr;
@@ -1103,12 +1129,10 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     // the points (its records take the edge weights once they are known).
     float* d_em = nullptr;
     const size_t b_em = edge_correction ? sizeof(float) * (size_t)eg->ncols * (size_t)eg->nrows : 0;
-    cudaEvent_t em_ready = nullptr;
     if (st == MGK_OK && edge_correction) {
         if ((st = mgk_alloc(c, (void**)&d_em, b_em)) == MGK_OK) {
-            ce = cudaEventCreateWithFlags(&em_ready, cudaEventDisableTiming);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_em, emask, b_em, cudaMemcpyHostToDevice, pipe.h2d);
-            if (ce == cudaSuccess) ce = cudaEventRecord(em_ready, pipe.h2d);
+            ce = cudaMemcpyAsync(d_em, emask, b_em, cudaMemcpyHostToDevice, pipe.h2d);
+            if (ce == cudaSuccess) ce = cudaEventRecord(pipe.em_ready, pipe.h2d);
             if (ce != cudaSuccess) st = mgk_cuda_fail(c, ce, "kde_raster edge mask");
         }
         if (st == MGK_OK) st = mgk_raster_wrap(c, eg, d_em, &em);
@@ -1124,7 +1148,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
             if (h_pp)
                 for (int64_t i = 0; i < n; i++) hmax = std::max(hmax, h_pp[i]);
             const double reach = 3.0 * (double)hmax * (1.0 + 1e-6);
-            if ((ce = cudaStreamWaitEvent(c->stream, em_ready, 0)) != cudaSuccess)
+            if ((ce = cudaStreamWaitEvent(c->stream, pipe.em_ready, 0)) != cudaSuccess)
                 st = mgk_cuda_fail(c, ce, "kde_raster edge mask");
             if (st == MGK_OK && (st = mgk_boundary_dist_within(c, p, em, reach)) == MGK_OK &&
                 (st = mgk_edge_weights(c, p, em, hfix, evals ? &ev_edge : nullptr)) == MGK_OK)
@@ -1157,9 +1181,6 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     // the counting kernel of tile k has finished, the density of tile k - 2
     // (queued before it) has too, so that plan and its staging slot are free.
     mgk_dplan* plans[2] = {nullptr, nullptr};
-    cudaEvent_t counted = nullptr;
-    if (st == MGK_OK && (ce = cudaEventCreateWithFlags(&counted, cudaEventDisableTiming)) != cudaSuccess)
-        st = mgk_cuda_fail(c, ce, "kde_raster event");
     unsigned long long* d_ev = evals ? c->d_counter + 4 : nullptr;
     auto plan_of = [&](int64_t k) -> int {  // after tile k's counting kernel has finished
         int64_t r0, c0, nr, nc;
@@ -1204,8 +1225,8 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         if (st == MGK_OK && (ce = cudaStreamSynchronize(c->stream)) != cudaSuccess)
             st = mgk_cuda_fail(c, ce, "kde_raster plan");
         // the alternate stream follows the preparation on the context stream
-        if (st == MGK_OK && two && ((ce = cudaEventRecord(counted, c->stream)) != cudaSuccess ||
-                                    (ce = cudaStreamWaitEvent(pipe.alt, counted, 0)) != cudaSuccess))
+        if (st == MGK_OK && two && ((ce = cudaEventRecord(pipe.counted, c->stream)) != cudaSuccess ||
+                                    (ce = cudaStreamWaitEvent(pipe.alt, pipe.counted, 0)) != cudaSuccess))
             st = mgk_cuda_fail(c, ce, "kde_raster");
         const int64_t* counts = st == MGK_OK ? mgk_density_counts_host(c, 0) : nullptr;
         const int64_t nbx = (dg->ncols + 127) / 128;
@@ -1279,7 +1300,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         }
         if (k + 1 < ntiles) {
             if ((st = count_of(k + 1))) break;
-            if ((ce = cudaEventRecord(counted, c->stream)) != cudaSuccess) {
+            if ((ce = cudaEventRecord(pipe.counted, c->stream)) != cudaSuccess) {
                 st = mgk_cuda_fail(c, ce, "kde_raster");
                 break;
             }
@@ -1299,7 +1320,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
             break;
         }
         if (k + 1 < ntiles) {
-            if ((ce = cudaEventSynchronize(counted)) != cudaSuccess) {
+            if ((ce = cudaEventSynchronize(pipe.counted)) != cudaSuccess) {
                 st = mgk_cuda_fail(c, ce, "kde_raster plan");
                 break;
             }
@@ -1315,7 +1336,6 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     for (int i = 0; i < 2; i++) mgk_density_discard(c, plans[i]);  // every kernel has ended
     for (mgk_dplan* D : band_plans) mgk_density_discard(c, D);
     if (d_flag) mgk_free(c, d_flag, sizeof(unsigned) * ntiles);
-    if (counted) cudaEventDestroy(counted);
     if (st == MGK_OK) {  // counters 4 (density evals) and 7 (staging-wait flag)
         ce = cudaMemcpy(c->h_counter + 4, c->d_counter + 4, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
         if (ce != cudaSuccess) st = mgk_cuda_fail(c, ce, "kde_raster counters");
@@ -1329,7 +1349,6 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
     mgk_index_destroy(idx);
     mgk_raster_destroy(em);
     if (d_em) mgk_free(c, d_em, b_em);
-    if (em_ready) cudaEventDestroy(em_ready);
     mgk_points_destroy(p);
     if (st == MGK_OK && evals) *evals = ev_den + ev_edge;
     return st;

@@ -23,6 +23,8 @@
 #define MGK_LN2F 0.69314718055994531f
 
 // ---- host-side objects -----------------------------------------------------
+struct mgk_raster_pipe;  // streams and events of the whole-raster path (api.cu)
+
 struct mgk_ctx {
     int device = 0;
     int sm_count = 0;
@@ -46,6 +48,7 @@ struct mgk_ctx {
     // a small mapped page-locked page: word 0 the index sort's wait flag, words
     // 64.. the extents of k_extent's CTAs
     unsigned *h_map = nullptr, *d_map = nullptr;
+    mgk_raster_pipe* pipe = nullptr;
     std::multimap<size_t, void*> pool;        // cached device blocks by size class
     uint64_t launches = 0;                    // kernels launched by this context
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
