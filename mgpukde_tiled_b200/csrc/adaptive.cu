@@ -335,14 +335,24 @@ __global__ void k_adaptive_h(int64_t n, const double* __restrict__ den0, const d
     hs[i] = (float)((double)h * pow(den0[i] / gml, (double)alpha));
 }
 
-// Per bin: 9 h^2 of its widest point (-1 for an empty bin).
-__global__ void k_bin_reach2(int64_t nbins, const int32_t* __restrict__ bin_start, const MgkPt* __restrict__ pts,
-                             float* __restrict__ r2) {
-    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (b >= nbins) return;
-    float m = -1.0f;
-    for (int64_t t = bin_start[b]; t < bin_start[b + 1]; t++) m = fmaxf(m, pts[t].hh);
-    r2[b] = m < 0.0f ? -1.0f : 9.0f * m;
+// Per bin: 9 h^2 of its widest point.  r2 starts at -1 (an empty bin), and
+// non-negative floats order as their bits, so the maximum is an integer one
+// (a thread per bin walking its points took 25 us, the densest bin's chain).
+__global__ void k_bin_reach2(int64_t n, const MgkPt* __restrict__ pts, double ox, double oy, double inv_side,
+                             int64_t nbx, int64_t nby, float* __restrict__ r2) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const MgkPt p = pts[i];
+    int64_t bx = (int64_t)floor(((double)(p.xh + p.xl) - ox) * inv_side);
+    int64_t by = (int64_t)floor(((double)(p.yh + p.yl) - oy) * inv_side);
+    bx = bx < 0 ? 0 : (bx >= nbx ? nbx - 1 : bx);
+    by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
+    atomicMax(reinterpret_cast<int*>(r2) + by * nbx + bx, __float_as_int(9.0f * p.hh));
+}
+
+__global__ void k_fill_f32(int64_t n, float v, float* __restrict__ out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = v;
 }
 
 // Counters of a likelihood computation: context counter slots 5 (edge-mask
@@ -399,7 +409,9 @@ int point_density(mgk_ctx* c, const mgk_index* idx, bool self, double* d_den, do
     }
     const dim3 grid((unsigned)g, (unsigned)nsplit);
     if (idx->varh) {
-        k_bin_reach2<<<(unsigned)((nbins + 255) / 256), 256, 0, s>>>(nbins, idx->bin_start, idx->pts, r2);
+        k_fill_f32<<<(unsigned)((nbins + 255) / 256), 256, 0, s>>>(nbins, -1.0f, r2);
+        k_bin_reach2<<<(unsigned)((idx->n + 255) / 256), 256, 0, s>>>(idx->n, idx->pts, idx->ox, idx->oy,
+                                                                     1.0 / idx->side, idx->nbx, idx->nby, r2);
         k_point_density<true, false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
                                                            idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
                                                            idx->h2, r2, psum,
@@ -424,7 +436,7 @@ int point_density(mgk_ctx* c, const mgk_index* idx, bool self, double* d_den, do
     mgk_free(c, psum, b_psum);
     if (r2) mgk_free(c, r2, b_r2);
     if (e != cudaSuccess) return mgk_cuda_fail(c, e, "k_point_density");
-    MGK_COUNT_LAUNCH(c, idx->varh ? 4 : 3);
+    MGK_COUNT_LAUNCH(c, idx->varh ? 5 : 3);
     return MGK_OK;
 }
 
