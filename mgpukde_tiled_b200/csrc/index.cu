@@ -27,7 +27,36 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kMaxDigits = 512;   // digits of up to 9 bits: 18-bit bin ids sort in two passes
 constexpr int kMaxPasses = 4;     // 32-bit keys
 constexpr long long kSortSpin = 1ll << 24;
+constexpr int kBuildLevels = 16;  // indexes built together
 constexpr int kExtentCtas = 512;  // their words fit the context's mapped page
+
+// The kernels of a build take up to N indexes of the same points (the levels of
+// a bandwidth batch) in one launch: blockIdx.y is the index.
+template <typename T, int N>
+struct Jobs {
+    T j[N];
+};
+struct KeyJob {
+    double inv_side;
+    int64_t nbx, nby;
+    const MgkPt* pts;  // the records (Z-order keys), else null
+    unsigned *keys, *hist;
+};
+struct SortJob {  // from (ka, indexes) through (kb, vb) and back
+    unsigned *ka, *kb;
+    int32_t *va, *vb;
+    unsigned* scratch;
+};
+struct StartJob {
+    const unsigned* keys;
+    int64_t nbins;
+    int32_t* start;
+};
+struct GatherJob {
+    const int32_t* perm;
+    MgkPt* out;
+    int qexp;
+};
 
 __device__ __forceinline__ unsigned f2ord(float f) {
     unsigned u = __float_as_uint(f);
@@ -81,10 +110,13 @@ __device__ __forceinline__ void keys_and_hist(int64_t n, const KeyOf& key_of, in
         if (sh[d]) atomicAdd(&hist[d], sh[d]);
 }
 
+template <int N>
 __global__ void __launch_bounds__(256) k_bin_keys(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
-                                                  double ox, double oy, double inv_side, int64_t nbx, int64_t nby,
-                                                  int db, int passes, unsigned* __restrict__ keys,
-                                                  unsigned* __restrict__ hist) {
+                                                  double ox, double oy, int db, int passes,
+                                                  const __grid_constant__ Jobs<KeyJob, N> J) {
+    const KeyJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    const double inv_side = B.inv_side;
+    const int64_t nbx = B.nbx, nby = B.nby;
     keys_and_hist(
         n,
         [&](int64_t i) {
@@ -94,7 +126,7 @@ __global__ void __launch_bounds__(256) k_bin_keys(int64_t n, const float* __rest
             by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
             return (unsigned)(by * nbx + bx);
         },
-        db, passes, keys, hist);
+        db, passes, B.keys, B.hist);
 }
 
 // Exclusive scan of `len` counts in one CTA of 1024 threads (chunked).
@@ -131,15 +163,21 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(unsigned* __restrict__ 
 // tiles' counts in one CTA, a scatter in rounds of 256 items with five
 // barriers each, tiles of 8,192) took 85 us a pass on 10^6 points and 29 us on
 // 2,000, where one CTA did everything; this takes 36 and 6 us (an index build
-// 289 -> 144 and 99 -> 54 us).  vals_in null: the values are the items'
-// indexes.
-template <int IPT, typename W>
-__global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, const unsigned* __restrict__ keys_in,
-                                                             const int32_t* __restrict__ vals_in,
-                                                             unsigned* __restrict__ keys_out,
-                                                             int32_t* __restrict__ vals_out, int shift, int db,
-                                                             const unsigned* __restrict__ hist, W* look,
-                                                             unsigned* tick, unsigned* err) {
+// 289 -> 144 and 99 -> 54 us).  Before the first pass the values are the
+// items' indexes.
+template <int IPT, typename W, int N>
+__global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, int db, size_t look_bytes,
+                                                             const __grid_constant__ Jobs<SortJob, N> J,
+                                                             unsigned* err) {
+    const SortJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    const unsigned* __restrict__ keys_in = p & 1 ? B.kb : B.ka;
+    const int32_t* __restrict__ vals_in = p == 0 ? nullptr : p & 1 ? B.vb : B.va;
+    unsigned* __restrict__ keys_out = p & 1 ? B.ka : B.kb;
+    int32_t* __restrict__ vals_out = p & 1 ? B.va : B.vb;
+    const unsigned* __restrict__ hist = B.scratch + (p << db);
+    unsigned* tick = B.scratch + kMaxPasses * kMaxDigits + p;
+    W* look = reinterpret_cast<W*>(reinterpret_cast<char*>(B.scratch + kMaxPasses * kMaxDigits + 8) + p * look_bytes);
+    const int shift = p * db;
     constexpr int kTop = sizeof(W) * 8 - 2;
     constexpr W kVal = ((W)1 << kTop) - 1;
     __shared__ unsigned cnt[kSortWarps][kMaxDigits];  // a warp's digit counts, then its offsets in the tile
@@ -243,36 +281,21 @@ SortPlan sort_plan(int64_t n, int bits) {
     return P;
 }
 
-unsigned* sort_hist(void* scratch) { return static_cast<unsigned*>(scratch); }
-
-// Sorts (keys in ka, values = indexes) with the histograms already in the
-// scratch, through kb, vb and back; the sorted keys and values end in kb, vb
-// after an odd number of passes, else in ka, va.
-void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, unsigned* ka, int32_t* va, unsigned* kb, int32_t* vb,
-                 void* scratch, unsigned* err) {
-    unsigned* hist = sort_hist(scratch);
-    unsigned* tick = hist + kMaxPasses * kMaxDigits;
-    char* look = reinterpret_cast<char*>(tick + 8);
+// Sorts the keys in ka (values: indexes) with the histograms already in the
+// scratch; the sorted keys and values end in kb, vb after an odd number of
+// passes, else in ka, va.
+template <int N>
+void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, int nj, const Jobs<SortJob, N>& J, unsigned* err) {
+    const dim3 g((unsigned)P.ntiles, (unsigned)nj);
     for (int p = 0; p < P.passes; p++) {
-        const unsigned* ki = p & 1 ? kb : ka;
-        const int32_t* vi = p == 0 ? nullptr : p & 1 ? vb : va;
-        unsigned* ko = p & 1 ? ka : kb;
-        int32_t* vo = p & 1 ? va : vb;
-        const unsigned* h = hist + p * (1 << P.db);
-        char* lk = look + (size_t)p * P.look_bytes();
-        const unsigned g = (unsigned)P.ntiles;
         if (P.wide)
-            k_radix_pass<16, unsigned long long><<<g, kSortThreads, 0, s>>>(
-                n, ki, vi, ko, vo, p * P.db, P.db, h, reinterpret_cast<unsigned long long*>(lk), tick + p, err);
+            k_radix_pass<16, unsigned long long, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
         else if (P.ipt == 16)
-            k_radix_pass<16, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
-                                                                  reinterpret_cast<unsigned*>(lk), tick + p, err);
+            k_radix_pass<16, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
         else if (P.ipt == 4)
-            k_radix_pass<4, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
-                                                                 reinterpret_cast<unsigned*>(lk), tick + p, err);
+            k_radix_pass<4, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
         else
-            k_radix_pass<1, unsigned><<<g, kSortThreads, 0, s>>>(n, ki, vi, ko, vo, p * P.db, P.db, h,
-                                                                 reinterpret_cast<unsigned*>(lk), tick + p, err);
+            k_radix_pass<1, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
     }
 }
 
@@ -283,9 +306,12 @@ void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, unsigned* ka, int
 // 58 us on 800,000 points in 7.5 million bins, where the gaps are long, this
 // 36 us).  One stretch per warp where that leaves warps enough for the GPU
 // (the searches are chains of loads), eight above 2^20 bins.
-template <int STRETCHES>
-__global__ void __launch_bounds__(256) k_bin_starts(int64_t n, const unsigned* __restrict__ keys, int64_t nbins,
-                                                    int32_t* __restrict__ start) {
+template <int STRETCHES, int N>
+__global__ void __launch_bounds__(256) k_bin_starts(int64_t n, const __grid_constant__ Jobs<StartJob, N> J) {
+    const StartJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    const unsigned* __restrict__ keys = B.keys;
+    const int64_t nbins = B.nbins;
+    int32_t* __restrict__ start = B.start;
     const int lane = threadIdx.x & 31;
     const int64_t b0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * (32 * STRETCHES);
     if (b0 > nbins) return;
@@ -326,10 +352,14 @@ __global__ void k_refresh_wk(int64_t n, const int32_t* __restrict__ perm, const 
     if (i < n) out[i].wk = record_wk(w, ew, hpp, perm[i]);
 }
 
-__global__ void k_gather(int64_t n, const int32_t* __restrict__ perm, const float* __restrict__ x,
-                         const float* __restrict__ y, const float* __restrict__ w,
-                         const float* __restrict__ ew, const float* __restrict__ hpp, int qexp,
-                         MgkPt* __restrict__ out) {
+template <int N>
+__global__ void k_gather(int64_t n, const float* __restrict__ x, const float* __restrict__ y,
+                         const float* __restrict__ w, const float* __restrict__ ew, const float* __restrict__ hpp,
+                         const __grid_constant__ Jobs<GatherJob, N> J) {
+    const GatherJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    const int32_t* __restrict__ perm = B.perm;
+    MgkPt* __restrict__ out = B.out;
+    const int qexp = B.qexp;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int32_t j = perm[i];
@@ -360,9 +390,13 @@ __device__ __forceinline__ unsigned spread16(unsigned v) {
     return v;
 }
 
-__global__ void __launch_bounds__(256) k_morton_keys(int64_t n, const MgkPt* __restrict__ pts, double ox, double oy,
-                                                     double inv_side, int64_t nbx, int64_t nby, int db, int passes,
-                                                     unsigned* __restrict__ keys, unsigned* __restrict__ hist) {
+template <int N>
+__global__ void __launch_bounds__(256) k_morton_keys(int64_t n, double ox, double oy, int db, int passes,
+                                                     const __grid_constant__ Jobs<KeyJob, N> J) {
+    const KeyJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    const MgkPt* __restrict__ pts = B.pts;
+    const double inv_side = B.inv_side;
+    const int64_t nbx = B.nbx, nby = B.nby;
     keys_and_hist(
         n,
         [&](int64_t i) {
@@ -373,7 +407,7 @@ __global__ void __launch_bounds__(256) k_morton_keys(int64_t n, const MgkPt* __r
             by = by < 0 ? 0 : (by >= nby ? nby - 1 : by);
             return spread16((unsigned)bx) | (spread16((unsigned)by) << 1);
         },
-        db, passes, keys, hist);
+        db, passes, B.keys, B.hist);
 }
 
 // ---- halo selection: the points inside a rectangle, in input order -------
@@ -487,44 +521,102 @@ static unsigned key_grid(const mgk_ctx* ctx, int64_t n) {
 
 int64_t mgk_points_select_scratch(int64_t n) { return (n + kSelTile - 1) / kSelTile + 1; }
 
-// Positions of the index records in Z-order of their bins (stable: records
-// of one bin keep their order).  Consecutive runs of this order are compact
-// in both directions, unlike runs of the row-major record order.
-int mgk_index_zorder(mgk_ctx* ctx, const mgk_index* idx, int32_t* d_order) {
-    const int64_t n = idx->n;
-    if (n == 0) return MGK_OK;
-    if (idx->nbx > 65536 || idx->nby > 65536) return mgk_fail(ctx, MGK_ERR_INVALID, "index_zorder: bin grid too large");
-    cudaStream_t s = ctx->stream;
-    const uint64_t maxb = (uint64_t)std::max(idx->nbx, idx->nby) - 1;
+// One index's sort scratch: two key buffers, a value buffer, and the zeroed
+// digit counts and state words.
+struct SortBuf {
+    unsigned *k0, *k1;
+    int32_t* v0;
+    unsigned* scr;
+};
+
+static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+static SortPlan bin_plan(int64_t n, int64_t nbins) {
+    int bits = 0;
+    while (bits < 32 && ((uint64_t)(nbins - 1) >> bits) != 0) bits++;
+    return sort_plan(n, bits);
+}
+
+static SortPlan zorder_plan(int64_t n, int64_t nbx, int64_t nby) {
+    const uint64_t maxb = (uint64_t)std::max(nbx, nby) - 1;
     int bits = 0;
     while (bits < 16 && (maxb >> bits) != 0) bits++;
-    const SortPlan P = sort_plan(n, 2 * bits);
-    const size_t b_keys = sizeof(unsigned) * (size_t)n, b_vals = sizeof(int32_t) * (size_t)n, b_scr = P.bytes();
-    unsigned *k0 = nullptr, *k1 = nullptr;
-    int32_t* v0 = nullptr;
-    void* scr = nullptr;
-    int st;
-    if ((st = mgk_alloc(ctx, (void**)&k0, b_keys)) || (st = mgk_alloc(ctx, (void**)&k1, b_keys)) ||
-        (st = mgk_alloc(ctx, (void**)&v0, b_vals)) || (st = mgk_alloc(ctx, &scr, b_scr))) {
-        mgk_free(ctx, k0, b_keys);
-        mgk_free(ctx, k1, b_keys);
-        mgk_free(ctx, v0, b_vals);
-        return st;
+    return sort_plan(n, 2 * bits);
+}
+
+// The records, their permutation and the bin starts of nj indexes of the same
+// points, sorted by plan P (digits enough for the largest bin grid).
+template <int N>
+static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh, int nj, mgk_index* const* idx,
+                                 const SortBuf* buf, const SortPlan& P) {
+    const int64_t n = pts->n;
+    cudaStream_t s = ctx->stream;
+    const bool odd = P.passes & 1;  // the values end in perm
+    int64_t nbins = 0;
+    Jobs<KeyJob, N> K{};
+    Jobs<SortJob, N> S{};
+    Jobs<StartJob, N> T{};
+    Jobs<GatherJob, N> G{};
+    for (int j = 0; j < nj; j++) {
+        const mgk_index* I = idx[j];
+        const SortBuf& b = buf[j];
+        nbins = std::max(nbins, I->nbx * I->nby);
+        K.j[j] = KeyJob{1.0 / I->side, I->nbx, I->nby, nullptr, b.k0, b.scr};
+        S.j[j] = SortJob{b.k0, b.k1, odd ? b.v0 : I->perm, odd ? I->perm : b.v0, b.scr};
+        T.j[j] = StartJob{odd ? b.k1 : b.k0, I->nbx * I->nby, I->bin_start};
+        G.j[j] = GatherJob{I->perm, I->pts, I->qexp};
     }
-    cudaError_t e = cudaMemsetAsync(scr, 0, b_scr, s);
-    if (e == cudaSuccess) {
-        k_morton_keys<<<key_grid(ctx, n), 256, 0, s>>>(n, idx->pts, idx->ox, idx->oy, 1.0 / idx->side, idx->nbx,
-                                                       idx->nby, P.db, P.passes, k0, sort_hist(scr));
-        const bool odd = P.passes & 1;  // the values end in d_order
-        sort_passes(s, P, n, k0, odd ? v0 : d_order, k1, odd ? d_order : v0, scr, ctx->d_map);
-        e = cudaGetLastError();
+    const unsigned ny = (unsigned)nj;
+    k_bin_keys<N><<<dim3(key_grid(ctx, n), ny), 256, 0, s>>>(n, pts->x, pts->y, idx[0]->ox, idx[0]->oy, P.db, P.passes,
+                                                             K);
+    sort_passes<N>(s, P, n, nj, S, ctx->d_map);
+    if (nbins < (1 << 20))
+        k_bin_starts<1, N><<<dim3((unsigned)(nbins / 256 + 1), ny), 256, 0, s>>>(n, T);
+    else
+        k_bin_starts<8, N><<<dim3((unsigned)(nbins / 2048 + 1), ny), 256, 0, s>>>(n, T);
+    k_gather<N><<<dim3((unsigned)((n + 255) / 256), ny), 256, 0, s>>>(
+        n, pts->x, pts->y, pts->w, pts->has_ew ? pts->ew : nullptr, varh ? pts->h : nullptr, G);
+    MGK_COUNT_LAUNCH(ctx, 3 + P.passes);
+    return cudaGetLastError();
+}
+
+// Positions of the records of nj indexes in Z-order of their bins (stable:
+// records of one bin keep their order).  Consecutive runs of this order are
+// compact in both directions, unlike runs of the row-major record order.
+template <int N>
+static cudaError_t enqueue_zorder(mgk_ctx* ctx, int nj, mgk_index* const* idx, int32_t* const* order,
+                                  const SortBuf* buf, const SortPlan& P) {
+    const int64_t n = idx[0]->n;
+    const bool odd = P.passes & 1;  // the values end in order
+    Jobs<KeyJob, N> K{};
+    Jobs<SortJob, N> S{};
+    for (int j = 0; j < nj; j++) {
+        const mgk_index* I = idx[j];
+        const SortBuf& b = buf[j];
+        K.j[j] = KeyJob{1.0 / I->side, I->nbx, I->nby, I->pts, b.k0, b.scr};
+        S.j[j] = SortJob{b.k0, b.k1, odd ? b.v0 : order[j], odd ? order[j] : b.v0, b.scr};
     }
+    k_morton_keys<N><<<dim3(key_grid(ctx, n), (unsigned)nj), 256, 0, ctx->stream>>>(n, idx[0]->ox, idx[0]->oy, P.db,
+                                                                                    P.passes, K);
+    sort_passes<N>(ctx->stream, P, n, nj, S, ctx->d_map);
     MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
+    return cudaGetLastError();
+}
+
+// Z-order of one index's records.
+static int index_zorder(mgk_ctx* ctx, mgk_index* idx, int32_t* d_order) {
+    const int64_t n = idx->n;
+    const SortPlan P = zorder_plan(n, idx->nbx, idx->nby);
+    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
+    char* base = nullptr;
+    int st;
+    if ((st = mgk_alloc(ctx, (void**)&base, need))) return st;
+    const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
+                    (unsigned*)(base + 3 * b_buf)};
+    cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), ctx->stream);
+    if (e == cudaSuccess) e = enqueue_zorder<1>(ctx, 1, &idx, &d_order, &b, P);
     // back to the context's pool; later users are ordered after these kernels on the same stream
-    mgk_free(ctx, k0, b_keys);
-    mgk_free(ctx, k1, b_keys);
-    mgk_free(ctx, v0, b_vals);
-    mgk_free(ctx, scr, b_scr);
+    mgk_free(ctx, base, need);
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index_zorder");
     return MGK_OK;
 }
@@ -578,11 +670,11 @@ int mgk_sort_check(mgk_ctx* ctx) {
     return mgk_fail(ctx, MGK_ERR_TIMEOUT, "index sort: a wait for an earlier tile timed out");
 }
 
+// An index's numbers and its arrays, without the kernels that fill them.
 // extent: the points' (with per-point h: their largest h too) if known, else null.
-int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
-                           mgk_index* idx) {
+static int index_plan(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
+                      mgk_index* idx) {
     const int64_t n = pts->n;
-    cudaStream_t s = ctx->stream;
     idx->ctx = ctx;
     idx->n = n;
     idx->varh = (h <= 0.0f);
@@ -631,44 +723,99 @@ int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float b
     if ((st = mgk_alloc(ctx, (void**)&idx->pts, b_pts))) return st;
     if ((st = mgk_alloc(ctx, (void**)&idx->perm, b_perm))) return st;
     idx->bytes = b_start + b_pts + b_perm;
+    return MGK_OK;
+}
+
+// Fills a planned index.
+static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx) {
+    const int64_t n = pts->n, nbins = idx->nbx * idx->nby;
+    cudaStream_t s = ctx->stream;
     if (n == 0) {
-        MGK_CHECK_CUDA(ctx, cudaMemsetAsync(idx->bin_start, 0, b_start, s));
+        MGK_CHECK_CUDA(ctx, cudaMemsetAsync(idx->bin_start, 0, sizeof(int32_t) * (size_t)(nbins + 1), s));
         return MGK_OK;
     }
-    // the sort's scratch (two key buffers, one value buffer, digit counts and
-    // state words) lies in the record buffer, which the gather fills last
-    int bits = 0;
-    while (bits < 32 && ((uint64_t)(nbins - 1) >> bits) != 0) bits++;
-    const SortPlan P = sort_plan(n, bits);
-    auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
+    // the sort's scratch lies in the record buffer, which the gather fills last
+    const SortPlan P = bin_plan(n, nbins);
     const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
     char* base = reinterpret_cast<char*>(idx->pts);
     void* own = nullptr;
-    if (need > b_pts) {  // few points: a buffer of its own
+    int st;
+    if (need > sizeof(MgkPt) * (size_t)n) {  // few points: a buffer of its own
         if ((st = mgk_alloc(ctx, &own, need))) return st;
         base = static_cast<char*>(own);
     }
-    unsigned *k0 = reinterpret_cast<unsigned*>(base), *k1 = reinterpret_cast<unsigned*>(base + b_buf);
-    int32_t* v0 = reinterpret_cast<int32_t*>(base + 2 * b_buf);
-    void* scr = base + 3 * b_buf;
-    const unsigned gn = (unsigned)((n + 255) / 256);
-    cudaError_t e = cudaMemsetAsync(scr, 0, P.bytes(), s);
-    if (e == cudaSuccess) {
-        k_bin_keys<<<key_grid(ctx, n), 256, 0, s>>>(n, pts->x, pts->y, idx->ox, idx->oy, 1.0 / side, idx->nbx, idx->nby,
-                                                    P.db, P.passes, k0, sort_hist(scr));
-        const bool odd = P.passes & 1;  // the values end in perm
-        sort_passes(s, P, n, k0, odd ? v0 : idx->perm, k1, odd ? idx->perm : v0, scr, ctx->d_map);
-        const unsigned* sorted = odd ? k1 : k0;
-        if (nbins < (1 << 20))
-            k_bin_starts<1><<<(unsigned)(nbins / 256 + 1), 256, 0, s>>>(n, sorted, nbins, idx->bin_start);
-        else
-            k_bin_starts<8><<<(unsigned)(nbins / 2048 + 1), 256, 0, s>>>(n, sorted, nbins, idx->bin_start);
-        k_gather<<<gn, 256, 0, s>>>(n, idx->perm, pts->x, pts->y, pts->w, pts->has_ew ? pts->ew : nullptr,
-                                    idx->varh ? pts->h : nullptr, idx->qexp, idx->pts);
-        e = cudaGetLastError();
-        MGK_COUNT_LAUNCH(ctx, 3 + P.passes);
-    }
+    const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
+                    (unsigned*)(base + 3 * b_buf)};
+    cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), s);
+    if (e == cudaSuccess) e = enqueue_build<1>(ctx, pts, idx->varh, 1, &idx, &b, P);
     if (own) mgk_free(ctx, own, need);  // later users are ordered after these kernels on the same stream
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index build");
+    return MGK_OK;
+}
+
+int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
+                           mgk_index* idx) {
+    const int st = index_plan(ctx, pts, h, bin_size, extent, idx);
+    return st ? st : index_fill(ctx, pts, idx);
+}
+
+// The indexes of a bandwidth batch: bin sides side0 2^l for l < nlev, up to and
+// including the first whose side the bin-count limit raised to the one before,
+// each with the Z-order of its records.  All levels go through each kernel
+// together: one level's kernels on 2,000 points are 8 CTAs and 3 to 8 us each,
+// mostly launch and the chain of a tile's loads, so six levels one after the
+// other took 210 us of the device in 42 launches.  Together they are 9
+// launches: 16 bandwidths scored on 2,000 points 500 -> 281 us, a golden-section
+// search on 20,000 points (seven levels) 3.91 -> 3.56 ms.
+// From 2^19 points a level fills the GPU by itself, and the levels go one
+// after the other, as they do without the memory for all levels' scratch.
+int mgk_index_build_levels(mgk_ctx* ctx, const mgk_points* pts, float h, double side0, int nlev,
+                           const mgk_extent* extent, std::vector<mgk_index*>* lev, std::vector<int32_t*>* order) {
+    const int64_t n = pts->n;
+    int st;
+    SortPlan P{}, Z{};
+    size_t nl = 0;
+    for (int l = 0; l < nlev; l++) {
+        mgk_index* I = new (std::nothrow) mgk_index();
+        if (!I) return mgk_fail(ctx, MGK_ERR_INVALID, "index levels: out of host memory");
+        if ((st = index_plan(ctx, pts, h, (float)std::ldexp(side0, l), extent, I))) {
+            mgk_index_destroy(I);
+            return st;
+        }
+        lev->push_back(I);
+        int32_t* q = nullptr;
+        if ((st = mgk_alloc(ctx, (void**)&q, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)))) return st;
+        order->push_back(q);
+        nl++;
+        if (l == 0) {  // the finest level has the most bins
+            P = bin_plan(n, I->nbx * I->nby);
+            Z = zorder_plan(n, I->nbx, I->nby);
+        } else if (I->side <= (*lev)[l - 1]->side) {
+            break;
+        }
+    }
+    const size_t zp = up256(P.bytes()), zz = up256(Z.bytes()), zero = nl * (zp + zz);
+    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = zero + nl * 3 * b_buf;
+    char* base = nullptr;
+    if (n == 0 || n >= (1 << 19) || nl == 1 || nl > kBuildLevels || mgk_alloc(ctx, (void**)&base, need)) {
+        for (size_t l = 0; l < nl; l++) {
+            if ((st = index_fill(ctx, pts, (*lev)[l]))) return st;
+            if (n > 0 && (st = index_zorder(ctx, (*lev)[l], (*order)[l]))) return st;
+        }
+        return MGK_OK;
+    }
+    SortBuf bp[kBuildLevels], bz[kBuildLevels];
+    for (size_t l = 0; l < nl; l++) {
+        char* keys = base + zero + l * 3 * b_buf;
+        bp[l] = SortBuf{(unsigned*)keys, (unsigned*)(keys + b_buf), (int32_t*)(keys + 2 * b_buf),
+                        (unsigned*)(base + l * zp)};
+        bz[l] = bp[l];
+        bz[l].scr = (unsigned*)(base + nl * zp + l * zz);
+    }
+    cudaError_t e = cudaMemsetAsync(base, 0, zero, ctx->stream);
+    if (e == cudaSuccess) e = enqueue_build<kBuildLevels>(ctx, pts, false, (int)nl, lev->data(), bp, P);
+    if (e == cudaSuccess) e = enqueue_zorder<kBuildLevels>(ctx, (int)nl, lev->data(), order->data(), bz, Z);
+    mgk_free(ctx, base, need);  // later users are ordered after these kernels on the same stream
+    if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index levels");
     return MGK_OK;
 }

@@ -596,23 +596,7 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     const int nlev = std::min(kMaxLev, 1 + std::max(0, (int)std::ceil(std::log2((double)h_hi / (double)h_lo))));
     mgk_extent ext;
     st = mgk_points_extent(c, &view, false, &ext);
-    for (int l = 0; l < nlev && st == MGK_OK; l++) {
-        const float side = (float)(0.75 * (double)h_lo * std::ldexp(1.0, l));
-        mgk_index* idx = nullptr;
-        st = mgk_index_build_async(c, &view, h_lo, side, &ext, &idx);
-        if (st == MGK_OK) {
-            B->lev.push_back(idx);
-            int32_t* q = nullptr;
-            st = mgk_alloc(c, (void**)&q, sizeof(int32_t) * (size_t)std::max<int64_t>(p->n, 1));
-            if (st == MGK_OK) {
-                B->qord.push_back(q);
-                st = mgk_index_zorder(c, idx, q);
-            }
-            if (st) break;
-            // levels whose side was raised to the bin-count limit repeat the previous one
-            if (l > 0 && idx->side <= B->lev[l - 1]->side) break;
-        }
-    }
+    if (st == MGK_OK) st = mgk_index_build_levels(c, &view, h_lo, 0.75 * (double)h_lo, nlev, &ext, &B->lev, &B->qord);
     const size_t n1 = (size_t)std::max<int64_t>(p->n, 1);
     B->bytes_ew = r ? sizeof(float) * n1 * (size_t)nh : 16;
     B->bytes_part = sizeof(double) * (size_t)nh * (size_t)std::max(B->gcount, 1) * kLooSub;

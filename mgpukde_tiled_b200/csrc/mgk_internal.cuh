@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <map>
 #include <string>
+#include <vector>
 
 #include "../../include/mgk.h"
 
@@ -328,8 +329,10 @@ int mgk_index_build_async(mgk_ctx* ctx, const mgk_points* pts, float h, float bi
 // The index records' weights from the points' current edge weights (an index
 // built before the edge weights were known), stream-ordered on ctx->stream.
 int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pts);
-// d_order[k] = position of the k-th record of idx in Z-order of the bins (n entries, device).
-int mgk_index_zorder(mgk_ctx* ctx, const mgk_index* idx, int32_t* d_order);
+// Indexes with bin sides side0 2^l (l < nlev, fewer when the bin-count limit raises a side) and for each
+// the positions of its records in Z-order of the bins; what is made before a failure is the caller's to free.
+int mgk_index_build_levels(mgk_ctx* ctx, const mgk_points* pts, float h, double side0, int nlev,
+                           const mgk_extent* extent, std::vector<mgk_index*>* lev, std::vector<int32_t*>* order);
 int mgk_launch_density(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* g, int64_t row0,
                        int64_t col0, int64_t nr, int64_t nc, const float* d_mask, float* d_out,
                        unsigned long long* d_evals, bool fp64);
