@@ -27,6 +27,15 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kMaxDigits = 512;   // digits of up to 9 bits: 18-bit bin ids sort in two passes
 constexpr int kMaxPasses = 4;     // 32-bit keys
 constexpr long long kSortSpin = 1ll << 24;
+// Bins up to which the gather fills the bin starts on its way instead of a
+// kernel of searches (9 to 12 us of chained loads whatever the size).  A gap
+// between two points can be all bins, which one warp then fills: 2^16 take it
+// about as long as the searches.  Index builds on the way / by searches:
+// 50,000 points in 7,600 bins 64 / 72 us, 200,000 in 2,000 70 / 83 us; a line at
+// 2^12 or 2^18 is no faster.  With 2^19 points and more the build takes 120 us
+// and up, and the sorted keys, which must outlive the gather's stores, stay in
+// the record buffer instead of one of their own.
+constexpr int64_t kFillBins = 1 << 16;
 constexpr int kBuildLevels = 16;  // indexes built together
 constexpr int kExtentCtas = 512;  // their words fit the context's mapped page
 
@@ -53,9 +62,12 @@ struct StartJob {
     int32_t* start;
 };
 struct GatherJob {
-    const int32_t* perm;
+    int32_t* perm;
     MgkPt* out;
     int qexp;
+    const unsigned* keys;  // the sorted keys, where the gather fills the bin starts, else null
+    unsigned nbins;
+    int32_t* start;
 };
 
 __device__ __forceinline__ unsigned f2ord(float f) {
@@ -309,6 +321,7 @@ void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, int nj, const Job
 template <int STRETCHES, int N>
 __global__ void __launch_bounds__(256) k_bin_starts(int64_t n, const __grid_constant__ Jobs<StartJob, N> J) {
     const StartJob& B = J.j[N > 1 ? blockIdx.y : 0];
+    if (!B.start) return;  // the gather fills these
     const unsigned* __restrict__ keys = B.keys;
     const int64_t nbins = B.nbins;
     int32_t* __restrict__ start = B.start;
@@ -330,6 +343,27 @@ __global__ void __launch_bounds__(256) k_bin_starts(int64_t n, const __grid_cons
         const int64_t lo = __shfl_sync(0xffffffffu, edge, k), hi = __shfl_sync(0xffffffffu, edge, k + 1);
         const int64_t b = b0 + 32 * k + lane;
         if (b <= nbins) start[b] = (int32_t)first_at(b, lo, hi);
+    }
+}
+
+// The starts of the bins after the key at i - 1, up to the key at i, are i
+// (after the last key: n).  Gaps of more than four bins are filled by the warp.
+__device__ __forceinline__ void fill_starts(int64_t n, int64_t i, const unsigned* __restrict__ keys, unsigned nbins,
+                                            int32_t* __restrict__ start) {
+    const int lane = threadIdx.x & 31;
+    unsigned lo = 0, hi = 0;  // start[lo, hi) = i
+    if (i <= n) {
+        if (i > 0) lo = keys[i - 1] + 1;
+        hi = (i < n ? min(keys[i], nbins - 1) : nbins) + 1;  // in range also after a sort that failed
+    }
+    const bool wide = hi > lo + 4;
+    if (!wide)
+        for (unsigned b = lo; b < hi; b++) start[b] = (int32_t)i;
+    for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const unsigned l = __shfl_sync(0xffffffffu, lo, src), h = __shfl_sync(0xffffffffu, hi, src);
+        const int32_t at = (int32_t)(i - lane + src);
+        for (unsigned b = l + lane; b < h; b += 32) start[b] = at;
     }
 }
 
@@ -357,12 +391,14 @@ __global__ void k_gather(int64_t n, const float* __restrict__ x, const float* __
                          const float* __restrict__ w, const float* __restrict__ ew, const float* __restrict__ hpp,
                          const __grid_constant__ Jobs<GatherJob, N> J) {
     const GatherJob& B = J.j[N > 1 ? blockIdx.y : 0];
-    const int32_t* __restrict__ perm = B.perm;
+    int32_t* __restrict__ perm = B.perm;
     MgkPt* __restrict__ out = B.out;
     const int qexp = B.qexp;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (B.keys) fill_starts(n, i, B.keys, B.nbins, B.start);
     if (i >= n) return;
-    const int32_t j = perm[i];
+    int32_t j = perm[i];
+    if ((unsigned)j >= (unsigned)n) perm[i] = j = 0;  // a place that a failed sort left unwritten
     MgkPt r;
     mgk_qsplit(x[j], qexp, r.xh, r.xl);
     mgk_qsplit(y[j], qexp, r.yh, r.yl);
@@ -545,14 +581,17 @@ static SortPlan zorder_plan(int64_t n, int64_t nbx, int64_t nby) {
 }
 
 // The records, their permutation and the bin starts of nj indexes of the same
-// points, sorted by plan P (digits enough for the largest bin grid).
+// points, sorted by plan P (digits enough for the largest bin grid).  own: the
+// scratch is not the record buffer, so the sorted keys outlive the gather's
+// first stores.
 template <int N>
 static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh, int nj, mgk_index* const* idx,
-                                 const SortBuf* buf, const SortPlan& P) {
+                                 const SortBuf* buf, bool own, const SortPlan& P) {
     const int64_t n = pts->n;
     cudaStream_t s = ctx->stream;
     const bool odd = P.passes & 1;  // the values end in perm
     int64_t nbins = 0;
+    bool search = false;  // for some index's bin starts
     Jobs<KeyJob, N> K{};
     Jobs<SortJob, N> S{};
     Jobs<StartJob, N> T{};
@@ -564,19 +603,26 @@ static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh,
         K.j[j] = KeyJob{1.0 / I->side, I->nbx, I->nby, nullptr, b.k0, b.scr};
         S.j[j] = SortJob{b.k0, b.k1, odd ? b.v0 : I->perm, odd ? I->perm : b.v0, b.scr};
         T.j[j] = StartJob{odd ? b.k1 : b.k0, I->nbx * I->nby, I->bin_start};
-        G.j[j] = GatherJob{I->perm, I->pts, I->qexp};
+        G.j[j] = GatherJob{I->perm, I->pts, I->qexp, nullptr, 0u, nullptr};
+        if (own && T.j[j].nbins <= kFillBins) {
+            G.j[j].keys = T.j[j].keys;
+            G.j[j].nbins = (unsigned)T.j[j].nbins;
+            std::swap(G.j[j].start, T.j[j].start);
+        } else {
+            search = true;
+        }
     }
     const unsigned ny = (unsigned)nj;
     k_bin_keys<N><<<dim3(key_grid(ctx, n), ny), 256, 0, s>>>(n, pts->x, pts->y, idx[0]->ox, idx[0]->oy, P.db, P.passes,
                                                              K);
     sort_passes<N>(s, P, n, nj, S, ctx->d_map);
-    if (nbins < (1 << 20))
+    if (search && nbins < (1 << 20))
         k_bin_starts<1, N><<<dim3((unsigned)(nbins / 256 + 1), ny), 256, 0, s>>>(n, T);
-    else
+    else if (search)
         k_bin_starts<8, N><<<dim3((unsigned)(nbins / 2048 + 1), ny), 256, 0, s>>>(n, T);
-    k_gather<N><<<dim3((unsigned)((n + 255) / 256), ny), 256, 0, s>>>(
+    k_gather<N><<<dim3((unsigned)(n / 256 + 1), ny), 256, 0, s>>>(  // a thread past the last record ends the starts
         n, pts->x, pts->y, pts->w, pts->has_ew ? pts->ew : nullptr, varh ? pts->h : nullptr, G);
-    MGK_COUNT_LAUNCH(ctx, 3 + P.passes);
+    MGK_COUNT_LAUNCH(ctx, (search ? 3 : 2) + P.passes);
     return cudaGetLastError();
 }
 
@@ -734,20 +780,23 @@ static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx) {
         MGK_CHECK_CUDA(ctx, cudaMemsetAsync(idx->bin_start, 0, sizeof(int32_t) * (size_t)(nbins + 1), s));
         return MGK_OK;
     }
-    // the sort's scratch lies in the record buffer, which the gather fills last
+    // The sort's scratch lies in the record buffer, which the gather fills
+    // last, or, where the gather fills the bin starts, in a buffer of its own
+    // (while there is memory for it).
     const SortPlan P = bin_plan(n, nbins);
     const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
     char* base = reinterpret_cast<char*>(idx->pts);
     void* own = nullptr;
     int st;
-    if (need > sizeof(MgkPt) * (size_t)n) {  // few points: a buffer of its own
-        if ((st = mgk_alloc(ctx, &own, need))) return st;
-        base = static_cast<char*>(own);
+    const bool fits = need <= sizeof(MgkPt) * (size_t)n;
+    if (!fits || (nbins <= kFillBins && n < (1 << 19))) {
+        if ((st = mgk_alloc(ctx, &own, need)) && !fits) return st;
+        if (own) base = static_cast<char*>(own);
     }
     const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
                     (unsigned*)(base + 3 * b_buf)};
     cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), s);
-    if (e == cudaSuccess) e = enqueue_build<1>(ctx, pts, idx->varh, 1, &idx, &b, P);
+    if (e == cudaSuccess) e = enqueue_build<1>(ctx, pts, idx->varh, 1, &idx, &b, own != nullptr, P);
     if (own) mgk_free(ctx, own, need);  // later users are ordered after these kernels on the same stream
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index build");
     return MGK_OK;
@@ -813,7 +862,7 @@ int mgk_index_build_levels(mgk_ctx* ctx, const mgk_points* pts, float h, double 
         bz[l].scr = (unsigned*)(base + nl * zp + l * zz);
     }
     cudaError_t e = cudaMemsetAsync(base, 0, zero, ctx->stream);
-    if (e == cudaSuccess) e = enqueue_build<kBuildLevels>(ctx, pts, false, (int)nl, lev->data(), bp, P);
+    if (e == cudaSuccess) e = enqueue_build<kBuildLevels>(ctx, pts, false, (int)nl, lev->data(), bp, true, P);
     if (e == cudaSuccess) e = enqueue_zorder<kBuildLevels>(ctx, (int)nl, lev->data(), order->data(), bz, Z);
     mgk_free(ctx, base, need);  // later users are ordered after these kernels on the same stream
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index levels");

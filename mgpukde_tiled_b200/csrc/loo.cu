@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
         for (int i = 0; i < kLooSub; i++) {
             const int64_t qk = q0 + 32 * i + lane;
             if (qk >= P.n) continue;
-            const int qp = L.qord[qk];
+            const int qp = (int)min((unsigned)L.qord[qk], (unsigned)(P.n - 1));  // in range also after a sort that failed
             const float4 v = *reinterpret_cast<const float4*>(pts + qp);
             const float vx = v.x + v.z, vy = v.y + v.w;
             gmnx = fminf(gmnx, vx);
