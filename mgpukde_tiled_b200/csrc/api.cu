@@ -172,11 +172,11 @@ void mgk_free(mgk_ctx* ctx, void* p, size_t bytes) {
 }
 
 int mgk_index_build_async(mgk_ctx* c, const mgk_points* p, float h, float bin_size, const mgk_extent* extent,
-                          mgk_index** out) {
+                          mgk_index** out, int32_t* inv) {
     if (!c || !p || !out) return mgk_fail(c, MGK_ERR_INVALID, "index_build: bad arguments");
     mgk_index* idx = new (std::nothrow) mgk_index();
     if (!idx) return MGK_ERR_INVALID;
-    const int st = mgk_launch_index_build(c, p, h, bin_size, extent, idx);
+    const int st = mgk_launch_index_build(c, p, h, bin_size, extent, idx, inv);
     if (st) {
         mgk_index_destroy(idx);
         return st;

@@ -68,6 +68,7 @@ struct GatherJob {
     const unsigned* keys;  // the sorted keys, where the gather fills the bin starts, else null
     unsigned nbins;
     int32_t* start;
+    int32_t* inv;  // the place of each point's record, or null
 };
 
 __device__ __forceinline__ unsigned f2ord(float f) {
@@ -399,6 +400,7 @@ __global__ void k_gather(int64_t n, const float* __restrict__ x, const float* __
     if (i >= n) return;
     int32_t j = perm[i];
     if ((unsigned)j >= (unsigned)n) perm[i] = j = 0;  // a place that a failed sort left unwritten
+    if (B.inv) B.inv[j] = (int32_t)i;
     MgkPt r;
     mgk_qsplit(x[j], qexp, r.xh, r.xl);
     mgk_qsplit(y[j], qexp, r.yh, r.yl);
@@ -444,6 +446,37 @@ __global__ void __launch_bounds__(256) k_morton_keys(int64_t n, double ox, doubl
             return spread16((unsigned)bx) | (spread16((unsigned)by) << 1);
         },
         db, passes, B.keys, B.hist);
+}
+
+// Place along a Hilbert curve of a point's cell in a 65,536 x 65,536 raster
+// over the extent (quadrant by quadrant, each reflected and rotated as the
+// curve's definition has it).
+__global__ void __launch_bounds__(256) k_hilbert_keys(int64_t n, const float* __restrict__ x,
+                                                      const float* __restrict__ y, double ox, double oy, double scale,
+                                                      int db, int passes, unsigned* __restrict__ keys,
+                                                      unsigned* __restrict__ hist) {
+    keys_and_hist(
+        n,
+        [&](int64_t i) {
+            unsigned u = (unsigned)fmin(fmax(((double)x[i] - ox) * scale, 0.0), 65535.0);
+            unsigned v = (unsigned)fmin(fmax(((double)y[i] - oy) * scale, 0.0), 65535.0);
+            unsigned d = 0;
+            for (int b = 15; b >= 0; b--) {
+                const unsigned ru = (u >> b) & 1u, rv = (v >> b) & 1u;
+                d = (d << 2) | ((3u * ru) ^ rv);
+                if (!rv) {
+                    if (ru) {
+                        u = ~u;
+                        v = ~v;
+                    }
+                    const unsigned t = u;
+                    u = v;
+                    v = t;
+                }
+            }
+            return d;
+        },
+        db, passes, keys, hist);
 }
 
 // ---- halo selection: the points inside a rectangle, in input order -------
@@ -586,7 +619,8 @@ static SortPlan zorder_plan(int64_t n, int64_t nbx, int64_t nby) {
 // first stores.
 template <int N>
 static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh, int nj, mgk_index* const* idx,
-                                 const SortBuf* buf, bool own, const SortPlan& P) {
+                                 const SortBuf* buf, bool own, const SortPlan& P,
+                                 int32_t* inv) {
     const int64_t n = pts->n;
     cudaStream_t s = ctx->stream;
     const bool odd = P.passes & 1;  // the values end in perm
@@ -603,7 +637,7 @@ static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh,
         K.j[j] = KeyJob{1.0 / I->side, I->nbx, I->nby, nullptr, b.k0, b.scr};
         S.j[j] = SortJob{b.k0, b.k1, odd ? b.v0 : I->perm, odd ? I->perm : b.v0, b.scr};
         T.j[j] = StartJob{odd ? b.k1 : b.k0, I->nbx * I->nby, I->bin_start};
-        G.j[j] = GatherJob{I->perm, I->pts, I->qexp, nullptr, 0u, nullptr};
+        G.j[j] = GatherJob{I->perm, I->pts, I->qexp, nullptr, 0u, nullptr, inv};
         if (own && T.j[j].nbins <= kFillBins) {
             G.j[j].keys = T.j[j].keys;
             G.j[j].nbins = (unsigned)T.j[j].nbins;
@@ -649,10 +683,9 @@ static cudaError_t enqueue_zorder(mgk_ctx* ctx, int nj, mgk_index* const* idx, i
     return cudaGetLastError();
 }
 
-// Z-order of one index's records.
-static int index_zorder(mgk_ctx* ctx, mgk_index* idx, int32_t* d_order) {
-    const int64_t n = idx->n;
-    const SortPlan P = zorder_plan(n, idx->nbx, idx->nby);
+// Runs enqueue(scratch) with a sort's zeroed scratch for n items.
+template <typename Enqueue>
+static int with_sort_buf(mgk_ctx* ctx, int64_t n, const SortPlan& P, const char* what, const Enqueue& enqueue) {
     const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
     char* base = nullptr;
     int st;
@@ -660,11 +693,36 @@ static int index_zorder(mgk_ctx* ctx, mgk_index* idx, int32_t* d_order) {
     const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
                     (unsigned*)(base + 3 * b_buf)};
     cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), ctx->stream);
-    if (e == cudaSuccess) e = enqueue_zorder<1>(ctx, 1, &idx, &d_order, &b, P);
+    if (e == cudaSuccess) e = enqueue(b);
     // back to the context's pool; later users are ordered after these kernels on the same stream
     mgk_free(ctx, base, need);
-    if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index_zorder");
+    if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, what);
     return MGK_OK;
+}
+
+// Z-order of one index's records.
+static int index_zorder(mgk_ctx* ctx, mgk_index* idx, int32_t* d_order) {
+    const SortPlan P = zorder_plan(idx->n, idx->nbx, idx->nby);
+    return with_sort_buf(ctx, idx->n, P, "index_zorder",
+                         [&](const SortBuf& b) { return enqueue_zorder<1>(ctx, 1, &idx, &d_order, &b, P); });
+}
+
+int mgk_points_curve_order(mgk_ctx* ctx, const mgk_points* pts, const mgk_extent& extent, int32_t* d_order) {
+    const int64_t n = pts->n;
+    if (n == 0) return MGK_OK;
+    const double ext = std::max(extent.xmax - extent.xmin, extent.ymax - extent.ymin);
+    const SortPlan P = sort_plan(n, 32);
+    return with_sort_buf(ctx, n, P, "points_curve_order", [&](const SortBuf& b) {
+        const bool odd = P.passes & 1;  // the values end in d_order
+        Jobs<SortJob, 1> S{};
+        S.j[0] = SortJob{b.k0, b.k1, odd ? b.v0 : d_order, odd ? d_order : b.v0, b.scr};
+        k_hilbert_keys<<<key_grid(ctx, n), 256, 0, ctx->stream>>>(n, pts->x, pts->y, extent.xmin, extent.ymin,
+                                                                  ext > 0.0 ? 65536.0 / ext : 0.0, P.db, P.passes, b.k0,
+                                                                  b.scr);
+        sort_passes<1>(ctx->stream, P, n, 1, S, ctx->d_map);
+        MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
+        return cudaGetLastError();
+    });
 }
 
 int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pts) {
@@ -773,7 +831,7 @@ static int index_plan(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_si
 }
 
 // Fills a planned index.
-static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx) {
+static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx, int32_t* inv = nullptr) {
     const int64_t n = pts->n, nbins = idx->nbx * idx->nby;
     cudaStream_t s = ctx->stream;
     if (n == 0) {
@@ -796,16 +854,16 @@ static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx) {
     const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
                     (unsigned*)(base + 3 * b_buf)};
     cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), s);
-    if (e == cudaSuccess) e = enqueue_build<1>(ctx, pts, idx->varh, 1, &idx, &b, own != nullptr, P);
+    if (e == cudaSuccess) e = enqueue_build<1>(ctx, pts, idx->varh, 1, &idx, &b, own != nullptr, P, inv);
     if (own) mgk_free(ctx, own, need);  // later users are ordered after these kernels on the same stream
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index build");
     return MGK_OK;
 }
 
 int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
-                           mgk_index* idx) {
+                           mgk_index* idx, int32_t* inv) {
     const int st = index_plan(ctx, pts, h, bin_size, extent, idx);
-    return st ? st : index_fill(ctx, pts, idx);
+    return st ? st : index_fill(ctx, pts, idx, inv);
 }
 
 // The indexes of a bandwidth batch: bin sides side0 2^l for l < nlev, up to and
@@ -862,7 +920,7 @@ int mgk_index_build_levels(mgk_ctx* ctx, const mgk_points* pts, float h, double 
         bz[l].scr = (unsigned*)(base + nl * zp + l * zz);
     }
     cudaError_t e = cudaMemsetAsync(base, 0, zero, ctx->stream);
-    if (e == cudaSuccess) e = enqueue_build<kBuildLevels>(ctx, pts, false, (int)nl, lev->data(), bp, true, P);
+    if (e == cudaSuccess) e = enqueue_build<kBuildLevels>(ctx, pts, false, (int)nl, lev->data(), bp, true, P, nullptr);
     if (e == cudaSuccess) e = enqueue_zorder<kBuildLevels>(ctx, (int)nl, lev->data(), order->data(), bz, Z);
     mgk_free(ctx, base, need);  // later users are ordered after these kernels on the same stream
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, "index levels");

@@ -320,12 +320,15 @@ struct mgk_extent {
 int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_extent* out);
 int mgk_sort_check(mgk_ctx* ctx);
 // Builds the index on ctx->stream without waiting for it (mgk_sort_check after
-// a wait); the points' arrays are read until then.
+// a wait); the points' arrays are read until then.  inv (device, n entries, or
+// null): the place of each point's record.
 int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
-                           mgk_index* idx);
+                           mgk_index* idx, int32_t* inv = nullptr);
 // The same into a new index, for callers that wait later on the same stream.
 int mgk_index_build_async(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
-                          mgk_index** out);
+                          mgk_index** out, int32_t* inv = nullptr);
+// The points (n entries, device) along a Hilbert curve over their extent, stream-ordered.
+int mgk_points_curve_order(mgk_ctx* ctx, const mgk_points* pts, const mgk_extent& extent, int32_t* d_order);
 // The index records' weights from the points' current edge weights (an index
 // built before the edge weights were known), stream-ordered on ctx->stream.
 int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pts);
