@@ -71,10 +71,6 @@ struct GatherJob {
     int32_t* inv;  // the place of each point's record, or null
 };
 
-__device__ __forceinline__ unsigned f2ord(float f) {
-    unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 // The points' extent (and largest h): each CTA's ordered-integer minima and
 // maxima (min x, min y, max x, max y, max h) into its words of mapped host
 // memory, so that no copy goes through a copy engine.
@@ -83,12 +79,12 @@ __global__ void __launch_bounds__(256) k_extent(int64_t n, const float* __restri
     __shared__ unsigned sh[8][5];
     unsigned v[5] = {0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned ox = f2ord(x[i]), oy = f2ord(y[i]);
+        const unsigned ox = mgk_f2ord(x[i]), oy = mgk_f2ord(y[i]);
         v[0] = min(v[0], ox);
         v[1] = min(v[1], oy);
         v[2] = max(v[2], ox);
         v[3] = max(v[3], oy);
-        if (h) v[4] = max(v[4], f2ord(h[i]));
+        if (h) v[4] = max(v[4], mgk_f2ord(h[i]));
     }
 #pragma unroll
     for (int k = 0; k < 5; k++) {
@@ -752,17 +748,11 @@ int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_exte
             const unsigned u = m[5 * b + k];
             v[k] = k < 2 ? std::min(v[k], u) : std::max(v[k], u);
         }
-    auto o2f = [](unsigned u) {
-        unsigned w = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
-        float f;
-        memcpy(&f, &w, 4);
-        return f;
-    };
-    out->xmin = o2f(v[0]);
-    out->ymin = o2f(v[1]);
-    out->xmax = o2f(v[2]);
-    out->ymax = o2f(v[3]);
-    if (want_h) out->hmax = o2f(v[4]);
+    out->xmin = mgk_ord2f(v[0]);
+    out->ymin = mgk_ord2f(v[1]);
+    out->xmax = mgk_ord2f(v[2]);
+    out->ymax = mgk_ord2f(v[3]);
+    if (want_h) out->hmax = mgk_ord2f(v[4]);
     return MGK_OK;
 }
 

@@ -38,7 +38,6 @@ struct mgk_ctx {
     unsigned long long* d_counter = nullptr;  // 8 counters
     unsigned long long* h_counter = nullptr;  // pinned mirror
     double* d_sum = nullptr;                  // 256 doubles
-    double* h_sum = nullptr;                  // pinned mirror
     // mapped page-locked staging of plans and counts (mgk_host_stage), in
     // kStageSlots independent slots; h_stage[i] and d_stage[i] address the same
     // bytes.  Slot 3 holds the bit-packed density mask of mgk_kde_raster.
@@ -47,7 +46,8 @@ struct mgk_ctx {
     void* d_stage[kStageSlots] = {};
     size_t h_stage_bytes[kStageSlots] = {};
     // a small mapped page-locked page: word 0 the index sort's wait flag, words
-    // 64.. the extents of k_extent's CTAs
+    // 32 and 33 an adaptive likelihood (a double), words 64.. the extents of
+    // k_extent's CTAs or the largest h of k_adaptive_h's
     unsigned *h_map = nullptr, *d_map = nullptr;
     mgk_raster_pipe* pipe = nullptr;
     std::multimap<size_t, void*> pool;        // cached device blocks by size class
@@ -310,6 +310,18 @@ __device__ __host__ __forceinline__ void mgk_qsplit(float v, int qexp, float& hi
 __device__ __host__ __forceinline__ double mgk_h2(float h) {
     const float hh = h * h;
     return (double)hh;
+}
+
+// Floats as unsigned integers in the same order, and back.
+__device__ __forceinline__ unsigned mgk_f2ord(float f) {
+    const unsigned u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+inline float mgk_ord2f(unsigned u) {
+    u = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
+    float f;
+    memcpy(&f, &u, 4);
+    return f;
 }
 
 // ---- kernels launched across translation units ------------------------------
