@@ -610,17 +610,21 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_counter, sizeof(unsigned));
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_evals, 2 * sizeof(unsigned long long));
     if (st == MGK_OK) st = mgk_alloc(c, (void**)&B->d_lev, sizeof(LevelDesc) * kMaxLev);
-    // Parts of a group's candidates: enough work items for about two rounds of
-    // the resident CTAs (a golden-section step on 20,000 points has 314
-    // groups, 2 a CTA slot's quarter).  From the whole problem's groups, so a
-    // share of it sums each query as the whole does.
+    // Parts of a group's candidates: enough work items for about four rounds of
+    // the resident warps (a golden-section step on 20,000 points has 1,256 items
+    // for 2,368 warps, the dense groups' the longest: 3.33 ms per search with
+    // four rounds, 3.41 with three, 3.57 with two, 4.12 with one), for two below
+    // 2^13 points, whose items are short (16 bandwidths on 2,000 points 281 us
+    // with two, 283 with four; 8,000 points the same with both).  From the whole
+    // problem's groups, so a share of it sums each query as the whole does.
     int nsplit = 1;
     int occ = 1;
     if (st == MGK_OK && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_loo_multi, kLooWarps * 32, 0) != cudaSuccess)
         st = mgk_fail(c, MGK_ERR_CUDA, "loo batch: occupancy");
     const int64_t resident = (int64_t)c->sm_count * std::max(occ, 1) * kLooWarps;  // warps
     const int64_t items = (int64_t)nh * std::max(B->ngroups, 1) * kLooSub;
-    if (items < 2 * resident) nsplit = (int)std::min<int64_t>(kMaxSplit, (2 * resident + items - 1) / items);
+    const int64_t want = (p->n < (1 << 13) ? 2 : 4) * resident;
+    if (items < want) nsplit = (int)std::min<int64_t>(kMaxSplit, (want + items - 1) / items);
     if (st == MGK_OK && nsplit > 1) {
         B->bytes_psum = sizeof(double) * (size_t)nsplit * (size_t)nh * (size_t)std::max(B->gcount, 1) * kLooQ;
         if (mgk_alloc(c, (void**)&B->d_psum, B->bytes_psum)) nsplit = 1;  // no memory: whole groups
