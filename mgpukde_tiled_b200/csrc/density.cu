@@ -12,7 +12,7 @@
 // NoData stages no candidates and writes NoData (the reference skips NoData
 // cells, kde_kernel_kdtr.cu:426-428).  Candidates (points of the bins within
 // 3h of the block, one contiguous range per bin row) arrive in mini-batches
-// of 64, taken by two cursors across bin rows, through a double-buffered TMA
+// of 64, taken by one cursor across bin rows, through a double-buffered TMA
 // bulk copy (cp.async.bulk + mbarrier) into shared memory; the next batch is
 // staged during the current batch's phase B by the warp with the fewest
 // points to sum.  Per mini-batch:
@@ -38,8 +38,8 @@
 // into a Kahan-compensated FP32 accumulator in tensor memory (tcgen05: 128
 // columns per CTA, sum and compensation of each thread's 32 cells in 64
 // columns of its warp's lane quarter); the epilogue forms (s - c) times the
-// kernel normalisation in FP64.  With 126-128 registers per thread two CTAs
-// run per SM.  Heavy blocks are split into work items whose FP64 partials
+// kernel normalisation in FP64.  With 80 registers per thread three CTAs run
+// per SM.  Heavy blocks are split into work items whose FP64 partials
 // are merged in a fixed order, so results are bitwise reproducible.
 #include <algorithm>
 #include <cstring>
@@ -388,7 +388,10 @@ __device__ __forceinline__ unsigned amb_row(float s2, float eps_d2, float pc0, f
 // warps' phase-B work per batch; with one, neighbouring points share their
 // branches in phase A.  Since three CTAs share an SM (the others issue while
 // one waits at a batch barrier) one cursor is the faster: 8.01 ms on the C1
-// raster against 8.34 ms with two and 8.42 ms with eight.
+// raster against 8.34 ms with two and 8.42 ms with eight.  The batch is filled
+// by one thread: filled by a whole warp from a table of the rows' ranges it took
+// 3.01 ms instead of 3.12 on eight mixed tiles in one launch, but 9.4 instead
+// of 9.0 ms on the C1 study, whose registers it pushes over 80.
 #ifndef MGK_DENSITY_NCUR
 #define MGK_DENSITY_NCUR 1
 #endif
@@ -1204,8 +1207,9 @@ void fill_params(DParams& P, const mgk_index* idx, const mgk_grid* g, int64_t ro
 // Work items of one tile from its per-block candidate counts: blocks above K
 // candidates are split into items of at most K, each split item writing an
 // FP64 partial into its own scratch slot (fine: small tiles are split finer;
-// without the memory for that, coarsely).  K depends on this tile alone, so a tile gets the same items
-// (and bitwise the same result) alone or batched with others.
+// without the memory for that, coarsely).  K depends on this tile alone, so a
+// tile gets the same items (and bitwise the same result) alone or batched with
+// others.
 struct TilePlan {
     int nbx_t = 0, nby_t = 0;
     std::vector<Item> items;
