@@ -860,8 +860,8 @@ def run_bandwidth_select(args):
            "batch_ms": float(np.mean(loo_ms)), "argmax": best, "h_best": float(hgrid[best]),
            "gpu_launches": launches, "clocks": clocks,
            "roofline": algo_roofline(evals, float(np.mean(loo_ms)) / 1e3,
-                                     "one LOO batch: per-h edge weights, k_loo_multi (about 90 % of it), prep, "
-                                     "finish and argmax (the batch's CUDA-event time)", local)}
+                                     "one LOO batch: per-h edge weights, k_loo_multi (about 90 % of it), prep "
+                                     "and finish (the batch's CUDA-event time)", local)}
     if rank == 0:
         if world == 1:
             unbind_numa()
