@@ -57,6 +57,7 @@ constexpr int kBC = 128;        // cell columns of a CTA block
 constexpr int kCells = kBR * kBC;
 constexpr int kMergeParts = 8;  // CTAs per split block in the merge kernels (kCells / 8 cells each)
 constexpr int kMB = 64;         // points per mini-batch (a multiple of 32)
+static_assert(kMB == 64, "plan_tile shifts by 6");
 constexpr int kStage64 = 512;   // points staged per batch by the FP64 form
 constexpr float kAmbEps = 4e-6f;
 constexpr long long kSpinLimit = 1ll << 24;
@@ -1235,6 +1236,24 @@ void plan_tile(const int64_t* counts, int nbx_t, int nby_t, int sm_count, int wa
         !fine ? 2048 : std::min<int64_t>(2048, std::max<int64_t>(256, total / (2 * slots_resident)));
     int64_t K = std::max<int64_t>(least, total / std::max<int64_t>(1, slots_resident * waves));
     K = (K + kMB - 1) / kMB * kMB;
+    // A tile that leaves slots empty even when split batch by batch, or two by
+    // two, is split so where a block has more than twice that: its time is the
+    // longest block's, 10 us a batch, and a merge's.  2,000 points on 600 x 500
+    // cells 240 -> 214 us, 5,000 on 900 x 700 246 -> 222, a study of 8,000 with
+    // per-point h 1.14 -> 1.10 ms; blocks of two batches gain nothing, halves of
+    // a batch neither.  (Small tiles among large ones in one launch merge for
+    // nothing: 3.11 -> 3.13 ms for eight, whose plans are the same as alone.)
+    if (fine && nblk <= slots_resident) {
+        int64_t ones = 0, twos = 0, most = 0;
+        for (int b = 0; b < nblk; b++) {
+            const int64_t m = std::max<int64_t>(1, (counts[b] + kMB - 1) >> 6);
+            ones += m;
+            twos += (m + 1) >> 1;
+            most = std::max(most, m);
+        }
+        if (ones <= slots_resident && most > 2) K = kMB;
+        else if (twos <= slots_resident && most > 4) K = 2 * kMB;
+    }
     T.items.reserve(nblk + 16);
     for (int b = 0; b < nblk; b++) {
         const int64_t c = counts[b];
