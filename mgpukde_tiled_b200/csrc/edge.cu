@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kEdgeWarps * 32, 6) k_edge_rows(EdgeParams E) 
             const float hp = VARH ? E.hpp[p] : (E.hgrid ? E.hgrid[k] : E.hfix);
             h2_l = mgk_h2(hp);
             out = E.ew + k * E.ew_stride + p;
-            need = !E.dist2 || E.dist2[p] < MGK_CUT * h2_l;
+            need = !E.dist2 || !(E.dist2[p] >= MGK_CUT * h2_l);  // (a NaN bandwidth gives a NaN weight)
             if (!need) *out = 1.0f;
             if (need) {
                 fpx = E.x[p];
