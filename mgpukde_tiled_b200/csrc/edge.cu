@@ -293,14 +293,16 @@ __global__ void __launch_bounds__(kEdgeWarps * 32, 6) k_edge_rows(EdgeParams E) 
                     const float fl = fcol - tc, fh = fcol + tc;
                     const float il = ceilf(fl), ih = floorf(fh);
                     const float m = __fmaf_rn(1e-6f, tc, E.margin);
-                    int lo = icol + (int)il, hi = icol + (int)ih;
-                    if (il - fl < m || il - fl > 1.0f - m || fh - ih < m || fh - ih > 1.0f - m || tc < 2.0f * m) {
-                        const int2 ex = exact_interval(E.cx, c0, c1, lo, hi, px, dy2, cut);
+                    int lo, hi;
+                    // (false too where the chord has left FP32 and the differences are NaN)
+                    if (il - fl >= m && il - fl <= 1.0f - m && fh - ih >= m && fh - ih <= 1.0f - m && tc >= 2.0f * m) {
+                        lo = max(icol + (int)il, c0);
+                        hi = min(icol + (int)ih, c1);
+                    } else {
+                        const int2 ex = exact_interval(E.cx, c0, c1, icol + (int)fmaxf(il, -1.0e9f),
+                                                       icol + (int)fminf(ih, 1.0e9f), px, dy2, cut);
                         lo = ex.x;
                         hi = ex.y;
-                    } else {
-                        lo = max(lo, c0);
-                        hi = min(hi, c1);
                     }
                     if (lo > hi) continue;
                     // valid runs of the row clipped to [lo, hi]

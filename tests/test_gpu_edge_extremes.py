@@ -39,3 +39,14 @@ def test_nan_bandwidth_gives_nan_weights():
     got = weights(x, y, g, m, 0.0, hs)
     bad = np.isnan(hs)
     assert np.isnan(got[bad]).all() and np.array_equal(got[~bad], ref[~bad])
+
+
+@pytest.mark.parametrize("varh", [False, True])
+@pytest.mark.parametrize("h", [1e18, 6.0e18, 6.2e18, 9.0e18, 1.8e19])
+def test_reach_beyond_fp32(h, varh):
+    """9 h^2 is above FP32's range from h = 6.15e18, h^2 itself from 1.84e19."""
+    x, y, g, m = study()
+    got = weights(x, y, g, m, 0.0 if varh else h, np.full(len(x), h, np.float32) if varh else None)
+    h2 = float(np.float32(h) * np.float32(h))
+    ref = h2 * float(np.float32(6.283185307179586)) / (m == 1.0).sum()
+    assert np.all(np.abs(got - ref) <= 1e-6 * ref)
