@@ -246,8 +246,10 @@ __global__ void __launch_bounds__(kEdgeWarps * 32, 6) k_edge_rows(EdgeParams E) 
             const int64_t rl = __shfl_sync(0xffffffffu, rl_l, src), ru = __shfl_sync(0xffffffffu, ru_l, src);
             double acc = 0.0;
             unsigned long long cnt = 0;
-            for (int c0 = cl; c0 <= cu && rl <= ru; c0 += kEdgeChunk) {
-                const int c1 = min(cu, c0 + kEdgeChunk - 1);
+            // (counted from cl: a column beyond the last chunk may not fit 32 bits)
+            const int width = rl <= ru ? cu - cl + 1 : 0;
+            for (int done = 0; done < width; done += min(kEdgeChunk, width - done)) {
+                const int c0 = cl + done, c1 = c0 + min(kEdgeChunk, width - done) - 1;
                 const int len = c1 - c0 + 1;
                 // the column factors, then their prefix sums: Q[j] = sum of the first j
 #pragma unroll 2
