@@ -717,7 +717,8 @@ int mgk_launch_dist2(mgk_ctx* ctx, mgk_points* p, mgk_raster* r, double cap) {
         const unsigned parts = (unsigned)std::max<int64_t>(
             1, std::min<int64_t>((r->nb + 255) / 256, 4 * (int64_t)ctx->sm_count / (int64_t)gp));
         cudaError_t e = cudaSuccess;
-        if (parts > 1) e = cudaMemsetAsync(p->dist2, 0x7f, sizeof(double) * (size_t)n, s);  // above every distance
+        // the largest integer: above DBL_MAX, which a point at infinity or NaN keeps
+        if (parts > 1) e = cudaMemsetAsync(p->dist2, 0xff, sizeof(double) * (size_t)n, s);
         if (e == cudaSuccess) {
             k_dist2_all<<<dim3(gp, parts), 256, 0, s>>>(n, p->x, p->y, r->nb, r->bcells,
                                                        reinterpret_cast<unsigned long long*>(p->dist2));

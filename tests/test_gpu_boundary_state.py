@@ -1,0 +1,33 @@
+"""Boundary distances where a raster's or a point's state is out of the
+ordinary: points at infinity or NaN (no cell is nearest: DBL_MAX, on every
+path), and a raster marked again after its mask has changed, with too little
+memory for the new boundary (an error, then the right distances once there is
+memory, never the old cells)."""
+import numpy as np
+import pytest
+
+import oracle_py as o
+
+torch = pytest.importorskip("torch")
+import mgpukde_tiled_b200 as mk  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+# all pairs in one part, all pairs in several, the bins' lists
+@pytest.mark.parametrize("n,side", [(12, 40), (12, 400), (200_000, 400)])
+def test_points_without_a_nearest_cell(n, side):
+    g = o.grid(side, side, 0.0, 0.0, 1.0, -9999.0)
+    m = np.ones((side, side), np.float32)
+    r = np.random.default_rng(n)
+    x, y = r.uniform(0, side, n).astype(np.float32), r.uniform(0, side, n).astype(np.float32)
+    ref = o.dist2_boundary(x, y, g, o.mark_boundary(g, m))
+    bad = [(np.inf, 1.0), (1.0, -np.inf), (np.nan, 2.0), (3.0, np.nan), (np.inf, np.nan)]
+    for i, (px, py) in enumerate(bad):
+        x[2 * i], y[2 * i] = px, py
+        ref[2 * i] = np.finfo(np.float64).max
+    with mk.Context(0) as ctx:
+        pts = mk.Points.upload(ctx, x, y)
+        ras = mk.Raster.upload(ctx, mk.Grid.of(g), m)
+        mk.calc_dist2_boundary(ctx, pts, ras)
+        assert np.array_equal(pts.download(dist2=True, ew=False)[0], ref)
