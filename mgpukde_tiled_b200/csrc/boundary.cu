@@ -551,6 +551,13 @@ static int mask_pass(mgk_ctx* ctx, mgk_raster* r, bool mark) {
     r->runs = nullptr;
     r->nruns = 0;
     r->has_runs = false;
+    if (mark) {  // until the new cells are there the raster is unmarked: a failure leaves no count without cells
+        mgk_free(ctx, r->bcells, sizeof(float2) * (size_t)std::max<int64_t>(r->nb, 1));
+        r->bcells = nullptr;
+        r->nb = 0;
+        r->marked = r->binned = false;
+        r->cand_cap = -1.0;  // the lists are built by the distance search, for its reach
+    }
     if (g.ncols > (int64_t)INT32_MAX - 1) return mgk_fail(ctx, MGK_ERR_INVALID, "raster wider than 2^31 - 2 columns");
     const size_t ncell = (size_t)g.ncols * (size_t)g.nrows;
     int st;
@@ -585,11 +592,6 @@ static int mask_pass(mgk_ctx* ctx, mgk_raster* r, bool mark) {
     const int64_t nb = e == cudaSuccess ? (int64_t)ctx->h_counter[0] : 0;
     const int64_t total = e == cudaSuccess ? (int64_t)ctx->h_counter[1] : 0;
     if (mark && st == MGK_OK) {
-        if (r->bcells) mgk_free(ctx, r->bcells, sizeof(float2) * (size_t)std::max<int64_t>(r->nb, 1));
-        r->bcells = nullptr;
-        r->nb = nb;
-        r->binned = false;
-        r->cand_cap = -1.0;  // the lists are built by the distance search, for its reach
         // bins of kBinCells x kBinCells mask cells over the mask extent
         if (!r->bstart) {
             r->bnx = (int)((g.ncols + kBinCells - 1) / kBinCells);
@@ -597,6 +599,7 @@ static int mask_pass(mgk_ctx* ctx, mgk_raster* r, bool mark) {
             r->nbins = (int64_t)r->bnx * r->bny;
         }
         st = mgk_alloc(ctx, (void**)&r->bcells, sizeof(float2) * (size_t)std::max<int64_t>(nb, 1));
+        if (st == MGK_OK) r->nb = nb;
         if (st == MGK_OK && nb > 0 &&
             (e = cudaMemcpyAsync(r->bcells, cells, sizeof(float2) * (size_t)nb, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
             st = mgk_cuda_fail(ctx, e, "boundary cells");

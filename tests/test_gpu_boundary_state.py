@@ -31,3 +31,38 @@ def test_points_without_a_nearest_cell(n, side):
         ras = mk.Raster.upload(ctx, mk.Grid.of(g), m)
         mk.calc_dist2_boundary(ctx, pts, ras)
         assert np.array_equal(pts.download(dist2=True, ew=False)[0], ref)
+
+
+def test_marked_again_without_memory():
+    side = 300
+    g = o.grid(side, side, 0.0, 0.0, 1.0, -9999.0)
+    r = np.random.default_rng(8)
+    x, y = r.uniform(0, side, 5000).astype(np.float32), r.uniform(0, side, 5000).astype(np.float32)
+    plain = np.ones((side, side), np.float32)  # a ring of 1,196 cells, 10 KB of them
+    holes = np.where(r.random((side, side)) < 0.2, g.nodata, 1.0).astype(np.float32)  # most cells, 500 KB
+    ref = o.dist2_boundary(x, y, g, o.mark_boundary(g, holes))
+    refused = 0
+    for kib in range(512, 4096, 128):
+        mask = torch.from_numpy(plain).cuda()
+        with mk.Context(0, hbm_budget=kib << 10) as ctx:
+            try:
+                pts = mk.Points.upload(ctx, x, y)
+                ras = mk.Raster.wrap(ctx, mk.Grid.of(g), mask)
+                mk.mark_boundary(ctx, ras)
+            except mk.MgkError as e:
+                assert e.status == -3
+                continue
+            mask.copy_(torch.from_numpy(holes))
+            torch.cuda.synchronize()
+            try:
+                mk.mark_boundary(ctx, ras)
+            except mk.MgkError as e:
+                assert e.status == -3
+                refused += 1
+            try:
+                mk.calc_dist2_boundary(ctx, pts, ras)
+            except mk.MgkError as e:
+                assert e.status == -3
+                continue
+            assert np.array_equal(pts.download(dist2=True, ew=False)[0], ref)
+    assert refused >= 1
