@@ -1123,6 +1123,12 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         mgk_points_destroy(p);
         p = q;
     }
+    // The copy stream writes pooled blocks whose former users may still be
+    // queued on the context's stream (the selection reads the arrays of all the
+    // points, released above): its copies start after them.
+    if (st == MGK_OK && ((ce = cudaEventRecord(pipe.counted, c->stream)) != cudaSuccess ||
+                         (ce = cudaStreamWaitEvent(pipe.h2d, pipe.counted, 0)) != cudaSuccess))
+        st = mgk_cuda_fail(c, ce, "kde_raster");
     // The edge mask travels on the copy stream while the index is built from
     // the points (its records take the edge weights once they are known).
     float* d_em = nullptr;
