@@ -1418,13 +1418,18 @@ static int plan_from_counts(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* 
     P.evals = d_evals;
     P.err = ctx->d_counter + 7;
     const int nbx_t = (int)((nc + kBC - 1) / kBC), nby_t = (int)((nr + kBR - 1) / kBR);
-    int st;
+    int st = MGK_OK;
     TilePlan& T = D->T;
+    auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     for (const bool fine : {true, false}) {
         plan_tile(counts, nbx_t, nby_t, ctx->sm_count, ctx->split_waves, 0, fine, T);
         D->b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(T.nslots, 1);
-        st = T.nslots ? mgk_alloc(ctx, (void**)&P.scratch, D->b_scr) : MGK_OK;
-        if (st == MGK_OK) break;
+        if (T.nslots && (st = mgk_alloc(ctx, (void**)&P.scratch, D->b_scr))) continue;
+        // items and split tables (a 16-byte multiple)
+        D->b_tab = up16(sizeof(Item) * T.items.size()) + up16(sizeof(int32_t) * T.split_blocks.size()) +
+                   up16(sizeof(int32_t) * T.split_begin.size());
+        if ((st = mgk_alloc(ctx, &D->d_tab, D->b_tab)) == MGK_OK) break;
+        if (T.nslots) mgk_free(ctx, P.scratch, D->b_scr);
     }
     if (st) {
         delete D;
@@ -1434,7 +1439,6 @@ static int plan_from_counts(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* 
     const int32_t nslots = T.nslots;
     // the work list, the split tables and the error flag in the staging:
     // [items | split blocks | split begins | err]
-    auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t b_items = sizeof(Item) * T.items.size();
     const size_t b_sb = sizeof(int32_t) * T.split_blocks.size(), b_sbeg = sizeof(int32_t) * T.split_begin.size();
     const size_t o_sb = up16(b_items), o_sbeg = o_sb + up16(b_sb), o_err = o_sbeg + up16(b_sbeg);
@@ -1447,12 +1451,6 @@ static int plan_from_counts(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* 
     if (nslots) {
         memcpy(h_st + o_sb, T.split_blocks.data(), b_sb);
         memcpy(h_st + o_sbeg, T.split_begin.data(), b_sbeg);
-    }
-    D->b_tab = o_err;  // items and split tables (a 16-byte multiple)
-    if ((st = mgk_alloc(ctx, &D->d_tab, D->b_tab))) {
-        D->d_tab = nullptr;
-        dplan_release(ctx, D);
-        return st;
     }
     D->src_tab = d_st;
     const char* d_tab = static_cast<const char*>(D->d_tab);
@@ -1623,16 +1621,125 @@ int mgk_launch_density(mgk_ctx* ctx, const mgk_index* idx, const mgk_grid* g, in
     return mgk_density_execute(ctx, D);
 }
 
+// Counted jobs [lo, hi) in one launch.  *launched: whether that was reached;
+// a failure before it (no memory for the split blocks' partials) has done
+// nothing.
+static int run_jobs(mgk_ctx* ctx, int lo, int hi, std::vector<DParams>& Pall, const mgk_tile_job* jobs_all, const int* nbx,
+                    const int* nby, const int* off, const int64_t* counts, bool count, bool* launched) {
+    const int njobs = hi - lo;
+    const mgk_tile_job* jobs = jobs_all + lo;
+    DParams* P = Pall.data() + lo;
+    cudaStream_t s = ctx->stream;
+    // plan each job; items of both bandwidth kinds, merges, slot offsets
+    std::vector<Item> items_fix, items_var;
+    std::vector<int4> merges;
+    int32_t nslots = 0;
+    std::vector<int32_t> slot0(njobs, 0);
+    for (int j = 0; j < njobs; j++) {
+        if (!nbx[lo + j]) continue;
+        TilePlan T;
+        plan_tile(counts + off[lo + j], nbx[lo + j], nby[lo + j], ctx->sm_count, ctx->split_waves, j, true, T);
+        slot0[j] = nslots;
+        for (size_t b = 0; b < T.split_blocks.size(); b++)
+            merges.push_back(make_int4(j, T.split_blocks[b], T.split_begin[b], T.split_begin[b + 1]));
+        nslots += T.nslots;
+        std::vector<Item>& dst = jobs[j].index->varh ? items_var : items_fix;
+        dst.insert(dst.end(), T.items.begin(), T.items.end());
+    }
+    const size_t nitems = items_fix.size() + items_var.size();
+    if (nitems == 0) return MGK_OK;
+    const size_t b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(nslots, 1);
+    double* d_scr = nullptr;
+    int st;
+    if (nslots && (st = mgk_alloc(ctx, (void**)&d_scr, b_scr))) return st;
+    sort_items(items_fix);
+    sort_items(items_var);
+    for (int j = 0; j < njobs; j++)
+        P[j].scratch = d_scr ? d_scr + (size_t)slot0[j] * kCells : nullptr;  // slots are job-local
+    // staging: [job parameters | items (fixed h, then per-point h) | merges | err]
+    auto up16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
+    const size_t o_items = up16(sizeof(DParams) * njobs);
+    const size_t o_mg = o_items + up16(sizeof(Item) * std::max<size_t>(nitems, 1));
+    const size_t o_err = o_mg + up16(sizeof(int4) * std::max<size_t>(merges.size(), 1));
+    // (mapped page-locked staging, as for the counts)
+    char *h_st = nullptr, *d_st = nullptr;
+    if ((st = mgk_host_stage(ctx, o_err + sizeof(unsigned long long), (void**)&h_st, (void**)&d_st))) {
+        mgk_free(ctx, d_scr, b_scr);
+        return st;
+    }
+    memcpy(h_st, P, sizeof(DParams) * njobs);
+    memcpy(h_st + o_items, items_fix.data(), sizeof(Item) * items_fix.size());
+    memcpy(h_st + o_items + sizeof(Item) * items_fix.size(), items_var.data(), sizeof(Item) * items_var.size());
+    if (!merges.empty()) memcpy(h_st + o_mg, merges.data(), sizeof(int4) * merges.size());
+    volatile unsigned long long* h_err = reinterpret_cast<unsigned long long*>(h_st + o_err);
+    *h_err = 0;
+    // the job parameters, items and merges in device memory (stage_tables)
+    mgk_dplan tabs;
+    tabs.b_tab = o_err;
+    tabs.src_tab = d_st;
+    if ((st = mgk_alloc(ctx, &tabs.d_tab, tabs.b_tab))) {
+        mgk_free(ctx, d_scr, b_scr);
+        return st;
+    }
+    const char* d_tab = static_cast<const char*>(tabs.d_tab);
+    const DParams* d_jobs = reinterpret_cast<const DParams*>(d_tab);
+    const Item* d_items = reinterpret_cast<const Item*>(d_tab + o_items);
+    const int4* d_mg = reinterpret_cast<const int4*>(d_tab + o_mg);
+    cudaError_t ce = cudaSuccess;
+    *launched = true;
+    do {
+        if ((st = stage_tables(ctx, &tabs, s))) break;
+        cudaEventRecord(ctx->ev_a, s);
+        if (!items_fix.empty()) {
+            if (count) launch_density_jobs<false, true>((unsigned)items_fix.size(), s, d_jobs, d_items);
+            else launch_density_jobs<false, false>((unsigned)items_fix.size(), s, d_jobs, d_items);
+            MGK_COUNT_LAUNCH(ctx, 1);
+        }
+        if (!items_var.empty()) {
+            const Item* iv = d_items + items_fix.size();
+            if (count) launch_density_jobs<true, true>((unsigned)items_var.size(), s, d_jobs, iv);
+            else launch_density_jobs<true, false>((unsigned)items_var.size(), s, d_jobs, iv);
+            MGK_COUNT_LAUNCH(ctx, 1);
+        }
+        cudaEventRecord(ctx->ev_b, s);
+        if ((ce = cudaGetLastError()) != cudaSuccess) break;
+        if (!merges.empty()) {
+            k_merge_jobs<<<dim3((unsigned)merges.size(), kMergeParts), 256, 0, s>>>(d_jobs, d_mg);
+            if ((ce = cudaGetLastError()) != cudaSuccess) break;
+            MGK_COUNT_LAUNCH(ctx, 1);
+        }
+        k_store_flag<<<1, 1, 0, s>>>(ctx->d_counter + 7, reinterpret_cast<unsigned long long*>(d_st + o_err));
+        if ((ce = cudaGetLastError()) != cudaSuccess) break;
+        MGK_COUNT_LAUNCH(ctx, 1);
+        // the staging and the scratch are released below: wait for the kernels
+        ce = cudaStreamSynchronize(s);
+        float ms = 0.0f;
+        if (ce == cudaSuccess && cudaEventElapsedTime(&ms, ctx->ev_a, ctx->ev_b) == cudaSuccess)
+            ctx->last_density_ms += ms;
+    } while (0);
+    if (ce != cudaSuccess) st = mgk_cuda_fail(ctx, ce, "density jobs");
+    else if (st == MGK_OK && *h_err) st = mgk_fail(ctx, MGK_ERR_TIMEOUT, "density: a shared-memory staging wait timed out");
+    if (st != MGK_OK && ce == cudaSuccess) (void)cudaStreamSynchronize(s);  // nothing in flight reads the tables
+    mgk_free(ctx, d_scr, b_scr);
+    mgk_free(ctx, tabs.d_tab, tabs.b_tab);
+    tabs.d_tab = nullptr;
+    return st;
+}
+
 // Several tiles in one density launch (plus one merge launch): the tiles
 // are planned independently (their items and split slots are exactly those
 // of mgk_launch_density), their items concatenated and ordered heaviest
 // first, and each item finds its tile's parameters through its job index.
 // Jobs with per-point bandwidths and jobs with a fixed one go to two
-// launches.  evals (optional, device) receives per-job counters.
+// launches.  evals (optional, device) receives per-job counters.  Without the
+// memory for all tiles' split blocks at once the batch goes in halves, down to
+// the single-tile launch (coarsely split where that is), so that a tile's
+// result never depends on the others.
 int mgk_launch_density_jobs(mgk_ctx* ctx, int njobs, const mgk_tile_job* jobs, unsigned long long* d_evals) {
     if (njobs <= 0) return MGK_OK;
     cudaStream_t s = ctx->stream;
     std::vector<DParams> P(njobs);
+    ctx->last_density_ms = 0.0f;
     std::vector<int> nbx(njobs), nby(njobs), off(njobs + 1, 0);
     for (int j = 0; j < njobs; j++) {
         const mgk_tile_job& J = jobs[j];
@@ -1668,103 +1775,30 @@ int mgk_launch_density_jobs(mgk_ctx* ctx, int njobs, const mgk_tile_job* jobs, u
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
     if (ce != cudaSuccess) return mgk_cuda_fail(ctx, ce, "density jobs plan");
-    // plan each job; items of both bandwidth kinds, merges, slot offsets
-    std::vector<Item> items_fix, items_var;
-    std::vector<int4> merges;
-    int32_t nslots = 0;
-    std::vector<int32_t> slot0(njobs, 0);
-    size_t b_scr = 0;
-    double* d_scr = nullptr;
     const std::vector<int64_t> counts(reinterpret_cast<const int64_t*>(h_st),
                                       reinterpret_cast<const int64_t*>(h_st) + nblk_all);
-    for (const bool fine : {true, false}) {
-        items_fix.clear();
-        items_var.clear();
-        merges.clear();
-        nslots = 0;
-        for (int j = 0; j < njobs; j++) {
-            if (!nbx[j]) continue;
-            TilePlan T;
-            plan_tile(counts.data() + off[j], nbx[j], nby[j], ctx->sm_count, ctx->split_waves, j, fine, T);
-            slot0[j] = nslots;
-            for (size_t b = 0; b < T.split_blocks.size(); b++)
-                merges.push_back(make_int4(j, T.split_blocks[b], T.split_begin[b], T.split_begin[b + 1]));
-            nslots += T.nslots;
-            std::vector<Item>& dst = jobs[j].index->varh ? items_var : items_fix;
-            dst.insert(dst.end(), T.items.begin(), T.items.end());
+    std::vector<std::pair<int, int>> todo{{0, njobs}};  // ranges of jobs, the next one last
+    while (!todo.empty()) {
+        const int lo = todo.back().first, hi = todo.back().second;
+        todo.pop_back();
+        bool launched = false;
+        st = run_jobs(ctx, lo, hi, P, jobs, nbx.data(), nby.data(), off.data(), counts.data(), d_evals != nullptr,
+                      &launched);
+        if (st == MGK_ERR_BUDGET && !launched) {
+            if (hi - lo > 1) {
+                todo.push_back({(lo + hi) / 2, hi});
+                todo.push_back({lo, (lo + hi) / 2});
+                continue;
+            }
+            const mgk_tile_job& J = jobs[lo];
+            const float ms = ctx->last_density_ms;
+            st = mgk_launch_density(ctx, J.index, &J.grid, J.row0, J.col0, J.nrows, J.ncols, J.d_mask, J.d_out,
+                                    P[lo].evals, false);
+            ctx->last_density_ms += ms;
         }
-        b_scr = sizeof(double) * (size_t)kCells * (size_t)std::max(nslots, 1);
-        st = nslots ? mgk_alloc(ctx, (void**)&d_scr, b_scr) : MGK_OK;
-        if (st == MGK_OK) break;
+        if (st) return st;
     }
-    if (st) return st;
-    sort_items(items_fix);
-    sort_items(items_var);
-    for (int j = 0; j < njobs; j++)
-        P[j].scratch = d_scr ? d_scr + (size_t)slot0[j] * kCells : nullptr;  // slots are job-local
-    // staging: [job parameters | items (fixed h, then per-point h) | merges | err]
-    auto up16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
-    const size_t nitems = items_fix.size() + items_var.size();
-    const size_t o_items = up16(sizeof(DParams) * njobs);
-    const size_t o_mg = o_items + up16(sizeof(Item) * std::max<size_t>(nitems, 1));
-    const size_t o_err = o_mg + up16(sizeof(int4) * std::max<size_t>(merges.size(), 1));
-    if ((st = mgk_host_stage(ctx, o_err + sizeof(unsigned long long), (void**)&h_st, (void**)&d_st))) {
-        mgk_free(ctx, d_scr, b_scr);
-        return st;
-    }
-    memcpy(h_st, P.data(), sizeof(DParams) * njobs);
-    memcpy(h_st + o_items, items_fix.data(), sizeof(Item) * items_fix.size());
-    memcpy(h_st + o_items + sizeof(Item) * items_fix.size(), items_var.data(), sizeof(Item) * items_var.size());
-    if (!merges.empty()) memcpy(h_st + o_mg, merges.data(), sizeof(int4) * merges.size());
-    volatile unsigned long long* h_err = reinterpret_cast<unsigned long long*>(h_st + o_err);
-    *h_err = 0;
-    // the job parameters, items and merges in device memory (stage_tables)
-    mgk_dplan tabs;
-    tabs.b_tab = o_err;
-    tabs.src_tab = d_st;
-    if ((st = mgk_alloc(ctx, &tabs.d_tab, tabs.b_tab))) {
-        mgk_free(ctx, d_scr, b_scr);
-        return st;
-    }
-    const char* d_tab = static_cast<const char*>(tabs.d_tab);
-    const DParams* d_jobs = reinterpret_cast<const DParams*>(d_tab);
-    const Item* d_items = reinterpret_cast<const Item*>(d_tab + o_items);
-    const int4* d_mg = reinterpret_cast<const int4*>(d_tab + o_mg);
-    do {
-        if ((st = stage_tables(ctx, &tabs, s))) break;
-        cudaEventRecord(ctx->ev_a, s);
-        if (!items_fix.empty()) {
-            if (d_evals) launch_density_jobs<false, true>((unsigned)items_fix.size(), s, d_jobs, d_items);
-            else launch_density_jobs<false, false>((unsigned)items_fix.size(), s, d_jobs, d_items);
-            MGK_COUNT_LAUNCH(ctx, 1);
-        }
-        if (!items_var.empty()) {
-            const Item* iv = d_items + items_fix.size();
-            if (d_evals) launch_density_jobs<true, true>((unsigned)items_var.size(), s, d_jobs, iv);
-            else launch_density_jobs<true, false>((unsigned)items_var.size(), s, d_jobs, iv);
-            MGK_COUNT_LAUNCH(ctx, 1);
-        }
-        cudaEventRecord(ctx->ev_b, s);
-        if ((ce = cudaGetLastError()) != cudaSuccess) break;
-        if (!merges.empty()) {
-            k_merge_jobs<<<dim3((unsigned)merges.size(), kMergeParts), 256, 0, s>>>(d_jobs, d_mg);
-            if ((ce = cudaGetLastError()) != cudaSuccess) break;
-            MGK_COUNT_LAUNCH(ctx, 1);
-        }
-        k_store_flag<<<1, 1, 0, s>>>(ctx->d_counter + 7, reinterpret_cast<unsigned long long*>(d_st + o_err));
-        if ((ce = cudaGetLastError()) != cudaSuccess) break;
-        MGK_COUNT_LAUNCH(ctx, 1);
-        // the staging and the scratch are released below: wait for the kernels
-        ce = cudaStreamSynchronize(s);
-        if (ce == cudaSuccess) cudaEventElapsedTime(&ctx->last_density_ms, ctx->ev_a, ctx->ev_b);
-    } while (0);
-    if (ce != cudaSuccess) st = mgk_cuda_fail(ctx, ce, "density jobs");
-    else if (st == MGK_OK && *h_err) st = mgk_fail(ctx, MGK_ERR_TIMEOUT, "density: a shared-memory staging wait timed out");
-    if (st != MGK_OK && ce == cudaSuccess) (void)cudaStreamSynchronize(s);  // nothing in flight reads the tables
-    mgk_free(ctx, d_scr, b_scr);
-    mgk_free(ctx, tabs.d_tab, tabs.b_tab);
-    tabs.d_tab = nullptr;
-    return st;
+    return MGK_OK;
 }
 
 // ---------------------------------------------------------------------------
