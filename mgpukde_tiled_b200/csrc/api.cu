@@ -1192,7 +1192,18 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         const int b = (int)(k & 1), db = (int)(k % kDepth);
         mgk_density_discard(c, plans[b]);  // tile k - 2's
         plans[b] = nullptr;
-        return mgk_density_plan_counted(c, idx, dg, r0, c0, nr, nc, d_mask[db], d_out[db], d_ev, 1 + b, &plans[b]);
+        auto plan = [&] {
+            return mgk_density_plan_counted(c, idx, dg, r0, c0, nr, nc, d_mask[db], d_out[db], d_ev, 1 + b, &plans[b]);
+        };
+        int s1 = plan();
+        if (s1 == MGK_ERR_BUDGET && plans[b ^ 1]) {  // tile k - 1 may hold the memory: after it, then
+            const cudaError_t e = cudaStreamSynchronize(c->stream);
+            if (e != cudaSuccess) return mgk_cuda_fail(c, e, "kde_raster plan");
+            mgk_density_discard(c, plans[b ^ 1]);
+            plans[b ^ 1] = nullptr;
+            s1 = plan();
+        }
+        return s1;
     };
     auto count_of = [&](int64_t k) -> int {
         int64_t r0, c0, nr, nc;
@@ -1250,10 +1261,26 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
                 st = mgk_fail(c, MGK_ERR_INVALID, "kde_raster: band layout");
                 break;
             }
-            if ((st = mgk_density_plan_from_counts(c, idx, dg, r0, 0, nr, dg->ncols, counts + (r0 - row_lo) / 64 * nbx,
-                                                   packed ? nullptr : d_mask[db], d_out[db], d_ev, 1 + (int)(k & 1),
-                                                   &band_plans[k])))
-                break;
+            auto plan = [&] {
+                return mgk_density_plan_from_counts(c, idx, dg, r0, 0, nr, dg->ncols, counts + (r0 - row_lo) / 64 * nbx,
+                                                    packed ? nullptr : d_mask[db], d_out[db], d_ev, 1 + (int)(k & 1),
+                                                    &band_plans[k]);
+            };
+            st = plan();
+            if (st == MGK_ERR_BUDGET && k > 0) {  // the bands before it may hold the memory: after them, then
+                for (const cudaStream_t q : {c->stream, pipe.alt, pipe.mrg})
+                    if ((ce = cudaStreamSynchronize(q)) != cudaSuccess) break;
+                if (ce != cudaSuccess) {
+                    st = mgk_cuda_fail(c, ce, "kde_raster plan");
+                    break;
+                }
+                for (int64_t j = 0; j < k; j++) {
+                    mgk_density_discard(c, band_plans[j]);
+                    band_plans[j] = nullptr;
+                }
+                st = plan();
+            }
+            if (st) break;
             if (packed)
                 mgk_density_set_mask_bits(band_plans[k], reinterpret_cast<const unsigned char*>(d_mask[db]), mstride);
             if (two) mgk_density_set_tail_flag(band_plans[k], d_flag + k);

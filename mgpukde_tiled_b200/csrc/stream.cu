@@ -171,8 +171,18 @@ extern "C" int mgk_density_stream(mgk_ctx* c, const mgk_index* idx, const mgk_gr
         const int b = (int)(k & 1);
         mgk_density_discard(c, plans[b]);  // tile k - 2's, whose kernels have ended
         plans[b] = nullptr;
-        return mgk_density_plan_counted(c, idx, g, r0, c0, nr, nc, mask_src ? d_mask : nullptr, d_out[k % kOutBufs], d_ev,
-                                        1 + b, &plans[b]);
+        auto plan = [&] {
+            return mgk_density_plan_counted(c, idx, g, r0, c0, nr, nc, mask_src ? d_mask : nullptr, d_out[k % kOutBufs],
+                                            d_ev, 1 + b, &plans[b]);
+        };
+        int s1 = plan();
+        if (s1 == MGK_ERR_BUDGET && plans[b ^ 1]) {  // tile k - 1 may hold the memory: after it, then
+            if (cudaStreamSynchronize(c->stream) != cudaSuccess) return mgk_fail(c, MGK_ERR_CUDA, "density_stream: plan");
+            mgk_density_discard(c, plans[b ^ 1]);
+            plans[b ^ 1] = nullptr;
+            s1 = plan();
+        }
+        return s1;
     };
     if (st == MGK_OK && !todo.empty() && (st = count_of(0)) == MGK_OK) {
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) st = mgk_fail(c, MGK_ERR_CUDA, "density_stream: plan");
