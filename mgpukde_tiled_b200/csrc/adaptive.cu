@@ -429,7 +429,8 @@ int count_end(mgk_ctx* c) {
 
 // The points in the order in which they are queried, once per search (they do
 // not move), and the places of their records in the index at hand; null
-// for few points, or without the memory for both: the order of the records.
+// for few points, or without the memory for both: the order of the records.  A
+// later step that lacks memory gets theirs (needing).
 struct QueryOrder {
     mgk_ctx* c = nullptr;
     int64_t n = 0;
@@ -449,10 +450,18 @@ struct QueryOrder {
         order = inv = nullptr;
     }
     ~QueryOrder() { release(); }
+    // step(), again without the order if it lacked memory (it has launched nothing then)
+    template <typename Step>
+    int needing(const Step& step) {
+        const int st = step();
+        if (st != MGK_ERR_BUDGET || !order) return st;
+        release();
+        return step();
+    }
 };
 
 // den[input order] and logsum[0] = sum_j log(max(den_j, floor_v)).
-int point_density(mgk_ctx* c, const mgk_index* idx, const QueryOrder& qo, bool self, double* d_den, double floor_v,
+int point_density(mgk_ctx* c, const mgk_index* idx, QueryOrder& qo, bool self, double* d_den, double floor_v,
                   double* d_logsum) {
     cudaStream_t s = c->stream;
     const int64_t g = (idx->n + kPdQ - 1) / kPdQ;
@@ -461,24 +470,31 @@ int point_density(mgk_ctx* c, const mgk_index* idx, const QueryOrder& qo, bool s
         return MGK_OK;
     }
     // bin rows split over enough warps to keep every SM busy to the end
-    const int nsplit = (int)std::min<int64_t>(24, std::max<int64_t>(1, (kPdWarps * (int64_t)c->sm_count + g - 1) / g));
+    int nsplit = (int)std::min<int64_t>(24, std::max<int64_t>(1, (kPdWarps * (int64_t)c->sm_count + g - 1) / g));
     const int64_t gc = (idx->n + kPdC - 1) / kPdC;
     const int64_t nbins = idx->varh ? idx->nbx * idx->nby : 0;
     const size_t b_part = sizeof(double) * (size_t)gc, b_r2 = sizeof(float) * (size_t)std::max<int64_t>(nbins, 1);
-    const size_t b_psum = sizeof(double) * (size_t)idx->n * (size_t)nsplit;
+    size_t b_psum = 0;
     double *part = nullptr, *psum = nullptr;
     float* r2 = nullptr;
-    int st = mgk_alloc(c, (void**)&part, b_part);
+    auto scratch = [&] {
+        part = psum = nullptr;
+        b_psum = sizeof(double) * (size_t)idx->n * (size_t)nsplit;
+        int st = mgk_alloc(c, (void**)&part, b_part);
+        if (st == MGK_OK) st = mgk_alloc(c, (void**)&psum, b_psum);
+        if (st == MGK_OK && idx->varh) st = mgk_alloc(c, (void**)&r2, b_r2);
+        if (st) {
+            mgk_free(c, part, b_part);
+            mgk_free(c, psum, b_psum);
+        }
+        return st;
+    };
+    int st = qo.needing(scratch);
+    while (st == MGK_ERR_BUDGET && nsplit > 1) {  // fewer warps a group then
+        nsplit /= 2;
+        st = scratch();
+    }
     if (st) return st;
-    if ((st = mgk_alloc(c, (void**)&psum, b_psum))) {
-        mgk_free(c, part, b_part);
-        return st;
-    }
-    if (idx->varh && (st = mgk_alloc(c, (void**)&r2, b_r2))) {
-        mgk_free(c, part, b_part);
-        mgk_free(c, psum, b_psum);
-        return st;
-    }
     const dim3 grid((unsigned)g, (unsigned)nsplit);
     if (idx->varh) {
         k_fill_f32<<<(unsigned)((nbins + 255) / 256), 256, 0, s>>>(nbins, -1.0f, r2);
@@ -551,16 +567,22 @@ int pilot_density(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, Pilot
     for (int i = 0; i < PilotCache::kEntries; i++)  // a free entry, else the least recently used
         if (slot < 0 || !pc.buf[i] || (pc.buf[slot] && pc.last[i] < pc.last[slot])) slot = i;
     int st;
-    if (!pc.buf[slot] && (st = mgk_alloc(c, (void**)&pc.buf[slot], pc.bytes()))) return st;
+    if (!pc.buf[slot] && (st = pc.qo.needing([&] { return mgk_alloc(c, (void**)&pc.buf[slot], pc.bytes()); }))) return st;
     pc.hbits[slot] = hb;
     pc.last[slot] = ++pc.tick;
     double* den = pc.buf[slot];
-    if (r) st = mgk_launch_edge_weights(c, p->n, p->x, p->y, nullptr, h, p->dist2, r, p->ew, edge_count(c));
+    if (r)
+        st = pc.qo.needing([&] {
+            return mgk_launch_edge_weights(c, p->n, p->x, p->y, nullptr, h, p->dist2, r, p->ew, edge_count(c));
+        });
     else st = mgk_edge_weights_unit(c, p);
     if (st == MGK_OK) {
         p->has_ew = true;
         mgk_index* idx = nullptr;
-        if ((st = mgk_index_build_async(c, p, h, 0.0f, &pc.extent, &idx, pc.qo.inv)) == MGK_OK) {  // h > 0: fixed-h index
+        st = pc.qo.needing([&] {  // h > 0: fixed-h index
+            return mgk_index_build_async(c, p, h, 0.0f, &pc.extent, &idx, pc.qo.inv);
+        });
+        if (st == MGK_OK) {
             st = point_density(c, idx, pc.qo, true, den, 0.0, den + std::max<int64_t>(p->n, 1));
             mgk_index_destroy(idx);
         }
@@ -597,7 +619,9 @@ int loglik_adaptive(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, flo
     if (st) return st;
     if (!pc.have_h) MGK_CHECK_CUDA(c, cudaEventCreateWithFlags(&pc.have_h, cudaEventDisableTiming));
     MGK_CHECK_CUDA(c, cudaEventRecord(pc.have_h, c->stream));
-    if (r && (st = mgk_launch_edge_weights(c, p->n, p->x, p->y, p->h, 0.0f, p->dist2, r, p->ew, edge_count(c))))
+    if (r && (st = pc.qo.needing([&] {
+            return mgk_launch_edge_weights(c, p->n, p->x, p->y, p->h, 0.0f, p->dist2, r, p->ew, edge_count(c));
+        })))
         return st;
     // per-point h; bins of 0.75 h (the geometric mean of hs is h), not of the
     // widest h, so that the per-bin reach can cut the window down
@@ -613,7 +637,8 @@ int loglik_adaptive(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, flo
         extent.hmax = mgk_ord2f(m);
     }
     mgk_index* idx = nullptr;
-    if ((st = mgk_index_build_async(c, p, 0.0f, 0.75f * h, &extent, &idx, pc.qo.inv))) return st;
+    if ((st = pc.qo.needing([&] { return mgk_index_build_async(c, p, 0.0f, 0.75f * h, &extent, &idx, pc.qo.inv); })))
+        return st;
     double *sum = reinterpret_cast<double*>(c->h_map + 32), *d_sum = reinterpret_cast<double*>(c->d_map + 32);
     st = point_density(c, idx, pc.qo, false, d_den, (double)MGK_EPS_DENSITY_F, d_sum);
     mgk_index_destroy(idx);
