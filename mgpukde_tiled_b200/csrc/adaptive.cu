@@ -59,9 +59,6 @@ constexpr int64_t kPdCurve = 1 << 13;
 constexpr float kPdCut = (float)(0.5 * MGK_CUT * MGK_LOG2E);
 constexpr float kPdBand = 4e-6f * kPdCut;
 
-// i, or a place in range where a failed sort left i unwritten (the failure is reported by the host).
-__device__ __forceinline__ int64_t mgk_below(int32_t i, int64_t n) { return (uint32_t)i < (uint64_t)n ? i : 0; }
-
 // psum[y][q] = sum over candidates i (the points of the index within reach
 // of the CTA's 32 queries, in the bin rows y, y + nsplit, ... of
 // the window, y = blockIdx.y) of [in cutoff] K w_i e_i, unnormalised; the
@@ -109,7 +106,7 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
     const bool qv = slot < n;
     float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     int64_t qpos = slot;
-    if (qv && order) qpos = mgk_below(inv[mgk_below(order[slot], n)], n);
+    if (qv && order) qpos = inv[order[slot]];
     if (qv) q = *reinterpret_cast<const float4*>(pts + qpos);
     const float qx = q.x + q.z, qy = q.y + q.w;
     float mnx = qv ? qx : FLT_MAX, mxx = qv ? qx : -FLT_MAX, mny = qv ? qy : FLT_MAX, mxy = qv ? qy : -FLT_MAX;
@@ -328,7 +325,7 @@ __global__ void __launch_bounds__(kPdC) k_pd_combine(int64_t n, int nsplit, cons
         double v = 0.0;
         for (int y = 0; y < nsplit; y++) v += psum[(int64_t)y * n + q];
         if (!varh) v /= h2 * (double)MGK_TWO_PI_F;
-        den[mgk_below(order[q], n)] = v;
+        den[order[q]] = v;
         lg = log(v > floor_v ? v : floor_v);
     }
     for (int o = 16; o; o >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
@@ -420,7 +417,6 @@ int count_end(mgk_ctx* c) {
     MGK_CHECK_CUDA(c, cudaMemcpyAsync(c->h_counter + 5, c->d_counter + 5, 2 * sizeof(unsigned long long),
                                       cudaMemcpyDeviceToHost, c->stream));
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (const int st = mgk_sort_check(c)) return st;
     c->last_loo_evals[0] = (int64_t)c->h_counter[5];
     c->last_loo_evals[1] = (int64_t)c->h_counter[6];
     MGK_CHECK_CUDA(c, cudaEventElapsedTime(&c->last_loo_ms, c->ev_a, c->ev_b));

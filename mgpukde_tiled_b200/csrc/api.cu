@@ -609,14 +609,13 @@ int mgk_edge_weights_unit(mgk_ctx* c, mgk_points* p) {
 // ------------------------------------------------------------------ index --
 int mgk_index_build(mgk_ctx* c, const mgk_points* p, float h, float bin_size, mgk_index** out) {
     mgk_index* idx = nullptr;
-    int st = mgk_index_build_async(c, p, h, bin_size, nullptr, &idx);
+    const int st = mgk_index_build_async(c, p, h, bin_size, nullptr, &idx);
     if (st) return st;
     // the index is complete on return: the points may go, and other streams may read it
     const cudaError_t e = cudaStreamSynchronize(c->stream);
-    st = e != cudaSuccess ? mgk_cuda_fail(c, e, "index build") : mgk_sort_check(c);
-    if (st) {
+    if (e != cudaSuccess) {
         mgk_index_destroy(idx);
-        return st;
+        return mgk_cuda_fail(c, e, "index build");
     }
     *out = idx;
     return MGK_OK;
@@ -1371,7 +1370,7 @@ static int kde_raster_rows(mgk_ctx* c, int64_t n, const float* x, const float* y
         ce = cudaMemcpy(c->h_counter + 4, c->d_counter + 4, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
         if (ce != cudaSuccess) st = mgk_cuda_fail(c, ce, "kde_raster counters");
         else if (c->h_counter[7]) st = mgk_fail(c, MGK_ERR_TIMEOUT, "density: a shared-memory staging wait timed out");
-        else if ((st = mgk_sort_check(c)) == MGK_OK) ev_den = (int64_t)c->h_counter[4];
+        else ev_den = (int64_t)c->h_counter[4];
     }
     for (int i = 0; i < kDepth; i++) {
         if (d_out[i]) mgk_free(c, d_out[i], tb);

@@ -26,7 +26,11 @@ constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kMaxDigits = 512;   // digits of up to 9 bits: 18-bit bin ids sort in two passes
 constexpr int kMaxPasses = 4;     // 32-bit keys
-constexpr long long kSortSpin = 1ll << 24;
+// Looks at an earlier tile's state word before a digit is counted in its items instead.
+#ifndef MGK_SORT_SPIN
+#define MGK_SORT_SPIN (1ll << 24)
+#endif
+constexpr long long kSortSpin = MGK_SORT_SPIN;
 // Bins up to which the gather fills the bin starts on its way instead of a
 // kernel of searches (9 to 12 us of chained loads whatever the size).  A gap
 // between two points can be all bins, which one warp then fills: 2^16 take it
@@ -62,7 +66,7 @@ struct StartJob {
     int32_t* start;
 };
 struct GatherJob {
-    int32_t* perm;
+    const int32_t* perm;
     MgkPt* out;
     int qexp;
     const unsigned* keys;  // the sorted keys, where the gather fills the bin starts, else null
@@ -162,13 +166,22 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(unsigned* __restrict__ 
     }
 }
 
+// Of the first n keys, those with digit d.
+__device__ __noinline__ unsigned count_digit(const unsigned* __restrict__ keys, int64_t n, int shift, unsigned mask,
+                                             unsigned d) {
+    unsigned c = 0;
+    for (int64_t i = 0; i < n; i++) c += ((keys[i] >> shift) & mask) == d ? 1u : 0u;
+    return c;
+}
+
 // One digit of the stable sort in one kernel.  Tiles of 256 IPT items are
 // handed out in order by a counter; a tile ranks its items in registers (each
 // warp its own run of 32 IPT, match_any per round), publishes its digit
 // counts, and adds up those of the tiles before it, which are all running or
 // done, from their published counts or sums (state in the top two bits of a
-// word: 1 counts, 2 sums including all earlier tiles).  A pass reads and
-// writes each item once; the earlier form (a histogram kernel, a scan of all
+// word: 1 counts, 2 sums including all earlier tiles).  The wait for a word is
+// bounded: after it the tile counts the earlier items itself, slowly, so the
+// sort always ends and always sorts.  A pass reads and writes each item once; the earlier form (a histogram kernel, a scan of all
 // tiles' counts in one CTA, a scatter in rounds of 256 items with five
 // barriers each, tiles of 8,192) took 85 us a pass on 10^6 points and 29 us on
 // 2,000, where one CTA did everything; this takes 36 and 6 us (an index build
@@ -176,8 +189,7 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(unsigned* __restrict__ 
 // items' indexes.
 template <int IPT, typename W, int N>
 __global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, int db, size_t look_bytes,
-                                                             const __grid_constant__ Jobs<SortJob, N> J,
-                                                             unsigned* err) {
+                                                             const __grid_constant__ Jobs<SortJob, N> J) {
     const SortJob& B = J.j[N > 1 ? blockIdx.y : 0];
     const unsigned* __restrict__ keys_in = p & 1 ? B.kb : B.ka;
     const int32_t* __restrict__ vals_in = p == 0 ? nullptr : p & 1 ? B.vb : B.va;
@@ -240,13 +252,16 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, i
         }
         lk[(size_t)tile * nd + d] = ((W)(tile ? 1 : 2) << kTop) | run;
         unsigned prev = 0;
-        for (unsigned p = tile; p > 0;) {
-            p--;
+        for (unsigned q = tile; q > 0;) {
+            q--;
             W v = 0;
             long long spin = 0;
-            while ((v = lk[(size_t)p * nd + d]) >> kTop == 0 && ++spin < kSortSpin) {
+            while ((v = lk[(size_t)q * nd + d]) >> kTop == 0 && ++spin < kSortSpin) {
             }
-            if (v >> kTop == 0) *err = 1u;  // ran out: reported by the host, the places stay in range
+            if (v >> kTop == 0) {
+                prev += count_digit(keys_in, (int64_t)(q + 1) * (kSortThreads * IPT), shift, (unsigned)nd - 1u, (unsigned)d);
+                break;
+            }
             prev += (unsigned)(v & kVal);
             if (v >> kTop != 1) break;
         }
@@ -294,17 +309,17 @@ SortPlan sort_plan(int64_t n, int bits) {
 // scratch; the sorted keys and values end in kb, vb after an odd number of
 // passes, else in ka, va.
 template <int N>
-void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, int nj, const Jobs<SortJob, N>& J, unsigned* err) {
+void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, int nj, const Jobs<SortJob, N>& J) {
     const dim3 g((unsigned)P.ntiles, (unsigned)nj);
     for (int p = 0; p < P.passes; p++) {
         if (P.wide)
-            k_radix_pass<16, unsigned long long, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
+            k_radix_pass<16, unsigned long long, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
         else if (P.ipt == 16)
-            k_radix_pass<16, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
+            k_radix_pass<16, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
         else if (P.ipt == 4)
-            k_radix_pass<4, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
+            k_radix_pass<4, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
         else
-            k_radix_pass<1, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J, err);
+            k_radix_pass<1, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
     }
 }
 
@@ -351,7 +366,7 @@ __device__ __forceinline__ void fill_starts(int64_t n, int64_t i, const unsigned
     unsigned lo = 0, hi = 0;  // start[lo, hi) = i
     if (i <= n) {
         if (i > 0) lo = keys[i - 1] + 1;
-        hi = (i < n ? min(keys[i], nbins - 1) : nbins) + 1;  // in range also after a sort that failed
+        hi = (i < n ? keys[i] : nbins) + 1;
     }
     const bool wide = hi > lo + 4;
     if (!wide)
@@ -388,14 +403,13 @@ __global__ void k_gather(int64_t n, const float* __restrict__ x, const float* __
                          const float* __restrict__ w, const float* __restrict__ ew, const float* __restrict__ hpp,
                          const __grid_constant__ Jobs<GatherJob, N> J) {
     const GatherJob& B = J.j[N > 1 ? blockIdx.y : 0];
-    int32_t* __restrict__ perm = B.perm;
+    const int32_t* __restrict__ perm = B.perm;
     MgkPt* __restrict__ out = B.out;
     const int qexp = B.qexp;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (B.keys) fill_starts(n, i, B.keys, B.nbins, B.start);
     if (i >= n) return;
-    int32_t j = perm[i];
-    if ((unsigned)j >= (unsigned)n) perm[i] = j = 0;  // a place that a failed sort left unwritten
+    const int32_t j = perm[i];
     if (B.inv) B.inv[j] = (int32_t)i;
     MgkPt r;
     mgk_qsplit(x[j], qexp, r.xh, r.xl);
@@ -645,7 +659,7 @@ static cudaError_t enqueue_build(mgk_ctx* ctx, const mgk_points* pts, bool varh,
     const unsigned ny = (unsigned)nj;
     k_bin_keys<N><<<dim3(key_grid(ctx, n), ny), 256, 0, s>>>(n, pts->x, pts->y, idx[0]->ox, idx[0]->oy, P.db, P.passes,
                                                              K);
-    sort_passes<N>(s, P, n, nj, S, ctx->d_map);
+    sort_passes<N>(s, P, n, nj, S);
     if (search && nbins < (1 << 20))
         k_bin_starts<1, N><<<dim3((unsigned)(nbins / 256 + 1), ny), 256, 0, s>>>(n, T);
     else if (search)
@@ -674,7 +688,7 @@ static cudaError_t enqueue_zorder(mgk_ctx* ctx, int nj, mgk_index* const* idx, i
     }
     k_morton_keys<N><<<dim3(key_grid(ctx, n), (unsigned)nj), 256, 0, ctx->stream>>>(n, idx[0]->ox, idx[0]->oy, P.db,
                                                                                     P.passes, K);
-    sort_passes<N>(ctx->stream, P, n, nj, S, ctx->d_map);
+    sort_passes<N>(ctx->stream, P, n, nj, S);
     MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
     return cudaGetLastError();
 }
@@ -715,7 +729,7 @@ int mgk_points_curve_order(mgk_ctx* ctx, const mgk_points* pts, const mgk_extent
         k_hilbert_keys<<<key_grid(ctx, n), 256, 0, ctx->stream>>>(n, pts->x, pts->y, extent.xmin, extent.ymin,
                                                                   ext > 0.0 ? 65536.0 / ext : 0.0, P.db, P.passes, b.k0,
                                                                   b.scr);
-        sort_passes<1>(ctx->stream, P, n, 1, S, ctx->d_map);
+        sort_passes<1>(ctx->stream, P, n, 1, S);
         MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
         return cudaGetLastError();
     });
@@ -754,14 +768,6 @@ int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_exte
     out->ymax = mgk_ord2f(v[3]);
     if (want_h) out->hmax = mgk_ord2f(v[4]);
     return MGK_OK;
-}
-
-// Fails when a sort kernel's bounded wait ran out (after a wait for the stream).
-int mgk_sort_check(mgk_ctx* ctx) {
-    volatile unsigned* f = ctx->h_map;
-    if (!*f) return MGK_OK;
-    *f = 0;
-    return mgk_fail(ctx, MGK_ERR_TIMEOUT, "index sort: a wait for an earlier tile timed out");
 }
 
 // An index's numbers and its arrays, without the kernels that fill them.

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
         for (int i = 0; i < kLooSub; i++) {
             const int64_t qk = q0 + 32 * i + lane;
             if (qk >= P.n) continue;
-            const int qp = (int)min((unsigned)L.qord[qk], (unsigned)(P.n - 1));  // in range also after a sort that failed
+            const int qp = L.qord[qk];
             const float4 v = *reinterpret_cast<const float4*>(pts + qp);
             const float vx = v.x + v.z, vy = v.y + v.w;
             gmnx = fminf(gmnx, vx);
@@ -772,7 +772,6 @@ int mgk_loo_batch_run(mgk_loo_batch* B, const float* hs, double* logl, int* best
     }
     MGK_CHECK_CUDA(c, cudaEventRecord(c->ev_b, s));
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(s));
-    if (const int st = mgk_sort_check(c)) return st;
     memcpy(logl, B->h_io + B->o_logl, sizeof(double) * (size_t)B->nh);
     const unsigned long long* tail = reinterpret_cast<const unsigned long long*>(B->h_io + B->o_evals);
     const int* hb = reinterpret_cast<const int*>(B->h_io + B->o_best);

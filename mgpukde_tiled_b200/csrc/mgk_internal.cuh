@@ -45,9 +45,9 @@ struct mgk_ctx {
     void* h_stage[kStageSlots] = {};
     void* d_stage[kStageSlots] = {};
     size_t h_stage_bytes[kStageSlots] = {};
-    // a small mapped page-locked page: word 0 the index sort's wait flag, words
-    // 32 and 33 an adaptive likelihood (a double), words 64.. the extents of
-    // k_extent's CTAs or the largest h of k_adaptive_h's
+    // a small mapped page-locked page: words 32 and 33 an adaptive likelihood (a
+    // double), words 64.. the extents of k_extent's CTAs or the largest h of
+    // k_adaptive_h's
     unsigned *h_map = nullptr, *d_map = nullptr;
     mgk_raster_pipe* pipe = nullptr;
     std::multimap<size_t, void*> pool;        // cached device blocks by size class
@@ -330,9 +330,8 @@ struct mgk_extent {
     float hmax = 0;
 };
 int mgk_points_extent(mgk_ctx* ctx, const mgk_points* pts, bool want_h, mgk_extent* out);
-int mgk_sort_check(mgk_ctx* ctx);
-// Builds the index on ctx->stream without waiting for it (mgk_sort_check after
-// a wait); the points' arrays are read until then.  inv (device, n entries, or
+// Builds the index on ctx->stream without waiting for it; the points' arrays
+// are read until it is done.  inv (device, n entries, or
 // null): the place of each point's record.
 int mgk_launch_index_build(mgk_ctx* ctx, const mgk_points* pts, float h, float bin_size, const mgk_extent* extent,
                            mgk_index* idx, int32_t* inv = nullptr);
