@@ -188,7 +188,7 @@ __device__ __noinline__ unsigned count_digit(const unsigned* __restrict__ keys, 
 // 289 -> 144 and 99 -> 54 us).  Before the first pass the values are the
 // items' indexes.
 template <int IPT, typename W, int N>
-__global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, int db, size_t look_bytes,
+__global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, int passes, int db, size_t look_bytes,
                                                              const __grid_constant__ Jobs<SortJob, N> J) {
     const SortJob& B = J.j[N > 1 ? blockIdx.y : 0];
     const unsigned* __restrict__ keys_in = p & 1 ? B.kb : B.ka;
@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_pass(int64_t n, int p, i
     unsigned* __restrict__ keys_out = p & 1 ? B.ka : B.kb;
     int32_t* __restrict__ vals_out = p & 1 ? B.va : B.vb;
     const unsigned* __restrict__ hist = B.scratch + (p << db);
-    unsigned* tick = B.scratch + kMaxPasses * kMaxDigits + p;
-    W* look = reinterpret_cast<W*>(reinterpret_cast<char*>(B.scratch + kMaxPasses * kMaxDigits + 8) + p * look_bytes);
+    unsigned* tick = B.scratch + (passes << db) + p;
+    W* look = reinterpret_cast<W*>(reinterpret_cast<char*>(B.scratch + (passes << db) + 8) + p * look_bytes);
     const int shift = p * db;
     constexpr int kTop = sizeof(W) * 8 - 2;
     constexpr W kVal = ((W)1 << kTop) - 1;
@@ -287,11 +287,12 @@ struct SortPlan {
     bool wide;  // counts of 2^30 items and more: 64-bit state words
     size_t look_bytes() const { return (size_t)ntiles * ((size_t)1 << db) * (wide ? 8 : 4); }
     size_t bytes() const {  // [digit counts | tile counters | state words], zeroed before the keys
-        return sizeof(unsigned) * (kMaxPasses * kMaxDigits + 8) + (size_t)passes * look_bytes();
+        return sizeof(unsigned) * (((size_t)passes << db) + 8) + (size_t)passes * look_bytes();
     }
 };
 
-SortPlan sort_plan(int64_t n, int bits) {
+// spare: the least scratch instead of the tiles that sort fastest.
+SortPlan sort_plan(int64_t n, int bits, bool spare) {
     SortPlan P;
     bits = std::max(bits, 1);
     P.passes = (bits + 8) / 9;
@@ -299,7 +300,7 @@ SortPlan sort_plan(int64_t n, int bits) {
     // Large tiles shorten the look back, small ones keep the SMs busy: 16, 4, 4
     // items a thread instead took 161 us for 10^6 points (144 with 16) and 4, 1
     // for 200,000 125 us (109 with 4).
-    P.ipt = n >= (1 << 19) ? 16 : n >= (1 << 16) ? 4 : 1;
+    P.ipt = spare || n >= (1 << 19) ? 16 : n >= (1 << 16) ? 4 : 1;
     P.ntiles = (n + (int64_t)kSortThreads * P.ipt - 1) / ((int64_t)kSortThreads * P.ipt);
     P.wide = n >= (1ll << 30);
     return P;
@@ -313,13 +314,14 @@ void sort_passes(cudaStream_t s, const SortPlan& P, int64_t n, int nj, const Job
     const dim3 g((unsigned)P.ntiles, (unsigned)nj);
     for (int p = 0; p < P.passes; p++) {
         if (P.wide)
-            k_radix_pass<16, unsigned long long, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
+            k_radix_pass<16, unsigned long long, N><<<g, kSortThreads, 0, s>>>(n, p, P.passes, P.db, P.look_bytes(),
+                                                                              J);
         else if (P.ipt == 16)
-            k_radix_pass<16, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
+            k_radix_pass<16, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.passes, P.db, P.look_bytes(), J);
         else if (P.ipt == 4)
-            k_radix_pass<4, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
+            k_radix_pass<4, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.passes, P.db, P.look_bytes(), J);
         else
-            k_radix_pass<1, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.db, P.look_bytes(), J);
+            k_radix_pass<1, unsigned, N><<<g, kSortThreads, 0, s>>>(n, p, P.passes, P.db, P.look_bytes(), J);
     }
 }
 
@@ -610,17 +612,17 @@ struct SortBuf {
 
 static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
-static SortPlan bin_plan(int64_t n, int64_t nbins) {
+static SortPlan bin_plan(int64_t n, int64_t nbins, bool spare = false) {
     int bits = 0;
     while (bits < 32 && ((uint64_t)(nbins - 1) >> bits) != 0) bits++;
-    return sort_plan(n, bits);
+    return sort_plan(n, bits, spare);
 }
 
-static SortPlan zorder_plan(int64_t n, int64_t nbx, int64_t nby) {
+static SortPlan zorder_plan(int64_t n, int64_t nbx, int64_t nby, bool spare = false) {
     const uint64_t maxb = (uint64_t)std::max(nbx, nby) - 1;
     int bits = 0;
     while (bits < 16 && (maxb >> bits) != 0) bits++;
-    return sort_plan(n, 2 * bits);
+    return sort_plan(n, 2 * bits, spare);
 }
 
 // The records, their permutation and the bin starts of nj indexes of the same
@@ -693,46 +695,61 @@ static cudaError_t enqueue_zorder(mgk_ctx* ctx, int nj, mgk_index* const* idx, i
     return cudaGetLastError();
 }
 
-// Runs enqueue(scratch) with a sort's zeroed scratch for n items.
-template <typename Enqueue>
-static int with_sort_buf(mgk_ctx* ctx, int64_t n, const SortPlan& P, const char* what, const Enqueue& enqueue) {
-    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
-    char* base = nullptr;
+// Runs enqueue(scratch, plan) with a sort's zeroed scratch for n items: in one
+// block, or without the memory for that by the plan of the least scratch in
+// blocks of their own.  plan_of(spare): the sort's plan.
+template <typename PlanOf, typename Enqueue>
+static int with_sort_buf(mgk_ctx* ctx, int64_t n, const PlanOf& plan_of, const char* what, const Enqueue& enqueue) {
+    SortPlan P = plan_of(false);
+    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), b_one = 3 * b_buf + P.bytes();
+    void* blk[4] = {};
+    size_t b_blk[4] = {b_one, b_buf, b_buf, b_buf};
+    SortBuf b{};
     int st;
-    if ((st = mgk_alloc(ctx, (void**)&base, need))) return st;
-    const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
+    if ((st = mgk_alloc(ctx, &blk[0], b_one)) == MGK_OK) {
+        char* base = static_cast<char*>(blk[0]);
+        b = SortBuf{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
                     (unsigned*)(base + 3 * b_buf)};
-    cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), ctx->stream);
-    if (e == cudaSuccess) e = enqueue(b);
+    } else {
+        P = plan_of(true);
+        b_blk[0] = P.bytes();
+        st = MGK_OK;
+        for (int i = 0; i < 4 && st == MGK_OK; i++) st = mgk_alloc(ctx, &blk[i], b_blk[i]);
+        b = SortBuf{(unsigned*)blk[1], (unsigned*)blk[2], (int32_t*)blk[3], (unsigned*)blk[0]};
+    }
+    cudaError_t e = cudaSuccess;
+    if (st == MGK_OK) e = cudaMemsetAsync(b.scr, 0, P.bytes(), ctx->stream);
+    if (st == MGK_OK && e == cudaSuccess) e = enqueue(b, P);
     // back to the context's pool; later users are ordered after these kernels on the same stream
-    mgk_free(ctx, base, need);
+    for (int i = 0; i < 4; i++) mgk_free(ctx, blk[i], b_blk[i]);
     if (e != cudaSuccess) return mgk_cuda_fail(ctx, e, what);
-    return MGK_OK;
+    return st;
 }
 
 // Z-order of one index's records.
 static int index_zorder(mgk_ctx* ctx, mgk_index* idx, int32_t* d_order) {
-    const SortPlan P = zorder_plan(idx->n, idx->nbx, idx->nby);
-    return with_sort_buf(ctx, idx->n, P, "index_zorder",
-                         [&](const SortBuf& b) { return enqueue_zorder<1>(ctx, 1, &idx, &d_order, &b, P); });
+    return with_sort_buf(
+        ctx, idx->n, [&](bool spare) { return zorder_plan(idx->n, idx->nbx, idx->nby, spare); }, "index_zorder",
+        [&](const SortBuf& b, const SortPlan& P) { return enqueue_zorder<1>(ctx, 1, &idx, &d_order, &b, P); });
 }
 
 int mgk_points_curve_order(mgk_ctx* ctx, const mgk_points* pts, const mgk_extent& extent, int32_t* d_order) {
     const int64_t n = pts->n;
     if (n == 0) return MGK_OK;
     const double ext = std::max(extent.xmax - extent.xmin, extent.ymax - extent.ymin);
-    const SortPlan P = sort_plan(n, 32);
-    return with_sort_buf(ctx, n, P, "points_curve_order", [&](const SortBuf& b) {
-        const bool odd = P.passes & 1;  // the values end in d_order
-        Jobs<SortJob, 1> S{};
-        S.j[0] = SortJob{b.k0, b.k1, odd ? b.v0 : d_order, odd ? d_order : b.v0, b.scr};
-        k_hilbert_keys<<<key_grid(ctx, n), 256, 0, ctx->stream>>>(n, pts->x, pts->y, extent.xmin, extent.ymin,
-                                                                  ext > 0.0 ? 65536.0 / ext : 0.0, P.db, P.passes, b.k0,
-                                                                  b.scr);
-        sort_passes<1>(ctx->stream, P, n, 1, S);
-        MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
-        return cudaGetLastError();
-    });
+    return with_sort_buf(
+        ctx, n, [&](bool spare) { return sort_plan(n, 32, spare); }, "points_curve_order",
+        [&](const SortBuf& b, const SortPlan& P) {
+            const bool odd = P.passes & 1;  // the values end in d_order
+            Jobs<SortJob, 1> S{};
+            S.j[0] = SortJob{b.k0, b.k1, odd ? b.v0 : d_order, odd ? d_order : b.v0, b.scr};
+            k_hilbert_keys<<<key_grid(ctx, n), 256, 0, ctx->stream>>>(n, pts->x, pts->y, extent.xmin, extent.ymin,
+                                                                      ext > 0.0 ? 65536.0 / ext : 0.0, P.db, P.passes,
+                                                                      b.k0, b.scr);
+            sort_passes<1>(ctx->stream, P, n, 1, S);
+            MGK_COUNT_LAUNCH(ctx, 1 + P.passes);
+            return cudaGetLastError();
+        });
 }
 
 int mgk_index_refresh_weights(mgk_ctx* ctx, mgk_index* idx, const mgk_points* pts) {
@@ -835,18 +852,21 @@ static int index_fill(mgk_ctx* ctx, const mgk_points* pts, mgk_index* idx, int32
         return MGK_OK;
     }
     // The sort's scratch lies in the record buffer, which the gather fills
-    // last, or, where the gather fills the bin starts, in a buffer of its own
-    // (while there is memory for it).
-    const SortPlan P = bin_plan(n, nbins);
-    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), need = 3 * b_buf + P.bytes();
+    // last, or, where the gather fills the bin starts or the record buffer is
+    // too small, in a buffer of its own.  Without the memory for one, the plan of
+    // the least scratch, which fits the record buffer from about 500 points.
+    SortPlan P = bin_plan(n, nbins);
+    const size_t b_buf = up256(sizeof(unsigned) * (size_t)n), room = sizeof(MgkPt) * (size_t)n;
+    size_t need = 3 * b_buf + P.bytes();
     char* base = reinterpret_cast<char*>(idx->pts);
     void* own = nullptr;
     int st;
-    const bool fits = need <= sizeof(MgkPt) * (size_t)n;
-    if (!fits || (nbins <= kFillBins && n < (1 << 19))) {
-        if ((st = mgk_alloc(ctx, &own, need)) && !fits) return st;
-        if (own) base = static_cast<char*>(own);
+    if ((need > room || (nbins <= kFillBins && n < (1 << 19))) && mgk_alloc(ctx, &own, need) && need > room) {
+        P = bin_plan(n, nbins, true);
+        need = 3 * b_buf + P.bytes();
+        if (need > room && (st = mgk_alloc(ctx, &own, need))) return st;
     }
+    if (own) base = static_cast<char*>(own);
     const SortBuf b{(unsigned*)base, (unsigned*)(base + b_buf), (int32_t*)(base + 2 * b_buf),
                     (unsigned*)(base + 3 * b_buf)};
     cudaError_t e = cudaMemsetAsync(b.scr, 0, P.bytes(), s);
