@@ -662,6 +662,14 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     const int64_t items = (int64_t)nh * std::max(B->ngroups, 1) * kLooSub;
     const int64_t want = (p->n < (1 << 13) ? 2 : 4) * resident;
     if (items < want) nsplit = (int)std::min<int64_t>(kMaxSplit, (want + items - 1) / items);
+    // What follows is left out where there is no memory for it, so it comes after
+    // all that is needed: the runs, and for one bandwidth the blocks that the edge
+    // weights take during the run (held here, and in the pool by then).
+    if (st == MGK_OK && r) st = mgk_raster_runs(c, const_cast<mgk_raster*>(r));
+    const size_t b_later[2] = {sizeof(int) * n1, 2 * sizeof(int)};
+    void* later[2] = {};
+    if (r && nh == 1)
+        for (int i = 0; i < 2 && st == MGK_OK; i++) st = mgk_alloc(c, &later[i], b_later[i]);
     if (st == MGK_OK && nsplit > 1) {
         B->bytes_psum = sizeof(double) * (size_t)nsplit * (size_t)nh * (size_t)std::max(B->gcount, 1) * kLooQ;
         if (mgk_alloc(c, (void**)&B->d_psum, B->bytes_psum)) nsplit = 1;  // no memory: whole groups
@@ -673,7 +681,7 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
         B->bytes_wl = sizeof(float) * n1 * (size_t)nh;
         if (mgk_alloc(c, (void**)&B->d_wl, B->bytes_wl)) B->d_wl = nullptr;
     }
-    if (st == MGK_OK && r) st = mgk_raster_runs(c, const_cast<mgk_raster*>(r));
+    for (int i = 0; i < 2; i++) mgk_free(c, later[i], b_later[i]);
     // a staging slot of the context (a batch lives within one call, whose
     // extent above has waited for the slot's former users)
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
