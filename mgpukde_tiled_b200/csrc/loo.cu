@@ -47,6 +47,7 @@ constexpr int kLooSum = 128;  // candidates of a bin row summed in plain FP32 be
 constexpr int kLooWarps = 4;  // warps per CTA, each with work items of its own
 constexpr int kMaxLev = 16;   // bandwidth octaves
 constexpr int kMaxSplit = 16;
+constexpr unsigned kMaxGridY = 65535;  // longer lists of bandwidths go through it again
 // candidates of a batch scanned at a time (one test for the rare cases)
 #ifndef MGK_LOO_TRIP
 #define MGK_LOO_TRIP 8
@@ -143,12 +144,13 @@ __global__ void k_loo_prep(LooParams P, LooHost H, float* __restrict__ hgrid, Le
 // wl[k][i] = w e(h_k) of record i of the level of h_k: the scan then reads its
 // candidates' weights in order instead of through the permutation.
 __global__ void k_loo_weights(LooParams P) {
-    const int k = blockIdx.y;
-    const LevelDesc L = P.lev[P.klevel[k]];
-    const float* ewk = P.ew + (int64_t)k * P.ew_chunk;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pi = L.perm[i], ch = pi / P.ew_chunk;
-        P.wl[(int64_t)k * P.n + i] = L.pts[i].wk * ewk[ch * P.ew_cstride + (pi - ch * P.ew_chunk)];
+    for (int k = blockIdx.y; k < P.nh; k += gridDim.y) {
+        const LevelDesc L = P.lev[P.klevel[k]];
+        const float* ewk = P.ew + (int64_t)k * P.ew_chunk;
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.n; i += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t pi = L.perm[i], ch = pi / P.ew_chunk;
+            P.wl[(int64_t)k * P.n + i] = L.pts[i].wk * ewk[ch * P.ew_cstride + (pi - ch * P.ew_chunk)];
+        }
     }
 }
 
@@ -454,17 +456,19 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
 // The log sums of the groups' quarters from the parts' sums of each query,
 // added in order (one warp per quarter).
 __global__ void __launch_bounds__(kLooWarps * 32) k_loo_combine(LooParams P) {
-    const int lane = threadIdx.x & 31, gi = blockIdx.x * kLooWarps + (threadIdx.x >> 5), k = blockIdx.y;
+    const int lane = threadIdx.x & 31, gi = blockIdx.x * kLooWarps + (threadIdx.x >> 5);
     const int64_t ngs = (int64_t)P.gcount * kLooSub;
     if (gi >= ngs) return;
-    double lg = 0.0;
-    if ((int64_t)P.g0 * kLooQ + (int64_t)gi * 32 + lane < P.n) {
-        double v = 0.0;
-        for (int sp = 0; sp < P.nsplit; sp++) v += P.psum[(((int64_t)sp * P.nh + k) * ngs + gi) * 32 + lane];
-        lg = loo_log(v, mgk_h2(P.hgrid[k]));
+    for (int k = blockIdx.y; k < P.nh; k += gridDim.y) {
+        double lg = 0.0;
+        if ((int64_t)P.g0 * kLooQ + (int64_t)gi * 32 + lane < P.n) {
+            double v = 0.0;
+            for (int sp = 0; sp < P.nsplit; sp++) v += P.psum[(((int64_t)sp * P.nh + k) * ngs + gi) * 32 + lane];
+            lg = loo_log(v, mgk_h2(P.hgrid[k]));
+        }
+        const double sum = warp_sum(lg);
+        if (lane == 0) P.part[k * ngs + gi] = sum;
     }
-    const double sum = warp_sum(lg);
-    if (lane == 0) P.part[k * ngs + gi] = sum;
 }
 
 // logL[k] = fixed-order sum of the group partials of h_k (one CTA per h).  The
@@ -565,12 +569,13 @@ static int loo_enqueue(mgk_loo_batch* B) {
     }
     if (B->P.wl) {
         const unsigned gx = (unsigned)std::min<int64_t>((B->n + 255) / 256, 4 * (int64_t)ctx->sm_count);
-        k_loo_weights<<<dim3(gx, (unsigned)B->nh), 256, 0, s>>>(B->P);
+        k_loo_weights<<<dim3(gx, std::min((unsigned)B->nh, kMaxGridY)), 256, 0, s>>>(B->P);
     }
     if (B->P.gcount > 0) {
         k_loo_multi<<<(unsigned)B->grid, kLooWarps * 32, 0, s>>>(B->P);
         if (B->P.psum)
-            k_loo_combine<<<dim3((unsigned)((B->P.gcount * kLooSub + kLooWarps - 1) / kLooWarps), (unsigned)B->nh),
+            k_loo_combine<<<dim3((unsigned)((B->P.gcount * kLooSub + kLooWarps - 1) / kLooWarps),
+                                 std::min((unsigned)B->nh, kMaxGridY)),
                             kLooWarps * 32, 0, s>>>(B->P);
     }
     k_loo_finish<<<B->nh, 256, 0, s>>>(B->P, B->io, B->P.gcount * kLooSub, B->d_logl);
