@@ -48,6 +48,7 @@ constexpr int kLooWarps = 4;  // warps per CTA, each with work items of its own
 constexpr int kMaxLev = 16;   // bandwidth octaves
 constexpr int kMaxSplit = 16;
 constexpr unsigned kMaxGridY = 65535;  // longer lists of bandwidths go through it again
+constexpr int64_t kMaxItems = 1ll << 31;  // work items of a launch (32-bit numbers, handed out past the last)
 // candidates of a batch scanned at a time (one test for the rare cases)
 #ifndef MGK_LOO_TRIP
 #define MGK_LOO_TRIP 8
@@ -73,6 +74,7 @@ struct LooParams {
     int ngroups;
     int g0, gcount;       // this share's query groups [g0, g0 + gcount) (all groups: 0, ngroups)
     int nh;
+    int k0, k1;           // places in the processing order that a launch of the scan takes
     const float* hgrid;   // [nh]
     int* korder;          // [nh] processing order (largest h first)
     int* klevel;          // [nh] level of each h
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
     int4* row = s_row[warp];
     const unsigned ngs = (unsigned)P.gcount * kLooSub;  // quarters of groups
     const unsigned per_h = ngs * (unsigned)P.nsplit;
-    const unsigned total = (unsigned)P.nh * per_h;
+    const unsigned total = (unsigned)(P.k1 - P.k0) * per_h;
     const f2 magic = f2_dup(12582912.0f);  // 1.5 2^23: adding it rounds to the nearest integer
     unsigned long long cnt_all = 0;
     for (;;) {
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
         if (lane == 0) item = atomicAdd(P.counter, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= total) break;
-        const int k = P.korder[item / per_h];
+        const int k = P.korder[P.k0 + (int)(item / per_h)];
         const int split = (int)((item % per_h) / ngs);
         const int gi = (int)((item % per_h) % ngs);  // quarter gi % kLooSub of group gi / kLooSub
         const LevelDesc& L = P.lev[P.klevel[k]];
@@ -553,9 +555,16 @@ struct mgk_loo_batch {
     int grid = 1;
 };
 
+// Bandwidths that one launch of the scan takes: all but for very long lists of very many points.
+static int scan_part(const mgk_loo_batch* B) {
+    const int64_t per_h = (int64_t)B->P.gcount * kLooSub * B->P.nsplit;
+    return (int)std::min<int64_t>(B->nh, std::max<int64_t>(1, kMaxItems / std::max<int64_t>(per_h, 1)));
+}
+
 // Kernels of a batch, the edge weights' aside.
 static int loo_launches(const mgk_loo_batch* B) {
-    return 2 + (B->P.wl ? 1 : 0) + (B->P.gcount > 0 ? 1 : 0) + (B->P.gcount > 0 && B->P.psum ? 1 : 0);
+    const int scans = (B->nh + scan_part(B) - 1) / scan_part(B);
+    return 2 + (B->P.wl ? 1 : 0) + (B->P.gcount > 0 ? scans : 0) + (B->P.gcount > 0 && B->P.psum ? 1 : 0);
 }
 
 static int loo_enqueue(mgk_loo_batch* B) {
@@ -572,7 +581,12 @@ static int loo_enqueue(mgk_loo_batch* B) {
         k_loo_weights<<<dim3(gx, std::min((unsigned)B->nh, kMaxGridY)), 256, 0, s>>>(B->P);
     }
     if (B->P.gcount > 0) {
-        k_loo_multi<<<(unsigned)B->grid, kLooWarps * 32, 0, s>>>(B->P);
+        LooParams P = B->P;
+        for (P.k0 = 0; P.k0 < B->nh; P.k0 = P.k1) {
+            P.k1 = P.k0 + std::min(scan_part(B), B->nh - P.k0);
+            if (P.k0) MGK_CHECK_CUDA(ctx, cudaMemsetAsync(B->d_counter, 0, sizeof(unsigned), s));
+            k_loo_multi<<<(unsigned)B->grid, kLooWarps * 32, 0, s>>>(P);
+        }
         if (B->P.psum)
             k_loo_combine<<<dim3((unsigned)((B->P.gcount * kLooSub + kLooWarps - 1) / kLooWarps),
                                  std::min((unsigned)B->nh, kMaxGridY)),
