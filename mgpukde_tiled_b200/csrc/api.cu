@@ -28,7 +28,7 @@
 constexpr int kDepth = MGK_RASTER_DEPTH;
 
 // Streams and events of the whole-raster path, made by a context's first call
-// and kept for the next (making and dropping the four streams and thirteen
+// and kept for the next (making and dropping the four streams and fourteen
 // events took about 0.2 ms of each call).  Every call waits for its streams
 // before it returns, on errors too, so nothing is in flight between calls;
 // a context serves one thread at a time.
@@ -43,7 +43,9 @@ struct mgk_raster_pipe {
             if (out_free[i]) cudaEventDestroy(out_free[i]);
             if (dens[i]) cudaEventDestroy(dens[i]);
         }
-                if (h2d) cudaStreamDestroy(h2d);
+        if (counted) cudaEventDestroy(counted);
+        if (em_ready) cudaEventDestroy(em_ready);
+        if (h2d) cudaStreamDestroy(h2d);
         if (d2h) cudaStreamDestroy(d2h);
         if (alt) cudaStreamDestroy(alt);
         if (mrg) cudaStreamDestroy(mrg);
