@@ -502,6 +502,8 @@ int mgk_mark_boundary(mgk_ctx* c, mgk_raster* r, int64_t* n_boundary) {
     if (!c || !r) return mgk_fail(c, MGK_ERR_INVALID, "mark_boundary: bad arguments");
     int st = mgk_launch_mark_boundary(c, r);
     if (st) return st;
+    // the cells and runs are complete with their count: other streams may read them
+    MGK_CHECK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (n_boundary) *n_boundary = r->nb;
     return MGK_OK;
 }

@@ -66,3 +66,25 @@ def test_marked_again_without_memory():
                 continue
             assert np.array_equal(pts.download(dist2=True, ew=False)[0], ref)
     assert refused >= 1
+
+
+def test_marked_on_one_stream_read_on_another():
+    side = 900
+    g = o.grid(side, side, 0.0, 0.0, 1.0, -9999.0)
+    r = np.random.default_rng(5)
+    m = np.where(r.random((side, side)) < 0.1, g.nodata, 1.0).astype(np.float32)
+    x, y = r.uniform(0, side, 100).astype(np.float32), r.uniform(0, side, 100).astype(np.float32)
+    bm = o.mark_boundary(g, m)
+    ref = o.dist2_boundary(x, y, g, bm)
+    ew, _ = o.edge_weights(x, y, 9.0, ref, g, m)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with mk.Context(0, stream=a) as ctx:
+        pts = mk.Points.upload(ctx, x, y)
+        ras = mk.Raster.upload(ctx, mk.Grid.of(g), m)
+        assert mk.mark_boundary(ctx, ras) == int(np.count_nonzero(bm))
+        ctx.set_stream(b)
+        mk.calc_dist2_boundary(ctx, pts, ras)
+        mk.edge_correction_weights(ctx, pts, ras, 9.0)
+        d2, got = pts.download(dist2=True)
+    assert np.array_equal(d2, ref)
+    assert np.all(np.abs(got - ew) <= 1e-6 * np.abs(ew))
