@@ -61,10 +61,11 @@ constexpr float kPdBand = 4e-6f * kPdCut;
 
 // psum[y][q] = sum over candidates i (the points of the index within reach
 // of the CTA's 32 queries, in the bin rows y, y + nsplit, ... of
-// the window, y = blockIdx.y) of [in cutoff] K w_i e_i, unnormalised; the
-// query itself is included when SELF.  Fixed h: terms exp2(-d^2 k2) w e;
-// per-point h (VARH): the candidate's own k2 and cutoff, weights already
-// carry 1/(h_i^2 TWO_PI).  Splitting the rows over nsplit CTAs gives a
+// the window, y = blockIdx.y) of [in cutoff] K w_i e_i, unnormalised.  Fixed h
+// (the pilot density): the query itself included, terms exp2(-d^2 k2) w e;
+// per-point h (VARH, the leave-one-out density): without the query itself, the
+// candidate's own k2 and cutoff, weights already carry 1/(h_i^2 TWO_PI).
+// Splitting the rows over nsplit CTAs gives a
 // launch enough CTAs for the whole GPU when there are few queries.
 //
 // The queries are the points along a Hilbert curve (order; record inv[order[q]]),
@@ -85,7 +86,7 @@ constexpr float kPdBand = 4e-6f * kPdCut;
 // (about 25 instructions per candidate and warp).  50,000 points, one
 // likelihood's sum with per-point h: 1.06 ms with 128 queries a CTA, scalar
 // FP32 and one span of bins per row, 0.41 ms now.
-template <bool VARH, bool SELF>
+template <bool VARH>
 __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const MgkPt* __restrict__ pts,
                                                             const int32_t* __restrict__ bin_start, double ox,
                                                             double oy, double side, int64_t nbx, int64_t nby,
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
         __syncwarp();
         // the query's own slot
         int jself = -1;
-        if (!SELF) {
+        if (VARH) {
             int pre = 0;
             for (int i = 0; i < nseg; i++) {
                 const int2 g = seg[i];
@@ -457,8 +458,8 @@ struct QueryOrder {
 };
 
 // den[input order] and logsum[0] = sum_j log(max(den_j, floor_v)).
-int point_density(mgk_ctx* c, const mgk_index* idx, QueryOrder& qo, bool self, double* d_den, double floor_v,
-                  double* d_logsum) {
+// A fixed-h index: every query itself included; per-point h: without it.
+int point_density(mgk_ctx* c, const mgk_index* idx, QueryOrder& qo, double* d_den, double floor_v, double* d_logsum) {
     cudaStream_t s = c->stream;
     const int64_t g = (idx->n + kPdQ - 1) / kPdQ;
     if (g == 0) {
@@ -496,23 +497,16 @@ int point_density(mgk_ctx* c, const mgk_index* idx, QueryOrder& qo, bool self, d
         k_fill_f32<<<(unsigned)((nbins + 255) / 256), 256, 0, s>>>(nbins, -1.0f, r2);
         k_bin_reach2<<<(unsigned)((idx->n + 255) / 256), 256, 0, s>>>(idx->n, idx->pts, idx->ox, idx->oy,
                                                                      1.0 / idx->side, idx->nbx, idx->nby, r2);
-        k_point_density<true, false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
-                                                           idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                           idx->h2, r2, qo.order, qo.inv, psum,
-                                                           pair_count(c));
-    } else if (self) {
-        k_point_density<false, true><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
-                                                           idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                           idx->h2, nullptr, qo.order, qo.inv, psum,
-                                                           pair_count(c));
+        k_point_density<true><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox, idx->oy, idx->side,
+                                                    idx->nbx, idx->nby, idx->reach, idx->h2, r2, qo.order, qo.inv,
+                                                    psum, pair_count(c));
     } else {
-        k_point_density<false, false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox,
-                                                            idx->oy, idx->side, idx->nbx, idx->nby, idx->reach,
-                                                            idx->h2, nullptr, qo.order, qo.inv, psum,
-                                                            pair_count(c));
+        k_point_density<false><<<grid, kPdQ, 0, s>>>(idx->n, idx->pts, idx->bin_start, idx->ox, idx->oy, idx->side,
+                                                     idx->nbx, idx->nby, idx->reach, idx->h2, nullptr, qo.order,
+                                                     qo.inv, psum, pair_count(c));
     }
-    k_pd_combine<<<(unsigned)gc, kPdC, 0, s>>>(idx->n, nsplit, psum, qo.order ? qo.order : idx->perm, idx->varh, idx->h2, floor_v, d_den,
-                                              part);
+    k_pd_combine<<<(unsigned)gc, kPdC, 0, s>>>(idx->n, nsplit, psum, qo.order ? qo.order : idx->perm, idx->varh,
+                                              idx->h2, floor_v, d_den, part);
     k_sum_parts<<<1, 256, 0, s>>>(gc, part, d_logsum);
     const cudaError_t e = cudaGetLastError();
     // pooled blocks: a later allocation of them is ordered on the same stream
@@ -579,7 +573,7 @@ int pilot_density(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, Pilot
             return mgk_index_build_async(c, p, h, 0.0f, &pc.extent, &idx, pc.qo.inv);
         });
         if (st == MGK_OK) {
-            st = point_density(c, idx, pc.qo, true, den, 0.0, den + std::max<int64_t>(p->n, 1));
+            st = point_density(c, idx, pc.qo, den, 0.0, den + std::max<int64_t>(p->n, 1));
             mgk_index_destroy(idx);
         }
     }
@@ -636,7 +630,7 @@ int loglik_adaptive(mgk_ctx* c, mgk_points* p, const mgk_raster* r, float h, flo
     if ((st = pc.qo.needing([&] { return mgk_index_build_async(c, p, 0.0f, 0.75f * h, &extent, &idx, pc.qo.inv); })))
         return st;
     double *sum = reinterpret_cast<double*>(c->h_map + 32), *d_sum = reinterpret_cast<double*>(c->d_map + 32);
-    st = point_density(c, idx, pc.qo, false, d_den, (double)MGK_EPS_DENSITY_F, d_sum);
+    st = point_density(c, idx, pc.qo, d_den, (double)MGK_EPS_DENSITY_F, d_sum);
     mgk_index_destroy(idx);
     if (st) return st;
     MGK_CHECK_CUDA(c, cudaStreamSynchronize(c->stream));

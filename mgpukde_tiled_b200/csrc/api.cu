@@ -229,7 +229,6 @@ int mgk_ctx_create(int device, uint64_t hbm_budget_bytes, mgk_ctx** out) {
     }
     c->stream = c->own_stream;
     if (cudaMalloc(&c->d_counter, 8 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&c->d_sum, 256 * sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&c->h_counter, 8 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaHostAlloc((void**)&c->h_map, 16384, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void**)&c->d_map, c->h_map, 0) != cudaSuccess ||
@@ -248,7 +247,6 @@ int mgk_ctx_destroy(mgk_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     release_pool(c);
     if (c->d_counter) cudaFree(c->d_counter);
-    if (c->d_sum) cudaFree(c->d_sum);
     if (c->h_counter) cudaFreeHost(c->h_counter);
     if (c->h_map) cudaFreeHost(c->h_map);
     delete c->pipe;

@@ -71,8 +71,7 @@ struct LooParams {
     int nlev;
     int nsplit;  // parts of a group's candidates, each a work item of its own
     int64_t n;
-    int ngroups;
-    int g0, gcount;       // this share's query groups [g0, g0 + gcount) (all groups: 0, ngroups)
+    int g0, gcount;       // this share's query groups [g0, g0 + gcount) (all groups: from 0)
     int nh;
     int k0, k1;           // places in the processing order that a launch of the scan takes
     const float* hgrid;   // [nh]
@@ -729,7 +728,6 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
                     (unsigned long long*)(d_io + B->o_evals), (int*)(d_io + B->o_best)};
     P.lev = B->d_lev;
     P.n = p->n;
-    P.ngroups = B->ngroups;
     P.g0 = B->g0;
     P.gcount = B->gcount;
     P.nh = nh;

@@ -37,7 +37,6 @@ struct mgk_ctx {
     // small pinned/device scratch for scalar results
     unsigned long long* d_counter = nullptr;  // 8 counters
     unsigned long long* h_counter = nullptr;  // pinned mirror
-    double* d_sum = nullptr;                  // 256 doubles
     // mapped page-locked staging of plans and counts (mgk_host_stage), in
     // kStageSlots independent slots; h_stage[i] and d_stage[i] address the same
     // bytes.  Slot 3 holds the bit-packed density mask of mgk_kde_raster.
@@ -179,16 +178,6 @@ __device__ __forceinline__ float mgk_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// 2^-a for a double exponent a >= 0, to about the accuracy of ex2.approx:
-// the exponent is split into float hi + lo and the lo part applied to first
-// order (2^-(hi+lo) = 2^-hi (1 - lo ln2 + ...), |lo| <= 2^-24 hi).
-__device__ __forceinline__ float mgk_exp2_neg(double a) {
-    const float ah = __double2float_rn(a);
-    const float al = __double2float_rn(a - (double)ah);
-    const float e = mgk_ex2(-ah);
-    return fmaf(-al * MGK_LN2F, e, e);
 }
 
 // 2^-a for 0 <= a < 120, without the special-function unit: a = n + f with
