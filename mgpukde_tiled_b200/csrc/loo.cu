@@ -119,7 +119,7 @@ __device__ __forceinline__ double loo_log(double sum, double h2) {
 
 // The run's bandwidths and the levels into device memory, the counters to
 // zero; level and processing order of every h (one CTA; nh is small).
-__global__ void k_loo_prep(LooParams P, LooHost H, float* __restrict__ hgrid, LevelDesc* __restrict__ lev) {
+__global__ void k_loo_prep(LooParams P, LooHost H, float* hgrid, LevelDesc* __restrict__ lev) {  // hgrid is P.hgrid
     for (int k = threadIdx.x; k < P.nh; k += blockDim.x) hgrid[k] = H.h[k];
     for (int l = threadIdx.x; l < P.nlev; l += blockDim.x) lev[l] = H.lev[l];
     if (threadIdx.x < 2) {
