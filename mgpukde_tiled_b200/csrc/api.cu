@@ -838,7 +838,7 @@ int mgk_mle_fixed_bandwidth(mgk_ctx* c, mgk_points* p, const mgk_raster* r, floa
 // ---------------------------------------------------------- whole raster --
 // The tiles go through a three-stream pipeline: the mask of tile k+1 is
 // copied in (stream h2d) and the density of tile k-1 copied out (stream d2h)
-// while tile k is computed on the context stream, with two device buffers
+// while tile k is computed on the context stream, with kDepth device buffers
 // of each kind and events between the stages.  Without an explicit tile
 // side the raster is cut into full-width bands of about an eighth of its
 // rows (at least 256, a multiple of the 64-row density block), so that the

@@ -1208,9 +1208,9 @@ void fill_params(DParams& P, const mgk_index* idx, const mgk_grid* g, int64_t ro
 // Work items of one tile from its per-block candidate counts: blocks above K
 // candidates are split into items of at most K, each split item writing an
 // FP64 partial into its own scratch slot (fine: small tiles are split finer;
-// without the memory for that, coarsely).  K depends on this tile alone, so a
-// tile gets the same items (and bitwise the same result) alone or batched with
-// others.
+// a tile whose own partials do not fit the memory, coarsely).  K depends on this
+// tile alone, so a tile gets the same items (and bitwise the same result) alone
+// or batched with others.
 struct TilePlan {
     int nbx_t = 0, nby_t = 0;
     std::vector<Item> items;
@@ -1226,12 +1226,14 @@ void plan_tile(const int64_t* counts, int nbx_t, int nby_t, int sm_count, int wa
     int64_t total = 0;
     for (int b = 0; b < nblk; b++) total += counts[b];
     const int64_t slots_resident = (int64_t)sm_count * 2;
-    // Below about 1,200 candidates a slot the waves do not matter and the
-    // longest item does: 2,048 candidates are 32 batches, 345 us on an SM of
-    // its own.  Two items a slot then, but not under 256 candidates (a split
-    // item also writes and merges 64 KB): a 2,311 x 1,873 raster of 60,000
-    // points 5.65 -> 3.73 ms against 2,048 at least, 1.40 -> 1.40 ms where
-    // 800,000 points keep every slot busy; four a slot 1.45 ms there.
+    // With t candidates a slot (two CTAs an SM, with which the rule was measured;
+    // three are resident) and four waves: from t = 8,192 the waves decide,
+    // K = t / 4.  Below, the longest item does (2,048 candidates are 32 batches,
+    // 345 us on an SM of its own): K = 2,048 down to t = 4,096, then two items a
+    // slot, K = t / 2, down to t = 512, and 256 below (a split item also writes
+    // and merges 64 KB).  A 2,311 x 1,873 raster of 60,000 points 5.65 -> 3.73 ms
+    // against 2,048 at least, 1.40 -> 1.40 ms where 800,000 points keep every
+    // slot busy; four items a slot 1.45 ms there.
     const int64_t least =
         !fine ? 2048 : std::min<int64_t>(2048, std::max<int64_t>(256, total / (2 * slots_resident)));
     int64_t K = std::max<int64_t>(least, total / std::max<int64_t>(1, slots_resident * waves));
