@@ -263,7 +263,8 @@ int mgk_ctx_destroy(mgk_ctx* c) {
 
 int mgk_ctx_set_stream(mgk_ctx* c, void* stream) {
     if (!c) return MGK_ERR_INVALID;
-    if (c->marking) MGK_CHECK_CUDA(c, cudaEventSynchronize(c->ev_marked));
+    if (c->marking)
+        MGK_CHECK_CUDA(c, c->stream == c->own_stream ? cudaStreamSynchronize(c->stream) : cudaEventSynchronize(c->ev_marked));
     c->marking = false;
     c->stream = stream ? (cudaStream_t)stream : c->own_stream;
     return MGK_OK;
@@ -505,8 +506,9 @@ int mgk_mark_boundary(mgk_ctx* c, mgk_raster* r, int64_t* n_boundary) {
     int st = mgk_launch_mark_boundary(c, r);
     if (st) return st;
     // the cells and runs may still be on their way: waited for when the context
-    // changes its stream (a wait here takes 10 us of every small study)
-    MGK_CHECK_CUDA(c, cudaEventRecord(c->ev_marked, c->stream));
+    // changes its stream (a wait here takes 10 us of every small study; a
+    // caller's stream may be gone by then, so an event stands for it)
+    if (c->stream != c->own_stream) MGK_CHECK_CUDA(c, cudaEventRecord(c->ev_marked, c->stream));
     c->marking = true;
     if (n_boundary) *n_boundary = r->nb;
     return MGK_OK;

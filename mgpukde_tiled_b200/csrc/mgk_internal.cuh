@@ -52,8 +52,8 @@ struct mgk_ctx {
     std::multimap<size_t, void*> pool;        // cached device blocks by size class
     uint64_t launches = 0;                    // kernels launched by this context
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
-    cudaEvent_t ev_marked = nullptr;  // after the last mgk_mark_boundary's kernels
-    bool marking = false;             // recorded since the stream was set
+    bool marking = false;             // mgk_mark_boundary has been called since the stream was set
+    cudaEvent_t ev_marked = nullptr;  // after its kernels, on a caller's stream
     float last_density_ms = 0.0f;
     int64_t last_loo_evals[2] = {0, 0};  // edge and LOO evals of the last LOO batch run
     float last_loo_ms = 0.0f;
