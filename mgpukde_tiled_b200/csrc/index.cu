@@ -167,9 +167,10 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(unsigned* __restrict__ 
 }
 
 // Of the first n keys, those with digit d.
-__device__ __noinline__ unsigned count_digit(const unsigned* __restrict__ keys, int64_t n, int shift, unsigned mask,
-                                             unsigned d) {
+__device__ __forceinline__ unsigned count_digit(const unsigned* __restrict__ keys, int64_t n, int shift,
+                                                unsigned mask, unsigned d) {
     unsigned c = 0;
+#pragma unroll 1
     for (int64_t i = 0; i < n; i++) c += ((keys[i] >> shift) & mask) == d ? 1u : 0u;
     return c;
 }
