@@ -54,10 +54,10 @@ constexpr int kPdWarps = 224;
 // of a search (records' order / curve: 400 points 2.96 / 3.05 ms, 5,000 5.47 /
 // 5.52, 10,000 5.95 / 5.74, 50,000 24.1 / 22.8)
 constexpr int64_t kPdCurve = 1 << 13;
-// The cutoff in exponents, 9 h^2 log2(e) / (2 h^2) for every h, and the band
-// around it in which FP32 does not decide.
+// The cutoff of per-point h in exponents, 9 h^2 log2(e) / (2 h^2) for every h,
+// and the relative band around a cutoff in which FP32 does not decide.
 constexpr float kPdCut = (float)(0.5 * MGK_CUT * MGK_LOG2E);
-constexpr float kPdBand = 4e-6f * kPdCut;
+constexpr float kPdBand = 4e-6f;
 
 // psum[y][q] = sum over candidates i (the points of the index within reach
 // of the CTA's 32 queries, in the bin rows y, y + nsplit, ... of
@@ -123,7 +123,12 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
     const double k2 = MGK_LOG2E / (2.0 * h2);
     const f2 k2hc = f2_dup((float)k2), k2lc = f2_dup((float)(k2 - (double)(float)k2));
     const f2 qxh = f2_dup(q.x), qyh = f2_dup(q.y), qxl = f2_dup(q.z), qyl = f2_dup(q.w);
-    const f2 cut2 = f2_dup(kPdCut), magic = f2_dup(12582912.0f);
+    // fixed h: the cutoff of d^2 itself
+    const float cutf = VARH ? kPdCut : (float)(MGK_CUT * h2), band = kPdBand * cutf;
+    const f2 cut2 = f2_dup(cutf), magic = f2_dup(12582912.0f);
+    // past the end: beyond every cutoff, for any h (with fixed h the exponent of
+    // a finite distance may overflow to either side)
+    constexpr float kFar = VARH ? 1e18f : INFINITY;
     float s = 0.0f, c = 0.0f, part = 0.0f;
     auto flush = [&] {
         const float y = part - c;
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int j = jb + 32 * i;
-                cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end: far outside the cutoff
+                cp[i] = make_float4(kFar, 0.0f, 0.0f, 0.0f);
                 cq[i] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
                 if (j >= T) continue;
                 while (j >= sg.x) sg = seg[++r];
@@ -213,7 +218,7 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
                     const f2 dy = f2_add(f2_sub(at(1), qyh), f2_sub(at(3), qyl));
                     const f2 d2 = f2_fma(dx, dx, f2_mul(dy, dy));
                     const f2 a = f2_fma(d2, VARH ? at(kComp - 2) : k2hc, f2_mul(d2, VARH ? at(kComp - 1) : k2lc));
-                    f2_get(f2_sub(a, cut2), x[u], x[u + 1]);
+                    f2_get(f2_sub(VARH ? a : d2, cut2), x[u], x[u + 1]);
                     const f2 m1 = f2_sub(f2_sub(magic, a), magic);  // -n, a = n + g
                     float g0, g1, n0, n1;
                     f2_get(f2_add(a, m1), g0, g1);
@@ -227,10 +232,10 @@ __global__ void __launch_bounds__(kPdQ, 16) k_point_density(int64_t n, const Mgk
 #pragma unroll
                 for (int u = 1; u + 1 < kPdTrip; u += 2) near = mgk_min3(near, fabsf(x[u]), fabsf(x[u + 1]));
                 near = fminf(near, fabsf(x[kPdTrip - 1]));
-                if (near <= kPdBand || (unsigned)ts < (unsigned)kPdTrip) {
+                if (near <= band || (unsigned)ts < (unsigned)kPdTrip) {
 #pragma unroll
                     for (int u = 0; u < kPdTrip; u++) {
-                        if (fabsf(x[u]) <= kPdBand) {  // near the cutoff: the oracle's FP64 decision
+                        if (fabsf(x[u]) <= band) {  // near the cutoff: the oracle's FP64 decision
                             int i = 0;
                             while (j + t + u >= seg[i].x) i++;
                             const MgkPt cc = pts[j + t + u + seg[i].y];

@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kLooWarps * 32, MGK_LOO_MIN_CTAS) k_loo_multi(
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
                     const int j = jb + 32 * i;
-                    cp[i] = make_float4(1e18f, 0.0f, 0.0f, 0.0f);  // past the end: far outside the cutoff
+                    cp[i] = make_float4(INFINITY, 0.0f, 0.0f, 0.0f);  // past the end: beyond the cutoff of any h
                     cw[i] = 0.0f;
                     bool first = false;
                     int o = INT_MAX;
