@@ -695,7 +695,7 @@ int mgk_loo_batch_create_share(mgk_ctx* c, const mgk_points* p, const mgk_raster
     // The weights in record order are a shortcut: without the memory for them
     // the scan gathers each weight through the permutation.
     const bool has_ew = r || ew_ext;
-    if (st == MGK_OK && has_ew) {
+    if (st == MGK_OK && has_ew && p->n > 0) {
         B->bytes_wl = sizeof(float) * n1 * (size_t)nh;
         if (mgk_alloc(c, (void**)&B->d_wl, B->bytes_wl)) B->d_wl = nullptr;
     }
